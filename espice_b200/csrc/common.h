@@ -98,6 +98,24 @@ enum OpKind : uint32_t {
   kOpNop = 7,
 };
 
+// One task of a block-lane program: up to kTaskOps updates v[dst] -= v[a] *
+// v[b] in order, then (kTaskDiv) v[dst] /= v[divisor]. Eight words: dst |
+// flags, divisor | flags, then a, b of each update, in two planes of four
+// words per lane (one 16-byte load each); padding updates multiply the
+// constant 0.0 by 1.0. Flags of word 0: kTaskNz (an update with v[b] == 0 is
+// skipped, the solves' zero skip), kTaskDiv, and the same in every lane of
+// the warp: kTaskMore (more than one update), kTaskCta (a CTA barrier
+// follows). Flags of word 1: the division's pivot tests (kOpDivGrowth,
+// kOpDivScaled), and kTaskDivAny (a lane of the warp divides). A dst field
+// of kTaskIdle: the warp has no task for word 1's number of barriers.
+constexpr uint32_t kTaskOps = 3, kTaskWords = 8;
+constexpr uint32_t kTaskIndex = 0x0fffffffu, kTaskIdle = kTaskIndex;
+constexpr uint32_t kTaskNz = 1u << 28, kTaskDiv = 1u << 29, kTaskMore = 1u << 30, kTaskCta = 1u << 31;
+constexpr uint32_t kTaskGrowth = 1u << 28, kTaskScaled = 1u << 29, kTaskDivAny = 1u << 30;
+// Chunks (a warp's 32 tasks) the kernel takes per trip through its loop, and
+// reads ahead past a warp's last one.
+constexpr uint32_t kTaskUnroll = 3;
+
 // Per-lane transient statistics (the same fields, in the same order, as the
 // oracle's step counters), and the run's status word.
 enum TranStat : uint32_t {

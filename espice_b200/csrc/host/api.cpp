@@ -248,7 +248,6 @@ struct esl_ctx {
   bool have_block = false;
   bool profile = false;  // block lanes: accumulate the phase cycles (esl_solve_mode.profile)
   BlockPrograms bprog;
-  uint32_t block_op_bytes = 8;     // 8: 16-bit value indices; 16: 32-bit
   uint32_t block_g_len = 0, block_g_ncells = 0;
   DevBuf d_ba, d_bb, d_bf, d_slab, d_refine, d_prof, d_bg_terms, d_bg_cells;
   SparseLu lead;
@@ -804,26 +803,6 @@ int32_t upload_tape(esl_ctx* ctx) {
   return ESL_OK;
 }
 
-// The block lanes' program rows in their device format: 8-byte words
-// {dst | kind << 28, a | b << 16} when the value space has 16-bit indices,
-// else the 16-byte words as built.
-std::vector<uint32_t> block_words(const std::vector<Op4>& ops, bool short_ops) {
-  std::vector<uint32_t> w;
-  w.reserve(ops.size() * (short_ops ? 2 : 4));
-  for (const Op4& o : ops) {
-    if (short_ops) {
-      w.push_back(o.w0);
-      w.push_back(o.a | (o.b << 16));
-    } else {
-      w.push_back(o.w0);
-      w.push_back(o.a);
-      w.push_back(o.b);
-      w.push_back(0u);
-    }
-  }
-  return w;
-}
-
 // The block lanes' assembly streams (block.cu block_assemble): every
 // residual row and pattern slot is a cell summing its staging terms in list
 // order; cells go to the CTA's threads longest first, each to the least
@@ -886,54 +865,23 @@ void build_block_gather(const esl_ctx* ctx, uint32_t W, std::vector<uint32_t>& t
 }
 
 void block_layout(const TopoDev& T, uint32_t nv, bool mixed, bool split, BlockDev& D);
-uint32_t block_ring_bytes(uint32_t op_bytes, uint32_t row_k);
 constexpr size_t kBlockSmemRoom = size_t(227) * 1024 - 256;
-
-// Ops a thread a program row: kSlabRowOps when no placement of the working
-// set (whole or its hot part, FP64 or mixed) fits a CTA's shared memory
-// beside the op ring, so that the lanes run from the slab; 1 otherwise.
-uint32_t block_row_k(const TopoDev& T, uint32_t op_bytes) {
-  BlockDev D{};
-  for (int mixed = 0; mixed < 2; ++mixed)
-    for (int split = 0; split < 2; ++split) {
-      block_layout(T, T.nv, mixed != 0, split != 0, D);
-      if (D.lane_bytes + block_ring_bytes(op_bytes, 1) <= kBlockSmemRoom) return 1;
-    }
-  return kSlabRowOps;
-}
-
-// The block programs at rows of k ops a thread, uploaded in the context's
-// op format.
-int32_t set_block_programs(esl_ctx* ctx, uint32_t k) {
-  cudaStream_t s = ctx->stream;
-  const bool short_ops = ctx->block_op_bytes == 8;
-  ctx->bprog = compile_block(ctx->prog, k * kBlockThreads);
-  ctx->bprog.row_k = k;
-  ESL_CUDA(upload(ctx->d_ba, block_words(ctx->bprog.a_ops, short_ops), s));
-  ESL_CUDA(upload(ctx->d_bb, block_words(ctx->bprog.b_ops, short_ops), s));
-  ESL_CUDA(upload(ctx->d_bf, block_words(ctx->bprog.f_ops, short_ops), s));
-  return ESL_OK;
-}
 
 // The block lanes' programs and assembly streams of the current tape.
 int32_t ensure_block(esl_ctx* ctx) {
   if (ctx->have_block) return ESL_OK;
   cudaStream_t s = ctx->stream;
-  ctx->block_op_bytes = ctx->prog.nv < 65536 ? 8 : 16;
-  if (int32_t rc = set_block_programs(ctx, block_row_k(ctx->topo, ctx->block_op_bytes))) return rc;
+  if (ctx->prog.nv > kTaskIdle) return ctx->fail(ESL_NOT_ELIGIBLE, "the tape's values exceed 28-bit indices");
+  ctx->bprog = compile_block(ctx->prog);
+  ESL_CUDA(upload(ctx->d_ba, ctx->bprog.a.words, s));
+  ESL_CUDA(upload(ctx->d_bb, ctx->bprog.b.words, s));
+  ESL_CUDA(upload(ctx->d_bf, ctx->bprog.f.words, s));
   std::vector<uint32_t> terms, cells;
   build_block_gather(ctx, kBlockThreads, terms, cells, ctx->block_g_len, ctx->block_g_ncells);
   ESL_CUDA(upload(ctx->d_bg_terms, terms, s));
   ESL_CUDA(upload(ctx->d_bg_cells, cells, s));
   ctx->have_block = true;
   return ESL_OK;
-}
-
-// The op ring a block-lane CTA streams its programs through (block.cu
-// block_rows_k): kDepth + 1 slots of row_k op words per thread, 4 rows
-// ahead for rows of one op a thread, 2 for rows of kSlabRowOps.
-uint32_t block_ring_bytes(uint32_t op_bytes, uint32_t row_k) {
-  return (row_k == 1 ? 5u : 3u) * row_k * kBlockThreads * op_bytes;
 }
 
 // A block lane's working set (block.cu carves the same): the hot part x,
@@ -974,15 +922,13 @@ int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D) {
   const TopoDev& T = ctx->topo;
   D = BlockDev{};
   D.T = T;
-  D.a_ops = ctx->d_ba.p;
-  D.b_ops = ctx->d_bb.p;
-  D.f_ops = ctx->d_bf.p;
-  D.a_rows = ctx->bprog.a_rows;
-  D.b_rows = ctx->bprog.b_rows;
-  D.f_rows = ctx->bprog.f_rows;
-  D.op_bytes = ctx->block_op_bytes;
-  D.row_k = ctx->bprog.row_k;
-  D.ring_bytes = block_ring_bytes(D.op_bytes, D.row_k);
+  auto program = [](BlockProgram& p, const DevBuf& d, const TaskStream& t) {
+    p.words = d.as<uint32_t>();
+    std::copy(std::begin(t.off), std::end(t.off), p.off);
+  };
+  program(D.a, ctx->d_ba, ctx->bprog.a);
+  program(D.b, ctx->d_bb, ctx->bprog.b);
+  program(D.f, ctx->d_bf, ctx->bprog.f);
   D.g_terms = ctx->d_bg_terms.as<uint32_t>();
   D.g_cells = ctx->d_bg_cells.as<uint4>();
   D.g_len = ctx->block_g_len;
@@ -990,13 +936,13 @@ int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D) {
   // The placement with the most CTAs an SM: the whole working set in shared
   // memory, its hot part there (the cold part in the slab), or all of it in
   // the slab; on a tie, the most in shared memory.
-  const bool long_ops = D.op_bytes == 16, b3 = topo_has_b3(T);
+  const bool b3 = topo_has_b3(T);
   int best = -1;
   uint32_t place = 2;
   for (uint32_t p = 0; p < 3; ++p) {
     block_layout(T, T.nv, mixed, p == 1, D);
-    if (p < 2 && D.lane_bytes + D.ring_bytes > kBlockSmemRoom) continue;
-    const int per_sm = block_occupancy(mixed, long_ops, b3, (p < 2 ? D.lane_bytes : 0) + D.ring_bytes);
+    if (p < 2 && D.lane_bytes > kBlockSmemRoom) continue;
+    const int per_sm = block_occupancy(mixed, b3, p < 2 ? D.lane_bytes : 0);
     if (per_sm > best) {
       best = per_sm;
       place = p;
@@ -1896,48 +1842,20 @@ int32_t group_block(esl_ctx* const* ctxs, uint32_t n_ctx, const esl_newton_opts*
   size_t smem = 0, stride = 16;
   for (uint32_t c = 0; c < n_ctx; ++c) {
     esl_ctx* x = ctxs[c];
-    // one op ring for the whole launch: rows of one op a thread for every
-    // topology (a slab topology's wider rows would size every CTA's ring
-    // for them); the context keeps these programs after the group
-    if (int32_t rc = ensure_block(x)) return rc;
-    if (x->bprog.row_k != 1) {
-      if (int32_t rc = set_block_programs(x, 1)) return rc;
-      ESL_CUDA(cudaStreamSynchronize(x->stream));
-    }
     if (int32_t rc = block_view(x, mixed, x->n_lanes, Ds[c])) return rc;
     if (Ds[c].refine_out) ESL_CUDA(cudaMemsetAsync(Ds[c].refine_out, 0, size_t(x->n_lanes) * 4, x->stream));
     ESL_CUDA(cudaStreamSynchronize(x->stream));
     b3 |= topo_has_b3(x->topo);
   }
-  // the group's own placement: the op ring of the widest op format after
-  // the working sets that fit shared memory within the group room
-  bool long_ops = false;
-  for (uint32_t c = 0; c < n_ctx; ++c) long_ops |= Ds[c].op_bytes == 16;
-  if (long_ops)
-    for (uint32_t c = 0; c < n_ctx; ++c)
-      if (Ds[c].op_bytes != 16) {
-        // one op format per launch: the long words for every topology
-        esl_ctx* x = ctxs[c];
-        ESL_CUDA(upload(x->d_ba, block_words(x->bprog.a_ops, false), x->stream));
-        ESL_CUDA(upload(x->d_bb, block_words(x->bprog.b_ops, false), x->stream));
-        ESL_CUDA(upload(x->d_bf, block_words(x->bprog.f_ops, false), x->stream));
-        ESL_CUDA(cudaStreamSynchronize(x->stream));
-        x->block_op_bytes = 16;
-        if (int32_t rc = block_view(x, mixed, x->n_lanes, Ds[c])) return rc;
-      }
-  uint32_t ring = 0;
-  for (uint32_t c = 0; c < n_ctx; ++c) ring = std::max(ring, block_ring_bytes(long_ops ? 16 : 8, Ds[c].row_k));
   std::vector<BlockDev> Dg = Ds;
   for (uint32_t c = 0; c < n_ctx; ++c) {
     // each topology keeps its own placement (block_view's), the whole
     // working set in the CTA's slab when its shared part misses the room
-    Dg[c].in_smem = Dg[c].in_smem && Dg[c].lane_bytes + ring <= kGroupSmemRoom;
+    Dg[c].in_smem = Dg[c].in_smem && Dg[c].lane_bytes <= kGroupSmemRoom;
     if (!Dg[c].in_smem && Dg[c].split) block_layout(ctxs[c]->topo, ctxs[c]->topo.nv, mixed, false, Dg[c]);
     if (Dg[c].in_smem) smem = std::max<size_t>(smem, Dg[c].lane_bytes);
     stride = std::max<size_t>(stride, Dg[c].split ? Dg[c].cold_bytes : Dg[c].in_smem ? 0 : Dg[c].lane_bytes);
   }
-  const uint32_t ring_at = uint32_t((smem + 15) & ~size_t(15));
-  smem = ring_at + ring;
   std::vector<uint32_t> order(n_ctx);
   for (uint32_t c = 0; c < n_ctx; ++c) order[c] = c;
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
@@ -1946,7 +1864,7 @@ int32_t group_block(esl_ctx* const* ctxs, uint32_t n_ctx, const esl_newton_opts*
   std::vector<uint2> items;
   for (uint32_t c : order)
     for (uint32_t l = 0; l < ctxs[c]->n_lanes; ++l) items.push_back(make_uint2(c, l));
-  const int per_sm = block_group_occupancy(mixed, long_ops, b3, smem);
+  const int per_sm = block_group_occupancy(mixed, b3, smem);
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(uint32_t(items.size()),
                                                                  uint32_t(c0->sms) * uint32_t(std::max(per_sm, 1))));
   cudaStream_t s = c0->stream;
@@ -1961,7 +1879,7 @@ int32_t group_block(esl_ctx* const* ctxs, uint32_t n_ctx, const esl_newton_opts*
   ESL_CUDA(launch_dc_block_group(c0->d_group_blocks.as<BlockDev>(), c0->d_group_lanes.as<LaneDev>(),
                                  c0->d_group_items.as<uint2>(), uint32_t(items.size()),
                                  c0->d_next_lane.as<uint32_t>(), o, c0->d_group_slab.as<unsigned char>(), stride,
-                                 smem, ring_at, grid, mixed, long_ops, b3, s));
+                                 smem, grid, mixed, b3, s));
   ESL_CUDA(cudaEventRecord(c0->ev1, s));
   ESL_CUDA(cudaEventSynchronize(c0->ev1));
   float ms = 0;
@@ -2127,9 +2045,9 @@ int32_t esl_block_info(esl_ctx* ctx, esl_block_info_t* info) {
   if (int32_t rc = ensure_block(ctx)) return rc;
   std::memset(info, 0, sizeof(*info));
   info->width = kBlockThreads;
-  info->a_rows = ctx->bprog.a_rows;
-  info->b_rows = ctx->bprog.b_rows;
-  info->f_rows = ctx->bprog.f_rows;
+  info->a_rows = ctx->bprog.a.rows;
+  info->b_rows = ctx->bprog.b.rows;
+  info->f_rows = ctx->bprog.f.rows;
   info->a_levels = ctx->bprog.a_levels;
   info->a_nops = ctx->prog.a_nops;
   info->b_nops = ctx->prog.b_nops;
@@ -2141,8 +2059,7 @@ int32_t esl_block_info(esl_ctx* ctx, esl_block_info_t* info) {
     info->lane_bytes[m] = D.lane_bytes;
     info->in_smem[m] = D.in_smem;
     info->ctas_per_sm[m] = uint32_t(std::max(
-        0, block_occupancy(m == 1, D.op_bytes == 16, topo_has_b3(ctx->topo),
-                           (D.in_smem ? D.lane_bytes : 0) + D.ring_bytes)));
+        0, block_occupancy(m == 1, topo_has_b3(ctx->topo), D.in_smem ? D.lane_bytes : 0)));
     info->split[m] = D.split;
     info->cold_bytes[m] = D.cold_bytes;
     info->gather_terms = D.g_len;

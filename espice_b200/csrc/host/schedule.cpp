@@ -119,11 +119,6 @@ void pack(const std::vector<SeqOp>& seq, uint32_t space, std::vector<Op>& rows, 
             encode(kOpSubNz, space - 1, space - 2, space - 3), rows, n_rows, n_levels);
 }
 
-// Block-lane ops: 32-bit value indices, padding as no-ops.
-Op4 encode4(const SeqOp& s) {
-  return Op4{s.dst | (s.kind << 28), s.a == kNone ? 0u : s.a, s.b == kNone ? 0u : s.b, 0u};
-}
-
 }  // namespace
 
 Programs compile_tape(const SparseLu& lu) {
@@ -215,22 +210,249 @@ std::vector<SeqOp> unpack(const std::vector<Op4>& ops) {
   return out;
 }
 
+// Estimated cycles of a task's parts, for the longest-path priorities: an
+// update, a division, and the step from one row to the next.
+constexpr int kCostOp = 12, kCostDiv = 115, kCostRow = 75;
+// A task far from the critical path (its longest path kSlack cycles shorter
+// than the longest in the ready list) waits until kTaskOps updates, or its
+// last ones, can run at once.
+constexpr int kSlack = 300;
+
+// Packs a sequential program into task rows. Every value's updates are one
+// list in sequential order; a value is read by other values only once its
+// list has run (the column replay and the triangular solves read finished
+// entries only), so a task, the next updates of one value, may run as soon
+// as their operands are finished in earlier rows. Row by row, the ready
+// tasks of the longest remaining paths run, up to one per thread of the
+// CTA; tasks with a division, then by updates, then by value (a column's
+// entries side by side: their multiplier is one broadcast, their other
+// operands neighbours) share a warp. A row of at most 32 tasks is warp 0's
+// alone, and between two such rows no CTA barrier is needed.
+// Against rows of single ops (434 rows for the 498-unknown analog block's
+// refactor, 233 for its back solve) a task keeps its value in a register
+// over its updates and its division: 176 and 101 rows, and 3 loads an update
+// in place of 4 accesses.
+TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv) {
+  const uint32_t sink = nv - 1, one = nv - 2, zero = nv - 3;
+  const size_t n = seq.size();
+  // vop[vptr[v] .. vptr[v + 1]): the ops of value v
+  std::vector<uint32_t> vptr(nv + 1, 0), vop(n), at_op(n);
+  for (const SeqOp& o : seq) ++vptr[o.dst + 1];
+  for (uint32_t v = 0; v < nv; ++v) vptr[v + 1] += vptr[v];
+  {
+    std::vector<uint32_t> at(vptr.begin(), vptr.end() - 1);
+    for (size_t i = 0; i < n; ++i) {
+      at_op[i] = at[seq[i].dst];
+      vop[at[seq[i].dst]++] = uint32_t(i);
+    }
+  }
+  auto divides = [&](uint32_t v) { return is_div(seq[vop[vptr[v + 1] - 1]].kind); };
+  // cycles from op `pos` of value v to its end
+  auto rest = [&](uint32_t v, uint32_t pos) {
+    const uint32_t left = vptr[v + 1] - pos;
+    const bool d = divides(v);
+    return int(left - (d ? 1u : 0u)) * kCostOp + (d ? kCostDiv : 0);
+  };
+  // tail[v]: the longest path from v's end to the program's
+  std::vector<int> tail(nv, 0);
+  for (size_t i = n; i-- > 0;) {
+    const SeqOp& o = seq[i];
+    const int path = kCostRow + rest(o.dst, at_op[i]) + tail[o.dst];
+    for (uint32_t s : {o.a, o.b})
+      if (s != kNone && s != o.dst) tail[s] = std::max(tail[s], path);
+  }
+  std::vector<uint32_t> pos(vptr.begin(), vptr.end() - 1), ready(pos);  // next op; ops before ready[v] can run
+  std::vector<uint8_t> done(nv, 0), queued(nv, 0);
+  for (uint32_t v = 0; v < nv; ++v) done[v] = vptr[v] == vptr[v + 1];
+  std::vector<std::vector<uint32_t>> waiting(nv);
+  auto advance = [&](uint32_t v) {
+    for (; ready[v] < vptr[v + 1]; ++ready[v]) {
+      const SeqOp& o = seq[vop[ready[v]]];
+      for (uint32_t s : {o.a, o.b})
+        if (s != kNone && s != v && !done[s]) {
+          waiting[s].push_back(v);
+          return;
+        }
+    }
+  };
+  std::vector<std::pair<int, uint32_t>> queue;
+  auto push = [&](uint32_t v) {
+    queue.push_back({rest(v, pos[v]) + tail[v], v});
+    std::push_heap(queue.begin(), queue.end());
+  };
+  auto offer = [&](uint32_t v) {
+    if (queued[v] || ready[v] == pos[v]) return;
+    queued[v] = 1;
+    push(v);
+  };
+  for (uint32_t v = 0; v < nv; ++v)
+    if (!done[v]) {
+      advance(v);
+      offer(v);
+    }
+  struct Task {
+    uint32_t v, lo, ops;  // ops updates from vop[lo], then the division when div
+    bool div;
+  };
+  auto take = [&](uint32_t v) {
+    const uint32_t run = ready[v] - pos[v];
+    const bool last = ready[v] == vptr[v + 1] && divides(v);
+    Task t{v, pos[v], std::min(run - (last ? 1u : 0u), kTaskOps), false};
+    t.div = last && t.ops + 1 == run;
+    return t;
+  };
+  std::vector<uint32_t> out[kTaskWarps];
+  uint32_t idle[kTaskWarps] = {};
+  uint32_t lane_words[32][kTaskWords];
+  auto put = [&](uint32_t w) {
+    for (int h = 0; h < 2; ++h)
+      for (int l = 0; l < 32; ++l)
+        for (int j = 0; j < 4; ++j) out[w].push_back(lane_words[l][4 * h + j]);
+  };
+  auto put_idle = [&](uint32_t w, uint32_t barriers) {
+    for (auto& l : lane_words) {
+      std::fill(std::begin(l), std::end(l), 0u);
+      l[0] = kTaskIdle;
+      l[1] = barriers;
+    }
+    put(w);
+  };
+  auto flush = [&](uint32_t w) {
+    if (idle[w]) put_idle(w, idle[w]);
+    idle[w] = 0;
+  };
+  TaskStream S;
+  // One row's tasks onto the warps; `cta`: a CTA barrier follows.
+  auto emit = [&](const std::vector<Task>& row, bool cta) {
+    for (uint32_t w = 0; w < kTaskWarps; ++w) {
+      if (32 * w >= row.size()) {
+        idle[w] += cta;
+        continue;
+      }
+      flush(w);
+      const size_t t0 = 32 * size_t(w), nt = std::min<size_t>(32, row.size() - t0);
+      uint32_t most = 0;
+      bool any_div = false;
+      for (size_t l = 0; l < nt; ++l) {
+        most = std::max(most, row[t0 + l].ops);
+        any_div |= row[t0 + l].div;
+      }
+      for (uint32_t l = 0; l < 32; ++l) {
+        uint32_t* x = lane_words[l];
+        x[0] = sink | (most > 1 ? kTaskMore : 0u) | (cta ? kTaskCta : 0u);
+        x[1] = one | (any_div ? kTaskDivAny : 0u);
+        for (uint32_t j = 0; j < kTaskOps; ++j) {
+          x[2 + 2 * j] = zero;
+          x[3 + 2 * j] = one;
+        }
+        if (l >= nt) continue;
+        const Task& t = row[t0 + l];
+        x[0] = (x[0] & ~kTaskIndex) | t.v;
+        for (uint32_t j = 0; j < t.ops; ++j) {
+          const SeqOp& o = seq[vop[t.lo + j]];
+          x[2 + 2 * j] = o.a;
+          x[3 + 2 * j] = o.b;
+          if (o.kind == kOpSubNz) x[0] |= kTaskNz;
+        }
+        if (t.div) {
+          const SeqOp& o = seq[vop[t.lo + t.ops]];
+          x[0] |= kTaskDiv;
+          x[1] = o.a | kTaskDivAny | (o.kind == kOpDivGrowth ? kTaskGrowth : 0u) |
+                 (o.kind == kOpDivScaled ? kTaskScaled : 0u);
+        }
+      }
+      put(w);
+    }
+    ++S.rows;
+  };
+  std::vector<Task> row, prev;
+  std::vector<uint32_t> later, finished;
+  size_t left = n;
+  while (left) {
+    row.clear();
+    later.clear();
+    const int top = queue.front().first;
+    while (!queue.empty() && row.size() < 32 * kTaskWarps) {
+      std::pop_heap(queue.begin(), queue.end());
+      const uint32_t v = queue.back().second;
+      const int path = queue.back().first;
+      queue.pop_back();
+      if (path < top - kSlack && ready[v] < vptr[v + 1] && ready[v] - pos[v] < kTaskOps) {
+        later.push_back(v);
+        continue;
+      }
+      queued[v] = 0;
+      row.push_back(take(v));
+    }
+    for (uint32_t v : later) push(v);
+    std::sort(row.begin(), row.end(), [&](const Task& x, const Task& y) {
+      if (row.size() > 32) {
+        if (x.div != y.div) return x.div;
+        if ((x.ops > 1) != (y.ops > 1)) return x.ops > 1;
+      }
+      return x.v < y.v;
+    });
+    // the row before goes out once it is known whether this one is warp 0's
+    if (!prev.empty()) emit(prev, prev.size() > 32 || row.size() > 32);
+    finished.clear();
+    for (const Task& t : row) {
+      const uint32_t k = t.ops + (t.div ? 1u : 0u);
+      pos[t.v] += k;
+      left -= k;
+      if (pos[t.v] == vptr[t.v + 1]) finished.push_back(t.v);
+    }
+    for (uint32_t v : finished) done[v] = 1;
+    for (uint32_t v : finished) {
+      const std::vector<uint32_t> w = std::move(waiting[v]);
+      for (uint32_t x : w) {
+        advance(x);
+        offer(x);
+      }
+    }
+    for (const Task& t : row) offer(t.v);
+    prev.swap(row);
+  }
+  if (!prev.empty()) emit(prev, true);
+  size_t total = 0;
+  for (uint32_t w = 0; w < kTaskWarps; ++w) {
+    flush(w);
+    constexpr size_t kChunk = 32 * kTaskWords;
+    const size_t have = out[w].size() / kChunk;
+    const size_t want = (have + kTaskUnroll - 1) / kTaskUnroll * kTaskUnroll + kTaskUnroll;
+    for (size_t c = have; c < want; ++c) put_idle(w, 0u);
+    total += out[w].size();
+    S.off[w + 1] = uint32_t(total / kChunk);
+  }
+  S.words.reserve(total);
+  for (auto& o : out) {
+    S.words.insert(S.words.end(), o.begin(), o.end());
+    std::vector<uint32_t>().swap(o);
+  }
+  return S;
+}
+
 }  // namespace
 
-BlockPrograms compile_block(const Programs& P, uint32_t width) {
+BlockPrograms compile_block(const Programs& P) {
   BlockPrograms B;
-  B.width = width;
-  const Op4 nop{uint32_t(kOpNop) << 28, 0u, 0u, 0u};
   const std::vector<SeqOp> a = unpack(P.a_seq), b = unpack(P.b_seq);
-  uint32_t lv = 0;
-  pack_rows(a, P.nv, width, encode4, nop, nop, B.a_ops, B.a_rows, B.a_levels);
-  pack_rows(b, P.nv, width, encode4, nop, nop, B.b_ops, B.b_rows, lv);
+  B.a = pack_tasks(a, P.nv);
+  B.b = pack_tasks(b, P.nv);
   // the forward substitution alone (program A's solve ops), for the mixed
   // form's refinement corrections on the finished factors
   std::vector<SeqOp> f;
   for (const SeqOp& s : a)
     if (s.kind == kOpSubNz) f.push_back(s);
-  pack_rows(f, P.nv, width, encode4, nop, nop, B.f_ops, B.f_rows, lv);
+  B.f = pack_tasks(f, P.nv);
+  // the longest dependence chain of single ops
+  std::vector<uint32_t> level(P.nv, 0);
+  for (const SeqOp& s : a) {
+    uint32_t l = level[s.dst];
+    for (uint32_t x : {s.a, s.b})
+      if (x != kNone) l = std::max(l, level[x]);
+    level[s.dst] = l + 1;
+    B.a_levels = std::max(B.a_levels, l + 1);
+  }
   return B;
 }
 

@@ -24,8 +24,8 @@ struct Op {
   uint32_t w0, w1;  // see common.h OpKind
 };
 
-// A block-lane op: w0 = dst | (kind << 28), then the two sources as full
-// 32-bit value indices (any tape size), 16 bytes for one vector load.
+// The same with full 32-bit value indices (any tape size): w0 = dst | (kind
+// << 28), then the two sources.
 struct Op4 {
   uint32_t w0, a, b, pad;
 };
@@ -46,15 +46,23 @@ struct Programs {
   bool has_void = false;
 };
 
-// The programs of a block lane: the same dependences list-scheduled into
-// rows of `width` ops (one per thread of the lane's CTA, a barrier between
-// rows), padding as no-ops, plus program F, the forward substitution alone
-// (the mixed form's refinement solves on finished factors).
+// A block-lane program as each warp's stream of chunks, a chunk the 32 tasks
+// (common.h) its lanes run between two barriers: warp w's chunks are
+// off[w] .. off[w + 1] (in chunks of 32 * kTaskWords words), a multiple of
+// kTaskUnroll and then kTaskUnroll that are only read ahead.
+constexpr uint32_t kTaskWarps = 8;
+struct TaskStream {
+  std::vector<uint32_t> words;
+  uint32_t off[kTaskWarps + 1] = {};
+  uint32_t rows = 0;  // steps between barriers (a warp's or the CTA's)
+};
+
+// The programs of a block lane: A (refactor + forward solve), B (back
+// solve) and F, the forward substitution alone (the mixed form's refinement
+// solves on finished factors).
 struct BlockPrograms {
-  uint32_t width = 0;  // ops a row: row_k * the CTA's threads
-  uint32_t row_k = 1;  // ops a thread a row
-  std::vector<Op4> a_ops, b_ops, f_ops;
-  uint32_t a_rows = 0, b_rows = 0, f_rows = 0, a_levels = 0;
+  TaskStream a, b, f;
+  uint32_t a_levels = 0;
 };
 
 // Every op reads final operands and every value's updates keep their
@@ -62,9 +70,8 @@ struct BlockPrograms {
 // sparse triangular solves.
 Programs compile_tape(const SparseLu& lu);
 
-// Rows of `width` for the block lanes (the warp programs, a_ops and b_ops,
-// exist only when the value space fits 16-bit indices: nv < 65536).
-BlockPrograms compile_block(const Programs& P, uint32_t width);
+// The block lanes' task streams.
+BlockPrograms compile_block(const Programs& P);
 
 constexpr uint32_t kRow = 32;
 

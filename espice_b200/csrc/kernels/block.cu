@@ -3,11 +3,10 @@
 // thousands of unknowns). One CTA owns a lane for its whole solve, every
 // phase in one persistent launch, as the warp lanes do (newton.cu); what
 // changes is the width: eval strides over the CTA's threads, the tape
-// programs are rows of one op per thread (a CTA barrier between rows), and
-// reductions run across the CTA. Nothing per topology is staged: the
+// programs are rows of one task per thread (tasks.cuh), and reductions run
+// across the CTA. Nothing per topology is staged: the
 // programs (L2-resident, shared by every lane of the topology) stream in,
-// each thread copying its own op words 4 rows ahead
-// into a private ring in shared memory with cp.async, and the assembly is a
+// each thread reading its own task words chunks ahead, and the assembly is a
 // per-thread stream of staging indices read eight terms ahead, so neither
 // waits on an L2 round trip per row or per term.
 //
@@ -39,6 +38,7 @@
 #include "block.h"
 #include "lane_eval.cuh"
 #include "ladder.cuh"
+#include "tasks.cuh"
 #include "tran_core.cuh"
 
 namespace esl {
@@ -87,175 +87,8 @@ __device__ __forceinline__ double block_fmax(double v, uint64_t* red) {
   return r;
 }
 
-// The op's arithmetic in the lane's precision, rounded as the CPU replay
-// rounds (FP64: bitwise; FP32: the same order in FP32).
-__device__ __forceinline__ double op_div(double b, double a) { return div_rn(b, a); }
-__device__ __forceinline__ float op_div(float b, float a) { return __fdiv_rn(b, a); }
-__device__ __forceinline__ double op_msub(double d, double a, double b) { return __dsub_rn(d, __dmul_rn(a, b)); }
-__device__ __forceinline__ float op_msub(float d, float a, float b) { return __fsub_rn(d, __fmul_rn(a, b)); }
-__device__ __forceinline__ double growth(double) { return 1e-12; }
-__device__ __forceinline__ float growth(float) { return 1e-12f; }
 __device__ __forceinline__ double inf_of(double) { return CUDART_INF; }
 __device__ __forceinline__ float inf_of(float) { return CUDART_INF_F; }
-
-// One op of a row (thread-local): a division with its pivot checks, or a
-// multiply-subtract (the solves skip a zero multiplier, the refactor never
-// does); no-ops pad the row. Returns true on a failed pivot test.
-template <typename V>
-__device__ __forceinline__ bool run_op(const uint4& op, V* v) {
-  const uint32_t kind = op.x >> 28;
-  if (kind == kOpNop) return false;
-  V* pd = v + (op.x & 0x0fffffffu);
-  const V a = v[op.y], b = v[op.z];
-  if (kind == kOpDivGrowth || kind == kOpDivScaled || kind == kOpDivY) {
-    const V q = op_div(b, a);
-    *pd = q;
-    if (kind == kOpDivGrowth) return !(fabs(a) >= growth(a) * fabs(b));
-    if (kind == kOpDivScaled) return !(fabs(q) < inf_of(q));
-    return false;
-  }
-  const V d = *pd;
-  if (kind == kOpFlop || b != V(0)) *pd = op_msub(d, a, b);
-  return false;
-}
-
-// K independent ops of one row: every operand loaded first, then the
-// results computed and stored in op order (run_op's arithmetic and checks).
-template <typename V, uint32_t K>
-__device__ __forceinline__ bool run_ops(const uint4 (&op)[K], V* v) {
-  V a[K], b[K], d[K];
-#pragma unroll
-  for (uint32_t j = 0; j < K; ++j) {
-    const uint32_t kind = op[j].x >> 28;
-    if (kind != kOpNop) {
-      a[j] = v[op[j].y];
-      b[j] = v[op[j].z];
-      d[j] = v[op[j].x & 0x0fffffffu];
-    }
-  }
-  bool bad = false;
-#pragma unroll
-  for (uint32_t j = 0; j < K; ++j) {
-    const uint32_t kind = op[j].x >> 28;
-    if (kind == kOpNop) continue;
-    V* pd = v + (op[j].x & 0x0fffffffu);
-    if (kind == kOpDivGrowth || kind == kOpDivScaled || kind == kOpDivY) {
-      const V q = op_div(b[j], a[j]);
-      *pd = q;
-      if (kind == kOpDivGrowth) bad |= !(fabs(a[j]) >= growth(a[j]) * fabs(b[j]));
-      if (kind == kOpDivScaled) bad |= !(fabs(q) < inf_of(q));
-    } else if (kind == kOpFlop || b[j] != V(0)) {
-      *pd = op_msub(d[j], a[j], b[j]);
-    }
-  }
-  return bad;
-}
-
-// Op words: 8 bytes {dst | kind << 28, a | b << 16} when the value space
-// has 16-bit indices, 16 bytes {dst | kind << 28, a, b, 0} otherwise. A
-// thread's ring holds kDepth + 1 op words (10 or 20 KB a CTA): kDepth rows
-// in flight (about 1,500 cycles ahead, past an L2 round trip), and the slot
-// being refilled is
-// never the one being read.
-template <typename OpT>
-struct OpFormat;
-template <>
-struct OpFormat<uint2> {
-  static constexpr uint32_t kDepth = 4;
-  __device__ static uint4 decode(uint2 o) { return make_uint4(o.x, o.y & 0xffffu, o.y >> 16, 0u); }
-};
-template <>
-struct OpFormat<uint4> {
-  static constexpr uint32_t kDepth = 4;
-  __device__ static uint4 decode(uint4 o) { return o; }
-};
-
-__device__ __forceinline__ void ring_copy(uint32_t dst, const void* src, uint32_t bytes) {
-  if (bytes == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-  else asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void ring_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void ring_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ uint2 ld_ring(uint32_t a, uint2*) {
-  uint2 r;
-  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(a));
-  return r;
-}
-__device__ __forceinline__ uint4 ld_ring(uint32_t a, uint4*) {
-  uint4 r;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(a));
-  return r;
-}
-
-// Runs a program over v: row r holds K * kW ops, this thread's are
-// ops[(r * K + j) * kW + tid] for j < K; a CTA barrier after each row. The
-// ops of a row are independent (no op reads or writes a value another op of
-// the row writes), so a thread loads the operands of all K before it stores
-// any: K loads in flight per thread, the rows' latency paid once per K ops.
-// Each thread keeps its next kDepth rows of op words in flight through its
-// ring (slot s at ring + s * K * kW * sizeof(OpT), op j of the slot
-// j * kW * sizeof(OpT) further, one commit group per row), so a row waits
-// only for its own op words, copied kDepth rows earlier. K = 1 (rows of kW
-// ops, 4 rows ahead) for working sets in shared memory; K = kSlabRowOps (2
-// rows ahead) for working sets in the CTA's global slab, whose operand
-// loads are L2 and HBM round trips. Returns this thread's pivot-test
-// failures.
-template <typename V, typename OpT, uint32_t kW, uint32_t K>
-__device__ bool block_rows_k(const OpT* __restrict__ ops, uint32_t rows, V* v, uint32_t ring, int tid) {
-  constexpr uint32_t D = K == 1 ? OpFormat<OpT>::kDepth : 2u, kSlot = K * kW * sizeof(OpT);
-  constexpr uint32_t kStep = kW * sizeof(OpT);
-  for (uint32_t d = 0; d < D; ++d) {
-    if (d < rows)
-#pragma unroll
-      for (uint32_t j = 0; j < K; ++j)
-        ring_copy(ring + d * kSlot + j * kStep, ops + (size_t(d) * K + j) * kW + tid, sizeof(OpT));
-    ring_commit();
-  }
-  bool bad = false;
-  uint32_t slot = 0, fill = D;  // the slot of row r, of row r + D
-  for (uint32_t r = 0; r < rows; ++r) {
-    ring_wait<D - 1>();  // row r's group has landed
-    if constexpr (K == 1) {
-      const uint4 op = OpFormat<OpT>::decode(ld_ring(ring + slot * kSlot, static_cast<OpT*>(nullptr)));
-      if (r + D < rows) ring_copy(ring + fill * kSlot, ops + size_t(r + D) * kW + tid, sizeof(OpT));
-      ring_commit();
-      bad |= run_op(op, v);
-    } else {
-      uint4 op[K];
-#pragma unroll
-      for (uint32_t j = 0; j < K; ++j)
-        op[j] = OpFormat<OpT>::decode(ld_ring(ring + slot * kSlot + j * kStep, static_cast<OpT*>(nullptr)));
-      if (r + D < rows)
-#pragma unroll
-        for (uint32_t j = 0; j < K; ++j)
-          ring_copy(ring + fill * kSlot + j * kStep, ops + (size_t(r + D) * K + j) * kW + tid, sizeof(OpT));
-      ring_commit();
-      bad |= run_ops<V, K>(op, v);
-    }
-    slot = slot == D ? 0 : slot + 1;
-    fill = fill == D ? 0 : fill + 1;
-    __syncthreads();
-  }
-  ring_wait<0>();
-  return bad;
-}
-
-// The wide rows out of line: their K operand sets would otherwise raise the
-// register pressure of every kernel that inlines the one-op rows.
-template <typename V, typename OpT, uint32_t kW>
-__device__ __noinline__ bool block_rows_wide(const OpT* __restrict__ ops, uint32_t rows, V* v, uint32_t ring,
-                                             int tid) {
-  return block_rows_k<V, OpT, kW, kSlabRowOps>(ops, rows, v, ring, tid);
-}
-
-template <typename V, typename OpT, uint32_t kW>
-__device__ bool block_rows(const OpT* __restrict__ ops, uint32_t rows, V* v, uint32_t ring, int tid, uint32_t k) {
-  if (k == kSlabRowOps) return block_rows_wide<V, OpT, kW>(ops, rows, v, ring, tid);
-  return block_rows_k<V, OpT, kW, 1>(ops, rows, v, ring, tid);
-}
 
 // The lane's views into its working set.
 template <typename V>
@@ -265,14 +98,12 @@ struct BlockMem {
   double* a64;  // nnz: the assembled matrix in FP64 (mixed form only)
   V* v;         // tape values | y | 0.0 | 1.0 | sink
   V* y;
-  uint32_t ring;  // this thread's op ring (shared address of its slot 0)
 };
 
 // base: the working set (its hot part when split); cold: the CTA's slab
 // for a split layout's cold part.
 template <typename V>
-__device__ __forceinline__ BlockMem<V> block_carve(const BlockDev& D, unsigned char* base, unsigned char* cold,
-                                                  unsigned char* ring = nullptr, uint32_t op_bytes = 8) {
+__device__ __forceinline__ BlockMem<V> block_carve(const BlockDev& D, unsigned char* base, unsigned char* cold) {
   BlockMem<V> b;
   unsigned char* cbase = D.split ? cold : base;
   b.m.base = reinterpret_cast<double*>(base);
@@ -288,7 +119,6 @@ __device__ __forceinline__ BlockMem<V> block_carve(const BlockDev& D, unsigned c
   b.a64 = reinterpret_cast<double*>(base + D.o_a64);
   b.v = reinterpret_cast<V*>(base + D.o_v);
   b.y = b.v + D.T.ntv;
-  b.ring = ring ? static_cast<uint32_t>(__cvta_generic_to_shared(ring)) + threadIdx.x * op_bytes : 0u;
   return b;
 }
 
@@ -379,13 +209,22 @@ __device__ void block_assemble(const BlockDev& D, const BlockMem<V>& b, double g
   for (uint32_t j = tid; j < T.n_fill; j += kW) b.v[T.fill[j]] = V(0);
 }
 
+// One of the programs over the lane's values; this thread's pivot-test
+// failures. Ends in a CTA barrier (a program without tasks has none).
+template <typename V>
+__device__ __forceinline__ bool block_program(const BlockDev& D, const BlockProgram& p, V* v) {
+  const uint32_t w = threadIdx.x >> 5, first = p.off[w], chunks = p.off[w + 1] - first - kTaskUnroll;
+  return (D.in_smem ? run_tasks<V, true>(p.words, first, chunks, v) : run_tasks<V, false>(p.words, first, chunks, v)) !=
+         0;
+}
+
 // Refactor + forward solve (program A), then the lane kernels' peel tests on
 // the finished tape values (lane_kernels.zig Bodies.refactor and
 // LaneSolver.wideMultipliers). CTA-uniform verdict.
-template <typename V, typename OpT, uint32_t kW>
-__device__ bool block_refactor(const BlockDev& D, V* v, uint32_t ring, int tid) {
+template <typename V, uint32_t kW>
+__device__ bool block_refactor(const BlockDev& D, V* v, int tid) {
   const TopoDev& T = D.T;
-  bool bad = block_rows<V, OpT, kW>(static_cast<const OpT*>(D.a_ops), D.a_rows, v, ring, tid, D.row_k);
+  bool bad = block_program(D, D.a, v);
   const uint32_t l0 = T.nu + T.n;
   for (uint32_t s = tid; s < T.nu; s += kW)
     if (!(fabs(v[s]) < inf_of(v[s]))) bad = true;
@@ -403,7 +242,7 @@ __device__ bool block_refactor(const BlockDev& D, V* v, uint32_t ring, int tid) 
 // stop when max |res| <= tol * max |rhs| or after refine_max corrections;
 // each correction solved on the FP32 factors (program F then program B)
 // and added to dx in FP64. Returns the corrections made.
-template <typename OpT, uint32_t kW>
+template <uint32_t kW>
 __device__ uint32_t block_refine(const BlockDev& D, const BlockMem<float>& b, uint64_t* red, int tid) {
   const TopoDev& T = D.T;
   uint32_t made = 0;
@@ -421,8 +260,8 @@ __device__ uint32_t block_refine(const BlockDev& D, const BlockMem<float>& b, ui
     rmax = block_max_abs<kW>(rmax, red);
     bmax = block_max_abs<kW>(bmax, red);
     if (!(rmax > D.refine_tol * bmax) || it >= D.refine_max) break;
-    block_rows<float, OpT, kW>(static_cast<const OpT*>(D.f_ops), D.f_rows, b.v, b.ring, tid, D.row_k);
-    block_rows<float, OpT, kW>(static_cast<const OpT*>(D.b_ops), D.b_rows, b.v, b.ring, tid, D.row_k);
+    block_program(D, D.f, b.v);
+    block_program(D, D.b, b.v);
     for (uint32_t j = tid; j < T.n; j += kW) {
       const uint32_t i = T.qcol[j];
       b.dx[i] = __dadd_rn(b.dx[i], double(b.y[j]));
@@ -439,7 +278,7 @@ __device__ uint32_t block_refine(const BlockDev& D, const BlockMem<float>& b, ui
 // test (a step farther out is taken as an inexact Newton step: its FP32
 // error, about 1e-7 of the step, is far below what the next iterate still
 // corrects). Returns the corrections made.
-template <typename OpT, uint32_t kW>
+template <uint32_t kW>
 __device__ uint32_t block_refine_step(const BlockDev& D, const BlockMem<float>& b, const LaneOpts& o, uint64_t* red,
                                       int tid) {
   const TopoDev& T = D.T;
@@ -454,7 +293,7 @@ __device__ uint32_t block_refine_step(const BlockDev& D, const BlockMem<float>& 
     }
     if (from_bits(block_max_bits<kW>(q, red)) > D.refine_skip) return 0;
   }
-  return block_refine<OpT, kW>(D, b, red, tid);
+  return block_refine<kW>(D, b, red, tid);
 }
 
 // Phase profile: thread 0 adds the cycles since `t` to prof[phase] and
@@ -470,10 +309,9 @@ __device__ __forceinline__ void phase_mark(unsigned long long* prof, uint32_t ph
 // One lane's DC Newton solve (converger.zig newtonLanes at W = 1 with the
 // lane's own direct solver), by the CTA that owns it: the warp lanes'
 // dc_solve_lane step for step, reductions across the CTA.
-template <typename V, typename OpT, bool kHasB3, uint32_t kW, bool kLadder = false>
+template <typename V, bool kHasB3, uint32_t kW, bool kLadder = false>
 __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& o, unsigned char* base,
-                           unsigned char* cold, unsigned char* ring, uint64_t* red, uint32_t lane,
-                           const LadderDev* ld = nullptr) {
+                           unsigned char* cold, uint64_t* red, uint32_t lane, const LadderDev* ld = nullptr) {
   constexpr bool kMixed = sizeof(V) == 4;
   const TopoDev& T = D.T;
   const int tid = threadIdx.x;
@@ -482,7 +320,7 @@ __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& 
   if (!(status == kRunning || resuming)) return;
 
   const uint32_t n = T.n;
-  const BlockMem<V> b = block_carve<V>(D, base, cold, ring, sizeof(OpT));
+  const BlockMem<V> b = block_carve<V>(D, base, cold);
   const LaneMem& m = b.m;
   const double* rec = L.rec + size_t(lane) * T.rec_size;
   for (uint32_t i = tid; i < n; i += kW) m.x[i] = L.x[size_t(lane) * n + i];
@@ -546,7 +384,7 @@ __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& 
       }
       const bool host_mode = (flags & 2u) != 0;
       bool bad = true;
-      if (!host_mode) bad = block_refactor<V, OpT, kW>(D, b.v, b.ring, tid);
+      if (!host_mode) bad = block_refactor<V, kW>(D, b.v, tid);
       phase_mark(D.prof, kBlockPhaseRefactor, t0);
       if (bad) {
         // Pause: the host factors this lane with its own FP64 direct solver.
@@ -569,12 +407,12 @@ __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& 
         }
         return;
       }
-      block_rows<V, OpT, kW>(static_cast<const OpT*>(D.b_ops), D.b_rows, b.v, b.ring, tid, D.row_k);
+      block_program(D, D.b, b.v);
       for (uint32_t j = tid; j < n; j += kW) b.dx[T.qcol[j]] = double(b.y[j]);
       __syncthreads();
       phase_mark(D.prof, kBlockPhaseSolve, t0);
       if constexpr (kMixed) {
-        refinements += block_refine_step<OpT, kW>(D, b, o, red, tid);
+        refinements += block_refine_step<kW>(D, b, o, red, tid);
         phase_mark(D.prof, kBlockPhaseRefine, t0);
       }
     }
@@ -639,26 +477,25 @@ __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& 
 // Persistent grid: each CTA takes lanes blockIdx.x, + gridDim.x, ...; its
 // working set in dynamic shared memory, split between shared memory and its
 // slab of D.slab, or all in its slab. Dynamic shared memory: the working set
-// (its hot part when split; nothing when all in the slab), then the op ring.
+// (its hot part when split; nothing when all in the slab).
 // Two CTAs an SM by registers (the BSIM3 instantiation spills a few words
 // of its evaluation for it), as many as shared memory then allows.
-template <typename V, typename OpT, bool kHasB3, uint32_t kW, bool kLadder>
+template <typename V, bool kHasB3, uint32_t kW, bool kLadder>
 __global__ void __launch_bounds__(kW, 2) dc_block_kernel(BlockDev D, LaneDev L, LaneOpts o) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t red[kW / 32];
   unsigned char* own = D.slab + size_t(blockIdx.x) * (D.split ? D.cold_bytes : D.lane_bytes);
   unsigned char* base = D.in_smem ? smem_raw : own;
-  unsigned char* ring = smem_raw + (D.in_smem ? D.lane_bytes : 0u);
   for (uint32_t lane = blockIdx.x; lane < L.n_lanes; lane += gridDim.x) {
     if constexpr (!kLadder) {
-      block_lane<V, OpT, kHasB3, kW>(D, L, o, base, own, ring, red, lane);
+      block_lane<V, kHasB3, kW>(D, L, o, base, own, red, lane);
     } else {
       // an operating-point lane runs Newton until the ladder is done or the
       // lane pauses for a host factor (a singular host factor ends a run)
       for (;;) {
         const uint32_t st = *(volatile uint32_t*)(L.status + lane);
         if (st == kRunning || (L.resume && st == kNeedSolve)) {
-          block_lane<V, OpT, kHasB3, kW, true>(D, L, o, base, own, ring, red, lane, L.ladder + lane);
+          block_lane<V, kHasB3, kW, true>(D, L, o, base, own, red, lane, L.ladder + lane);
           __syncthreads();
           if (*(volatile uint32_t*)(L.status + lane) == kNeedSolve) break;
         } else if (!(st == kSingular && L.ladder[lane].rung != kRungDone)) {
@@ -678,12 +515,11 @@ __global__ void __launch_bounds__(kW, 2) dc_block_kernel(BlockDev D, LaneDev L, 
 // copies that topology's tables into shared memory and solves the lane with
 // its working set in dynamic shared memory (when the topology's fits) or in
 // the CTA's slab. Every topology of a group runs in one precision and width.
-template <typename V, typename OpT, bool kHasB3, uint32_t kW>
+template <typename V, bool kHasB3, uint32_t kW>
 __global__ void __launch_bounds__(kW, 2) dc_block_group_kernel(const BlockDev* __restrict__ Ds,
                                                             const LaneDev* __restrict__ Ls, const uint2* items,
                                                             uint32_t n_items, uint32_t* next, LaneOpts o,
-                                                            unsigned char* slab, size_t slab_stride,
-                                                            uint32_t ring_at) {
+                                                            unsigned char* slab, size_t slab_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t red[kW / 32];
   __shared__ BlockDev D;
@@ -701,8 +537,7 @@ __global__ void __launch_bounds__(kW, 2) dc_block_group_kernel(const BlockDev* _
       L = Ls[w.x];
     }
     __syncthreads();
-    block_lane<V, OpT, kHasB3, kW>(D, L, o, D.in_smem ? smem_raw : own_slab, own_slab, smem_raw + ring_at, red,
-                                   w.y, nullptr);
+    block_lane<V, kHasB3, kW>(D, L, o, D.in_smem ? smem_raw : own_slab, own_slab, red, w.y, nullptr);
     __syncthreads();
   }
 }
@@ -750,17 +585,17 @@ __global__ void __launch_bounds__(kW) block_lead_kernel(BlockDev D, LaneDev L, u
   gather_pattern<kW>(T, b.m, out, tid);
 }
 
-template <typename V, typename OpT, bool kHasB3>
+template <typename V, bool kHasB3>
 cudaError_t launch_t(const BlockDev& D, const LaneDev& L, const LaneOpts& o, cudaStream_t s) {
   // operating-point lanes: the FP64 form with the ladder between runs
-  auto* k = dc_block_kernel<V, OpT, kHasB3, kBlockThreads, false>;
+  auto* k = dc_block_kernel<V, kHasB3, kBlockThreads, false>;
   if (o.ladder) {
     if constexpr (sizeof(V) == 8)
-      k = dc_block_kernel<V, OpT, kHasB3, kBlockThreads, true>;
+      k = dc_block_kernel<V, kHasB3, kBlockThreads, true>;
     else
       return cudaErrorNotSupported;
   }
-  const size_t smem = (D.in_smem ? D.lane_bytes : 0) + D.ring_bytes;
+  const size_t smem = (D.in_smem ? D.lane_bytes : 0);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   const uint32_t grid = D.grid < L.n_lanes ? D.grid : L.n_lanes;
@@ -768,32 +603,32 @@ cudaError_t launch_t(const BlockDev& D, const LaneDev& L, const LaneOpts& o, cud
   return cudaGetLastError();
 }
 
-template <typename V, typename OpT, bool kHasB3>
+template <typename V, bool kHasB3>
 int occupancy_t(size_t smem) {
   int per_sm = 0;
-  auto* k = dc_block_kernel<V, OpT, kHasB3, kBlockThreads, false>;
+  auto* k = dc_block_kernel<V, kHasB3, kBlockThreads, false>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, int(kBlockThreads), smem);
   return per_sm;
 }
 
-template <typename V, typename OpT, bool kHasB3>
+template <typename V, bool kHasB3>
 cudaError_t launch_group_t(const BlockDev* Ds, const LaneDev* Ls, const uint2* items, uint32_t n_items,
                            uint32_t* next, const LaneOpts& o, unsigned char* slab, size_t slab_stride, size_t smem,
-                           uint32_t ring_at, uint32_t grid, cudaStream_t s) {
-  auto* k = dc_block_group_kernel<V, OpT, kHasB3, kBlockThreads>;
+                           uint32_t grid, cudaStream_t s) {
+  auto* k = dc_block_group_kernel<V, kHasB3, kBlockThreads>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(next, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
-  k<<<grid, kBlockThreads, smem, s>>>(Ds, Ls, items, n_items, next, o, slab, slab_stride, ring_at);
+  k<<<grid, kBlockThreads, smem, s>>>(Ds, Ls, items, n_items, next, o, slab, slab_stride);
   return cudaGetLastError();
 }
 
-template <typename V, typename OpT, bool kHasB3>
+template <typename V, bool kHasB3>
 int group_occupancy_t(size_t smem) {
   int per_sm = 0;
-  auto* k = dc_block_group_kernel<V, OpT, kHasB3, kBlockThreads>;
+  auto* k = dc_block_group_kernel<V, kHasB3, kBlockThreads>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, int(kBlockThreads), smem);
   return per_sm;
@@ -875,7 +710,7 @@ __device__ void block_companion(const TopoDev& T, const BlockMem<V>& b, const Bl
 // The mixed form (V = float) refactors and solves in FP32 and refines the
 // step in FP64 as the DC block lanes do (block_refine, refine_skip), adding
 // the corrections made to `refinements`.
-template <typename V, typename OpT, bool kHasB3, uint32_t kW>
+template <typename V, bool kHasB3, uint32_t kW>
 __device__ int block_tran_newton(const BlockDev& D, const BlockMem<V>& b, const double* rec, const LaneOpts& o,
                                  const SimDev& sim, const BlockCompanion* cp, bool& lim_active, bool init_fix,
                                  uint32_t& iters, const double* vsrc, uint64_t* red, int tid,
@@ -913,14 +748,14 @@ __device__ int block_tran_newton(const BlockDev& D, const BlockMem<V>& b, const 
       const double scale = fmin(fmax(from_bits(xm), from_bits(fm) * gd), 1e18);
       limit = !(1e3 * scale > kXPlausible) ? kXPlausible : 1e3 * scale;
     }
-    if (block_refactor<V, OpT, kW>(D, b.v, b.ring, tid)) {
+    if (block_refactor<V, kW>(D, b.v, tid)) {
       iters = iter + 1;
       return 2;
     }
-    block_rows<V, OpT, kW>(static_cast<const OpT*>(D.b_ops), D.b_rows, b.v, b.ring, tid, D.row_k);
+    block_program(D, D.b, b.v);
     for (uint32_t j = tid; j < n; j += kW) b.dx[T.qcol[j]] = double(b.y[j]);
     __syncthreads();
-    if constexpr (kMixed) refinements += block_refine_step<OpT, kW>(D, b, o, red, tid);
+    if constexpr (kMixed) refinements += block_refine_step<kW>(D, b, o, red, tid);
     // finalizeStep: x_old = x, x += dx, delta score (updateAndNorm)
     uint64_t worst = 0;
     for (uint32_t i = tid; i < n; i += kW) {
@@ -978,14 +813,14 @@ __host__ __device__ inline size_t tran_block_slab_doubles(const TopoDev& T) {
 // One lane's whole transient on the CTA (tran_lane's run): the operating
 // point through op.zig's ladder, then the trapezoidal steps with the
 // predictor, LTE control, order promotion and source breakpoints.
-template <typename V, typename OpT, bool kHasB3, uint32_t kW>
+template <typename V, bool kHasB3, uint32_t kW>
 __device__ void block_tran_lane(const BlockDev& D, const LaneDev& L, const TranDev& P, const LaneOpts& o,
-                                unsigned char* base, unsigned char* cold, unsigned char* ring, double* tslab,
+                                unsigned char* base, unsigned char* cold, double* tslab,
                                 uint64_t* red, uint32_t lane) {
   const TopoDev& T = D.T;
   const int tid = threadIdx.x;
   const uint32_t n = T.n, nq = T.n_qt;
-  const BlockMem<V> b = block_carve<V>(D, base, cold, ring, sizeof(OpT));
+  const BlockMem<V> b = block_carve<V>(D, base, cold);
   uint32_t refinements = 0;
   const LaneMem& m = b.m;
   double* cur = tslab;
@@ -1065,7 +900,7 @@ __device__ void block_tran_lane(const BlockDev& D, const LaneDev& L, const TranD
       rs.gmin = run.gmin_dev;
       fill_sources<kW>(T, rec, rs, vsrc, tid);
       uint32_t it = 0;
-      const int r = block_tran_newton<V, OpT, kHasB3, kW>(D, b, rec, ro, rs, nullptr, lim_active, mv.init_fix, it,
+      const int r = block_tran_newton<V, kHasB3, kW>(D, b, rec, ro, rs, nullptr, lim_active, mv.init_fix, it,
                                                            vsrc, red, tid, refinements);
       if (r == 2) {
         left = true;
@@ -1141,7 +976,7 @@ __device__ void block_tran_lane(const BlockDev& D, const LaneDev& L, const TranD
       const BlockCompanion c{ag0, ag1, trap, slot(qh, n, 1), ipr};
       uint32_t iters = 0;
       fill_sources<kW>(T, rec, sim, vsrc, tid);
-      rc = block_tran_newton<V, OpT, kHasB3, kW>(D, b, rec, nr, sim, &c, lim_active, false, iters, vsrc, red, tid,
+      rc = block_tran_newton<V, kHasB3, kW>(D, b, rec, nr, sim, &c, lim_active, false, iters, vsrc, red, tid,
                                                  refinements);
       lim_active = false;
       if (rc == 2) {
@@ -1268,26 +1103,25 @@ __device__ void block_tran_lane(const BlockDev& D, const LaneDev& L, const TranD
 // Persistent grid over the lanes, one CTA per lane at a time; the working
 // set placed as the DC block lanes place it (shared memory, split or slab),
 // the run state in the CTA's part of tslab.
-template <typename V, typename OpT, bool kHasB3, uint32_t kW>
+template <typename V, bool kHasB3, uint32_t kW>
 __global__ void __launch_bounds__(kW, 2) tran_block_kernel(BlockDev D, LaneDev L, TranDev P, LaneOpts o,
                                                           double* tslab, size_t tslab_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t red[kW / 32];
   unsigned char* own = D.slab + size_t(blockIdx.x) * (D.split ? D.cold_bytes : D.lane_bytes);
   unsigned char* base = D.in_smem ? smem_raw : own;
-  unsigned char* ring = smem_raw + (D.in_smem ? D.lane_bytes : 0u);
   double* ts = tslab + size_t(blockIdx.x) * tslab_stride;
   for (uint32_t lane = blockIdx.x; lane < L.n_lanes; lane += gridDim.x) {
-    block_tran_lane<V, OpT, kHasB3, kW>(D, L, P, o, base, own, ring, ts, red, lane);
+    block_tran_lane<V, kHasB3, kW>(D, L, P, o, base, own, ts, red, lane);
     __syncthreads();
   }
 }
 
-template <typename V, typename OpT, bool kHasB3>
+template <typename V, bool kHasB3>
 cudaError_t launch_tran_t(const BlockDev& D, const LaneDev& L, const TranDev& P, const LaneOpts& o, double* tslab,
                           size_t tslab_stride, cudaStream_t s) {
-  auto* k = tran_block_kernel<V, OpT, kHasB3, kBlockThreads>;
-  const size_t smem = (D.in_smem ? D.lane_bytes : 0) + D.ring_bytes;
+  auto* k = tran_block_kernel<V, kHasB3, kBlockThreads>;
+  const size_t smem = (D.in_smem ? D.lane_bytes : 0);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   const uint32_t grid = D.grid < L.n_lanes ? D.grid : L.n_lanes;
@@ -1295,22 +1129,17 @@ cudaError_t launch_tran_t(const BlockDev& D, const LaneDev& L, const TranDev& P,
   return cudaGetLastError();
 }
 
-// The eight instantiations: precision x op format x BSIM3.
-#define ESL_BLOCK_DISPATCH(F, ...)                                                     \
-  do {                                                                                 \
-    if (mixed) {                                                                       \
-      if (long_ops) return has_b3 ? F<float, uint4, true>(__VA_ARGS__) : F<float, uint4, false>(__VA_ARGS__); \
-      return has_b3 ? F<float, uint2, true>(__VA_ARGS__) : F<float, uint2, false>(__VA_ARGS__);               \
-    }                                                                                  \
-    if (long_ops) return has_b3 ? F<double, uint4, true>(__VA_ARGS__) : F<double, uint4, false>(__VA_ARGS__); \
-    return has_b3 ? F<double, uint2, true>(__VA_ARGS__) : F<double, uint2, false>(__VA_ARGS__);               \
+// The four instantiations: precision x BSIM3.
+#define ESL_BLOCK_DISPATCH(F, ...)                                                           \
+  do {                                                                                       \
+    if (mixed) return has_b3 ? F<float, true>(__VA_ARGS__) : F<float, false>(__VA_ARGS__);   \
+    return has_b3 ? F<double, true>(__VA_ARGS__) : F<double, false>(__VA_ARGS__);            \
   } while (0)
 
 }  // namespace
 
 cudaError_t launch_dc_block(const BlockDev& D, const LaneDev& L, const LaneOpts& o, bool mixed, bool has_b3,
                             cudaStream_t s) {
-  const bool long_ops = D.op_bytes == 16;
   ESL_BLOCK_DISPATCH(launch_t, D, L, o, s);
 }
 
@@ -1319,23 +1148,20 @@ size_t tran_block_slab(const TopoDev& T) { return tran_block_slab_doubles(T); }
 cudaError_t launch_tran_block(const BlockDev& D, const LaneDev& L, const TranDev& P, const LaneOpts& o, bool mixed,
                               bool has_b3, double* tslab, cudaStream_t s) {
   const size_t stride = tran_block_slab_doubles(D.T);
-  const bool long_ops = D.op_bytes == 16;
   ESL_BLOCK_DISPATCH(launch_tran_t, D, L, P, o, tslab, stride, s);
 }
 
-int block_occupancy(bool mixed, bool long_ops, bool has_b3, size_t smem) {
+int block_occupancy(bool mixed, bool has_b3, size_t smem) {
   ESL_BLOCK_DISPATCH(occupancy_t, smem);
 }
 
 cudaError_t launch_dc_block_group(const BlockDev* d_Ds, const LaneDev* d_Ls, const uint2* d_items, uint32_t n_items,
                                   uint32_t* d_next, const LaneOpts& o, unsigned char* slab, size_t slab_stride,
-                                  size_t smem, uint32_t ring_at, uint32_t grid, bool mixed, bool long_ops, bool has_b3,
-                                  cudaStream_t s) {
-  ESL_BLOCK_DISPATCH(launch_group_t, d_Ds, d_Ls, d_items, n_items, d_next, o, slab, slab_stride, smem, ring_at, grid,
-                     s);
+                                  size_t smem, uint32_t grid, bool mixed, bool has_b3, cudaStream_t s) {
+  ESL_BLOCK_DISPATCH(launch_group_t, d_Ds, d_Ls, d_items, n_items, d_next, o, slab, slab_stride, smem, grid, s);
 }
 
-int block_group_occupancy(bool mixed, bool long_ops, bool has_b3, size_t smem) {
+int block_group_occupancy(bool mixed, bool has_b3, size_t smem) {
   ESL_BLOCK_DISPATCH(group_occupancy_t, smem);
 }
 

@@ -13,10 +13,6 @@ namespace esl {
 
 // Threads of a block lane's CTA (its program rows are this wide).
 constexpr uint32_t kBlockThreads = 256;
-// Ops per thread in a program row of a working set that lives in the CTA's
-// global slab (rows of kSlabRowOps * kBlockThreads ops); 1 in shared memory.
-constexpr uint32_t kSlabRowOps = 4;
-
 // The block lanes' assembly streams (see block_assemble): a term word is a
 // staging index, with kGTermEnd on a cell's last term. Three cells past the
 // device stamps hold constants, so every term is a plain load: n_stage +
@@ -29,17 +25,18 @@ constexpr uint32_t kGTermEnd = 0x80000000u;
 constexpr uint32_t kGCellZero = 0, kGCellOne = 1, kGCellX0 = 2, kGConstCells = 3;
 constexpr uint32_t kGCellRow = 0x80000000u;
 
+// A task program (host/schedule.hpp TaskStream): its words, and each warp's
+// chunks.
+struct BlockProgram {
+  const uint32_t* words;
+  uint32_t off[kBlockThreads / 32 + 1];
+};
+
 struct BlockDev {
   TopoDev T;  // the topology's tables (pattern, gathers, tape maps, batches)
   // Programs A (refactor + forward solve), B (back solve) and F (forward
-  // solve alone), rows of row_k * kBlockThreads ops (row_k 1 or
-  // kSlabRowOps), op_bytes each: 8 {dst | kind << 28, a | b << 16} (value
-  // space below 65,536) or 16 {dst | kind << 28, a, b, 0}; ring_bytes: the
-  // per-CTA ring the ops stream through.
-  const void* a_ops;
-  const void* b_ops;
-  const void* f_ops;
-  uint32_t a_rows, b_rows, f_rows, op_bytes, ring_bytes, row_k;
+  // solve alone).
+  BlockProgram a, b, f;
   // The assembly: term stream [g_len][kBlockThreads], cell stream
   // [g_ncells][kBlockThreads] (uint4).
   const uint32_t* g_terms;
@@ -87,20 +84,17 @@ enum BlockPhase : uint32_t {
 // values with FP64 refinement; has_b3: the BSIM3 instantiation.
 cudaError_t launch_dc_block(const BlockDev& D, const LaneDev& L, const LaneOpts& o, bool mixed, bool has_b3,
                             cudaStream_t s);
-// CTAs per SM of the DC kernel at this precision, op format and dynamic shared memory.
-int block_occupancy(bool mixed, bool long_ops, bool has_b3, size_t smem);
+// CTAs per SM of the DC kernel at this precision and dynamic shared memory.
+int block_occupancy(bool mixed, bool has_b3, size_t smem);
 // Uneven batching: the lanes of several topologies (device arrays of their
 // BlockDev and LaneDev) in one persistent launch over work items (topology,
 // lane), taken from the counter d_next in order; smem: the largest working
 // set of the topologies that keep theirs in shared memory; slab_stride: the
-// largest of the others (each CTA's slab at slab + blockIdx.x * stride);
-// ring_at: the op ring's offset in dynamic shared memory. Every topology
-// of a group has the same op format.
+// largest of the others (each CTA's slab at slab + blockIdx.x * stride).
 cudaError_t launch_dc_block_group(const BlockDev* d_Ds, const LaneDev* d_Ls, const uint2* d_items, uint32_t n_items,
                                   uint32_t* d_next, const LaneOpts& o, unsigned char* slab, size_t slab_stride,
-                                  size_t smem, uint32_t ring_at, uint32_t grid, bool mixed, bool long_ops, bool has_b3,
-                                  cudaStream_t s);
-int block_group_occupancy(bool mixed, bool long_ops, bool has_b3, size_t smem);
+                                  size_t smem, uint32_t grid, bool mixed, bool has_b3, cudaStream_t s);
+int block_group_occupancy(bool mixed, bool has_b3, size_t smem);
 
 // Transient block lanes: every lane's operating point and whole transient
 // (the warp lanes' tran_kernel run, no measure cards) on a CTA per lane,
