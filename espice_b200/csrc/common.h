@@ -99,22 +99,30 @@ enum OpKind : uint32_t {
 };
 
 // One task of a block-lane program: up to kTaskOps updates v[dst] -= v[a] *
-// v[b] in order, then (kTaskDiv) v[dst] /= v[divisor]. Eight words: dst |
-// flags, divisor | flags, then a, b of each update, in two planes of four
-// words per lane (one 16-byte load each); padding updates multiply the
-// constant 0.0 by 1.0. Flags of word 0: kTaskNz (an update with v[b] == 0 is
-// skipped, the solves' zero skip), kTaskDiv, and the same in every lane of
-// the warp: kTaskMore (more than one update), kTaskCta (a CTA barrier
-// follows). Flags of word 1: the division's pivot tests (kOpDivGrowth,
-// kOpDivScaled), and kTaskDivAny (a lane of the warp divides). A dst field
-// of kTaskIdle: the warp has no task for word 1's number of barriers.
-constexpr uint32_t kTaskOps = 3, kTaskWords = 8;
-constexpr uint32_t kTaskIndex = 0x0fffffffu, kTaskIdle = kTaskIndex;
-constexpr uint32_t kTaskNz = 1u << 28, kTaskDiv = 1u << 29, kTaskMore = 1u << 30, kTaskCta = 1u << 31;
-constexpr uint32_t kTaskGrowth = 1u << 28, kTaskScaled = 1u << 29, kTaskDivAny = 1u << 30;
-// Chunks (a warp's 32 tasks) the kernel takes per trip through its loop, and
-// reads ahead past a warp's last one.
-constexpr uint32_t kTaskUnroll = 3;
+// v[b] in order; or, with kTaskDiv, up to kTaskOps - 1 and then v[dst] /=
+// v[a of the last pair]. Padding updates multiply the constant 0.0 by 1.0.
+// Compact words (value spaces below 65,536): dst | flags << 16, then a | b
+// << 16 of each update, 16 bytes. Wide words: dst, flags, then a, b of each
+// update, two planes of 16 bytes per lane. A chunk is the tasks of a warp's
+// 32 lanes.
+constexpr uint32_t kTaskOps = 3;
+constexpr uint32_t task_words(bool compact) { return compact ? 4u : 8u; }
+enum TaskFlag : uint32_t {
+  kTaskNz = 1,        // an update with v[b] == 0 is skipped (the solves' zero skip)
+  kTaskDiv = 2,       // the division
+  kTaskGrowth = 4,    // its pivot tests: kOpDivGrowth's and the L entry's bound,
+  kTaskScaled = 8,    // or kOpDivScaled's
+  // the same in every lane of the warp:
+  kTaskMore = 16,     // a lane has more than one update
+  kTaskDivAny = 32,   // a lane divides
+  kTaskCta = 64,      // a CTA barrier follows
+  kTaskIdle = 128,    // no tasks: as many CTA barriers as the word after the flags' says
+};
+// Slots of a warp's ring of chunks, and the chunks read ahead past its last.
+constexpr uint32_t kTaskRing = 4;
+constexpr uint32_t task_ring_bytes(uint32_t warps, bool compact) {
+  return warps * kTaskRing * 32 * 4 * task_words(compact);
+}
 
 // Per-lane transient statistics (the same fields, in the same order, as the
 // oracle's step counters), and the run's status word.

@@ -208,6 +208,14 @@ cudaError_t upload(DevBuf& b, const std::vector<T>& v, cudaStream_t s) {
 
 }  // namespace
 
+// The block lanes' programs and assembly streams of a tape at one CTA width.
+struct BlockTables {
+  bool have = false;
+  BlockPrograms prog;
+  uint32_t g_len[kBlockThreads / 32] = {}, g_terms = 0, g_ncells = 0;
+  DevBuf d_a, d_b, d_f, d_terms, d_cells;
+};
+
 struct esl_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -245,11 +253,9 @@ struct esl_ctx {
   double refine_tol = 1e-12;
   uint32_t refine_max = 6;
   double refine_skip = 0.0;  // mixed: steps above this many tolerances go unrefined (0: none)
-  bool have_block = false;
   bool profile = false;  // block lanes: accumulate the phase cycles (esl_solve_mode.profile)
-  BlockPrograms bprog;
-  uint32_t block_g_len = 0, block_g_ncells = 0;
-  DevBuf d_ba, d_bb, d_bf, d_slab, d_refine, d_prof, d_bg_terms, d_bg_cells;
+  BlockTables block[2];  // CTAs of kBlockThreads, of kBlockNarrow threads
+  DevBuf d_slab, d_refine, d_prof;
   SparseLu lead;
   Programs prog;
 
@@ -723,7 +729,7 @@ int32_t upload_tape(esl_ctx* ctx) {
   T.l_scaled = ctx->d_l_scaled.as<uint8_t>();
   T.pinv = ctx->d_pinv.as<uint32_t>();
   T.qcol = ctx->d_q.as<uint32_t>();
-  ctx->have_block = false;  // a new tape needs its own block programs
+  for (BlockTables& t : ctx->block) t.have = false;  // a new tape needs its own block programs
   lu_jit_release(ctx->lu_jit);  // and its own compiled LU
   ctx->lu_jit_state = 0;
   lu_jit_release(ctx->lu_jit_mixed);
@@ -805,12 +811,16 @@ int32_t upload_tape(esl_ctx* ctx) {
 
 // The block lanes' assembly streams (block.cu block_assemble): every
 // residual row and pattern slot is a cell summing its staging terms in list
-// order; cells go to the CTA's threads longest first, each to the least
-// loaded thread; a thread's terms follow one another in its stream
-// (terms[k * W + t]), the last term of each cell flagged, and its cells'
-// destinations in its cell stream (cells[c * W + t]).
+// order. The cells, longest first, go to the warps 32 at a time, each group
+// to the least loaded warp, its shorter cells padded with +0.0 terms to its
+// longest: a warp's threads close their cells together, and the store is one
+// uniform branch. (Cells dealt one by one to the least loaded thread closed
+// at every term of some thread: 62k cycles an assembly of the analog block,
+// two CTAs an SM, against 51k, and 36k with the two batches in turn.) A thread's terms follow one another in its
+// stream (terms[k * W + t]), the last term of each cell flagged, and its
+// cells' destinations in its cell stream (cells[c * W + t]).
 void build_block_gather(const esl_ctx* ctx, uint32_t W, std::vector<uint32_t>& terms, std::vector<uint32_t>& cells,
-                        uint32_t& len, uint32_t& ncells) {
+                        BlockTables& B) {
   struct Cell {
     std::vector<uint32_t> src;
     uint32_t w0, w1, w2, w3;
@@ -836,27 +846,38 @@ void build_block_gather(const esl_ctx* ctx, uint32_t W, std::vector<uint32_t>& t
     for (uint32_t e = ctx->a_ptr[p]; e < ctx->a_ptr[p + 1]; ++e) c.src.push_back(code(ctx->a_src[e]));
     all.push_back(std::move(c));
   }
-  for (Cell& c : all) {
+  for (Cell& c : all)
     if (c.src.empty()) c.src.push_back(ns + kGCellZero);
-    c.src.back() |= kGTermEnd;
-  }
   std::stable_sort(all.begin(), all.end(), [](const Cell& a, const Cell& b) { return a.src.size() > b.src.size(); });
   std::vector<std::vector<uint32_t>> t_terms(W), t_cells(W);
-  std::vector<size_t> load(W, 0);
-  for (const Cell& c : all) {
-    const uint32_t t = uint32_t(std::min_element(load.begin(), load.end()) - load.begin());
-    t_terms[t].insert(t_terms[t].end(), c.src.begin(), c.src.end());
-    t_cells[t].insert(t_cells[t].end(), {c.w0, c.w1, c.w2, c.w3});
-    load[t] += c.src.size();
+  std::vector<size_t> load(W / 32, 0);
+  for (size_t g = 0; g < all.size(); g += 32) {
+    const uint32_t w = uint32_t(std::min_element(load.begin(), load.end()) - load.begin());
+    const size_t longest = all[g].src.size();
+    for (uint32_t l = 0; l < 32; ++l) {
+      const Cell& c = all[std::min(g + l, all.size() - 1)];  // past the last cell: the last one again, the same value
+      std::vector<uint32_t>& t = t_terms[32 * w + l];
+      t.insert(t.end(), c.src.begin(), c.src.end());
+      t.insert(t.end(), longest - c.src.size(), ns + kGCellZero);
+      t.back() |= kGTermEnd;
+      t_cells[32 * w + l].insert(t_cells[32 * w + l].end(), {c.w0, c.w1, c.w2, c.w3});
+    }
+    load[w] += longest + 4;  // the store's cost beside its terms
   }
-  len = 0;
-  ncells = 0;
-  for (uint32_t t = 0; t < W; ++t) {
-    len = std::max(len, uint32_t(t_terms[t].size()));
-    ncells = std::max(ncells, uint32_t(t_cells[t].size() / 4));
+  // whole pairs of batches, and one pair of +0.0 terms (and two cells) that
+  // are only read ahead
+  constexpr uint32_t kPair = 2 * kGBatch;
+  uint32_t rows = 0;
+  B.g_terms = B.g_ncells = 0;
+  for (uint32_t w = 0; w < W / 32; ++w) {
+    const uint32_t len = uint32_t(t_terms[32 * w].size());
+    B.g_terms = std::max(B.g_terms, len);
+    B.g_ncells = std::max(B.g_ncells, uint32_t(t_cells[32 * w].size() / 4));
+    B.g_len[w] = (len + kPair - 1) / kPair * kPair;
+    rows = std::max(rows, B.g_len[w] + kPair);
   }
-  terms.assign(size_t(std::max(len, 1u)) * W, ns + kGCellZero);
-  cells.assign(size_t(std::max(ncells, 1u)) * W * 4, 0u);
+  terms.assign(size_t(rows) * W, ns + kGCellZero);
+  cells.assign(size_t(B.g_ncells + 2) * W * 4, 0u);
   for (uint32_t t = 0; t < W; ++t) {
     for (size_t k = 0; k < t_terms[t].size(); ++k) terms[k * W + t] = t_terms[t][k];
     for (size_t c = 0; c < t_cells[t].size() / 4; ++c)
@@ -864,50 +885,54 @@ void build_block_gather(const esl_ctx* ctx, uint32_t W, std::vector<uint32_t>& t
   }
 }
 
-void block_layout(const TopoDev& T, uint32_t nv, bool mixed, bool split, BlockDev& D);
 constexpr size_t kBlockSmemRoom = size_t(227) * 1024 - 256;
 
-// The block lanes' programs and assembly streams of the current tape.
-int32_t ensure_block(esl_ctx* ctx) {
-  if (ctx->have_block) return ESL_OK;
+// The block lanes' tables of the current tape for CTAs of `threads`.
+int32_t ensure_block(esl_ctx* ctx, uint32_t threads) {
+  BlockTables& t = ctx->block[threads == kBlockNarrow];
+  if (t.have) return ESL_OK;
   cudaStream_t s = ctx->stream;
-  if (ctx->prog.nv > kTaskIdle) return ctx->fail(ESL_NOT_ELIGIBLE, "the tape's values exceed 28-bit indices");
-  ctx->bprog = compile_block(ctx->prog);
-  ESL_CUDA(upload(ctx->d_ba, ctx->bprog.a.words, s));
-  ESL_CUDA(upload(ctx->d_bb, ctx->bprog.b.words, s));
-  ESL_CUDA(upload(ctx->d_bf, ctx->bprog.f.words, s));
+  t.prog = compile_block(ctx->prog, threads / 32);
   std::vector<uint32_t> terms, cells;
-  build_block_gather(ctx, kBlockThreads, terms, cells, ctx->block_g_len, ctx->block_g_ncells);
-  ESL_CUDA(upload(ctx->d_bg_terms, terms, s));
-  ESL_CUDA(upload(ctx->d_bg_cells, cells, s));
-  ctx->have_block = true;
+  build_block_gather(ctx, threads, terms, cells, t);
+  ESL_CUDA(upload(t.d_a, t.prog.a.words, s));
+  ESL_CUDA(upload(t.d_b, t.prog.b.words, s));
+  ESL_CUDA(upload(t.d_f, t.prog.f.words, s));
+  ESL_CUDA(upload(t.d_terms, terms, s));
+  ESL_CUDA(upload(t.d_cells, cells, s));
+  t.have = true;
   return ESL_OK;
 }
 
-// A block lane's working set (block.cu carves the same): the hot part x,
-// rhs, diag, dx (FP64, n each), limited images, the FP64 matrix (mixed
-// form), the value space (nv values, FP64 or FP32); the cold part xo and
-// the staging cells; each 16-byte aligned. split: the cold part's offsets
-// start again from 0 (it lives in the CTA's slab).
-void block_layout(const TopoDev& T, uint32_t nv, bool mixed, bool split, BlockDev& D) {
-  size_t at = 0;
+// A block lane's working set (block.cu carves the same), each part 16-byte
+// aligned: limited images, the value space (nv values, FP64 or FP32), x,
+// rhs, diag, dx (FP64, n each), the FP64 matrix (mixed form), xo and the
+// staging cells. split 1: xo and the staging cells, split 2: all from x on,
+// live in the CTA's slab (their offsets start again from 0).
+void block_layout(const TopoDev& T, uint32_t nv, bool mixed, uint32_t split, BlockDev& D) {
+  size_t at = 0, hot = 0;
   auto take = [&at](size_t bytes) {
     const size_t o = at;
     at += (bytes + 15) & ~size_t(15);
     return uint32_t(o);
   };
+  auto cold_from = [&](uint32_t level) {
+    if (split != level) return;
+    hot = at;
+    at = 0;
+  };
+  D.o_lim = take(8 * size_t(std::max<uint32_t>(T.nlim, 1)));
+  D.o_v = take(size_t(mixed ? 4 : 8) * nv);
+  cold_from(2);
   D.o_x = take(8 * size_t(T.n));
   D.o_rhs = take(8 * size_t(T.n));
   D.o_diag = take(8 * size_t(T.n));
   D.o_dx = take(8 * size_t(T.n));
-  D.o_lim = take(8 * size_t(std::max<uint32_t>(T.nlim, 1)));
   D.o_a64 = take(mixed ? 8 * size_t(T.nnz) : 0);
-  D.o_v = take(size_t(mixed ? 4 : 8) * nv);
-  const size_t hot = at;
-  if (split) at = 0;
+  cold_from(1);
   D.o_xo = take(8 * size_t(T.n));
   D.o_st = take(8 * size_t(T.n_stage + kGConstCells));
-  D.split = split ? 1u : 0u;
+  D.split = split;
   D.lane_bytes = uint32_t(split ? hot : at);
   D.cold_bytes = uint32_t(split ? at : 0);
 }
@@ -915,41 +940,65 @@ void block_layout(const TopoDev& T, uint32_t nv, bool mixed, bool split, BlockDe
 // Shared memory a block lane may take (kBlockSmemRoom: a CTA's 227 KB, less
 // the static reduction words).
 
-// The launch view of the block lanes for n_lanes lanes: programs, layout,
-// where the working set lives, the persistent grid and its slab.
-int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D) {
-  if (int32_t rc = ensure_block(ctx)) return rc;
-  const TopoDev& T = ctx->topo;
-  D = BlockDev{};
-  D.T = T;
-  auto program = [](BlockProgram& p, const DevBuf& d, const TaskStream& t) {
-    p.words = d.as<uint32_t>();
-    std::copy(std::begin(t.off), std::end(t.off), p.off);
-  };
-  program(D.a, ctx->d_ba, ctx->bprog.a);
-  program(D.b, ctx->d_bb, ctx->bprog.b);
-  program(D.f, ctx->d_bf, ctx->bprog.f);
-  D.g_terms = ctx->d_bg_terms.as<uint32_t>();
-  D.g_cells = ctx->d_bg_cells.as<uint4>();
-  D.g_len = ctx->block_g_len;
-  D.g_ncells = ctx->block_g_ncells;
-  // The placement with the most CTAs an SM: the whole working set in shared
-  // memory, its hot part there (the cold part in the slab), or all of it in
-  // the slab; on a tie, the most in shared memory.
+// The placement with the most CTAs an SM: the working set in shared memory,
+// its hot part there (split 1, 2; the rest in the CTA's slab), or all of it
+// in the slab; on a tie, the most in shared memory. Returns the CTAs.
+int block_place(const TopoDev& T, bool mixed, uint32_t threads, BlockDev& D) {
   const bool b3 = topo_has_b3(T);
+  D.compact = T.nv < 65536;
+  D.ring_bytes = task_ring_bytes(threads / 32, D.compact);
   int best = -1;
-  uint32_t place = 2;
-  for (uint32_t p = 0; p < 3; ++p) {
-    block_layout(T, T.nv, mixed, p == 1, D);
-    if (p < 2 && D.lane_bytes > kBlockSmemRoom) continue;
-    const int per_sm = block_occupancy(mixed, b3, p < 2 ? D.lane_bytes : 0);
+  uint32_t place = 3;
+  for (uint32_t p = 0; p < 4; ++p) {
+    block_layout(T, T.nv, mixed, p < 3 ? p : 0, D);
+    if (p < 3 && D.lane_bytes + D.ring_bytes > kBlockSmemRoom) continue;
+    const int per_sm = block_occupancy(mixed, b3, threads, D.ring_bytes + (p < 3 ? D.lane_bytes : 0));
     if (per_sm > best) {
       best = per_sm;
       place = p;
     }
   }
-  block_layout(T, T.nv, mixed, place == 1, D);
-  D.in_smem = place < 2;
+  block_layout(T, T.nv, mixed, place < 3 ? place : 0, D);
+  D.in_smem = place < 3;
+  return std::max(best, 1);
+}
+
+// The launch view of the block lanes for n_lanes lanes: the CTA's width,
+// programs, layout, where the working set lives, the persistent grid and its
+// slab. The narrow CTAs (DC lanes alone) when there are more lanes than the
+// wide ones hold at once and the narrow ones hold more of them: a lane's
+// rows are a chain of latencies that issues on a quarter of the cycles, so
+// four narrow lanes on an SM take less than twice the time of two wide ones
+// (analog block, mixed, 12,288 points: 78.9 -> 64.7 ms when this came in);
+// with fewer lanes the wide CTA's lane is the faster one.
+int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D, bool narrow_ok = false) {
+  const TopoDev& T = ctx->topo;
+  D = BlockDev{};
+  uint32_t threads = kBlockThreads;
+  int best = block_place(T, mixed, threads, D);
+  if (narrow_ok && n_lanes > uint32_t(ctx->sms) * uint32_t(best)) {
+    BlockDev N{};
+    const int narrow = block_place(T, mixed, kBlockNarrow, N);
+    if (N.in_smem && narrow > best) {
+      D = N;
+      best = narrow;
+      threads = kBlockNarrow;
+    }
+  }
+  if (int32_t rc = ensure_block(ctx, threads)) return rc;
+  const BlockTables& B = ctx->block[threads == kBlockNarrow];
+  D.T = T;
+  D.threads = threads;
+  auto program = [](BlockProgram& p, const DevBuf& d, const TaskStream& t) {
+    p.words = d.as<uint32_t>();
+    std::copy(std::begin(t.off), std::end(t.off), p.off);
+  };
+  program(D.a, B.d_a, B.prog.a);
+  program(D.b, B.d_b, B.prog.b);
+  program(D.f, B.d_f, B.prog.f);
+  D.g_terms = B.d_terms.as<uint32_t>();
+  D.g_cells = B.d_cells.as<uint4>();
+  std::copy(std::begin(B.g_len), std::end(B.g_len), D.g_len);
   const uint32_t cap = uint32_t(ctx->sms) * uint32_t(std::max(best, 1));
   D.grid = std::max<uint32_t>(1, std::min(n_lanes, cap));
   ESL_CUDA(ctx->d_slab.ensure(size_t(D.in_smem && !D.split ? 1 : D.grid) * (D.split ? D.cold_bytes : D.lane_bytes)));
@@ -983,7 +1032,7 @@ cudaError_t lead_jacobian(esl_ctx* ctx, const LaneDev& L, double* out) {
   if (smem <= size_t(227) * 1024) return launch_assemble(T, L, 0, out, ctx->stream);
   BlockDev D{};
   D.T = T;
-  block_layout(T, 0, false, false, D);
+  block_layout(T, 0, false, 0, D);
   cudaError_t e = ctx->d_slab.ensure(D.lane_bytes);
   if (e != cudaSuccess) return e;
   D.slab = ctx->d_slab.as<unsigned char>();
@@ -1334,7 +1383,7 @@ int32_t dc_solve(esl_ctx* ctx, const esl_newton_opts* opts, double* d_x, int col
   const bool mixed = ctx->precision == ESL_PREC_MIXED && !d_rung;
   BlockDev D{};
   if (block) {
-    if (int32_t rc = block_view(ctx, mixed, N, D)) return rc;
+    if (int32_t rc = block_view(ctx, mixed, N, D, !d_rung)) return rc;
     if (D.refine_out) ESL_CUDA(cudaMemsetAsync(D.refine_out, 0, size_t(N) * 4, s));
     if (D.prof) ESL_CUDA(cudaMemsetAsync(D.prof, 0, kBlockPhases * sizeof(unsigned long long), s));
   }
@@ -1848,14 +1897,25 @@ int32_t group_block(esl_ctx* const* ctxs, uint32_t n_ctx, const esl_newton_opts*
     b3 |= topo_has_b3(x->topo);
   }
   std::vector<BlockDev> Dg = Ds;
+  uint32_t ring = 0;  // the widest word form's, the same for every topology
+  for (uint32_t c = 0; c < n_ctx; ++c) ring = std::max(ring, Ds[c].ring_bytes);
+  // A launch has one shared-memory size, the largest of the working sets
+  // that live there, and what it takes the slab lanes lose as L1. So the
+  // small topologies keep theirs in shared memory only when the slab's are
+  // not the larger part of the work (eight meshes of 50 to 2,000 unknowns).
+  double near = 0.0, far = 0.0;
+  for (uint32_t c = 0; c < n_ctx; ++c)
+    (Ds[c].in_smem ? near : far) += double(ctxs[c]->prog.a_nops) * ctxs[c]->n_lanes;
   for (uint32_t c = 0; c < n_ctx; ++c) {
+    Dg[c].ring_bytes = ring;
     // each topology keeps its own placement (block_view's), the whole
     // working set in the CTA's slab when its shared part misses the room
-    Dg[c].in_smem = Dg[c].in_smem && Dg[c].lane_bytes <= kGroupSmemRoom;
-    if (!Dg[c].in_smem && Dg[c].split) block_layout(ctxs[c]->topo, ctxs[c]->topo.nv, mixed, false, Dg[c]);
+    Dg[c].in_smem = Dg[c].in_smem && near >= far && Dg[c].lane_bytes + ring <= kGroupSmemRoom;
+    if (!Dg[c].in_smem && Dg[c].split) block_layout(ctxs[c]->topo, ctxs[c]->topo.nv, mixed, 0, Dg[c]);
     if (Dg[c].in_smem) smem = std::max<size_t>(smem, Dg[c].lane_bytes);
     stride = std::max<size_t>(stride, Dg[c].split ? Dg[c].cold_bytes : Dg[c].in_smem ? 0 : Dg[c].lane_bytes);
   }
+  smem += ring;
   std::vector<uint32_t> order(n_ctx);
   for (uint32_t c = 0; c < n_ctx; ++c) order[c] = c;
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
@@ -2042,13 +2102,14 @@ int32_t esl_block_profile(esl_ctx* ctx, uint64_t* cycles) {
 int32_t esl_block_info(esl_ctx* ctx, esl_block_info_t* info) {
   if (!ctx || !info || !ctx->have_tape) return ESL_INVALID_ARGUMENT;
   cudaSetDevice(ctx->device);
-  if (int32_t rc = ensure_block(ctx)) return rc;
+  if (int32_t rc = ensure_block(ctx, kBlockThreads)) return rc;
+  const BlockPrograms& prog = ctx->block[0].prog;
   std::memset(info, 0, sizeof(*info));
   info->width = kBlockThreads;
-  info->a_rows = ctx->bprog.a.rows;
-  info->b_rows = ctx->bprog.b.rows;
-  info->f_rows = ctx->bprog.f.rows;
-  info->a_levels = ctx->bprog.a_levels;
+  info->a_rows = prog.a.rows;
+  info->b_rows = prog.b.rows;
+  info->f_rows = prog.f.rows;
+  info->a_levels = prog.a_levels;
   info->a_nops = ctx->prog.a_nops;
   info->b_nops = ctx->prog.b_nops;
   info->ntv = ctx->prog.ntv;
@@ -2059,11 +2120,12 @@ int32_t esl_block_info(esl_ctx* ctx, esl_block_info_t* info) {
     info->lane_bytes[m] = D.lane_bytes;
     info->in_smem[m] = D.in_smem;
     info->ctas_per_sm[m] = uint32_t(std::max(
-        0, block_occupancy(m == 1, topo_has_b3(ctx->topo), D.in_smem ? D.lane_bytes : 0)));
-    info->split[m] = D.split;
+        0, block_occupancy(m == 1, topo_has_b3(ctx->topo), kBlockThreads,
+                           D.ring_bytes + (D.in_smem ? D.lane_bytes : 0))));
+    info->split[m] = D.split != 0;
     info->cold_bytes[m] = D.cold_bytes;
-    info->gather_terms = D.g_len;
-    info->gather_cells = D.g_ncells;
+    info->gather_terms = ctx->block[0].g_terms;
+    info->gather_cells = ctx->block[0].g_ncells;
   }
   return ESL_OK;
 }

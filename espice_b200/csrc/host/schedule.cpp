@@ -232,7 +232,7 @@ constexpr int kSlack = 300;
 // refactor, 233 for its back solve) a task keeps its value in a register
 // over its updates and its division: 176 and 101 rows, and 3 loads an update
 // in place of 4 accesses.
-TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv) {
+TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv, uint32_t warps, bool compact) {
   const uint32_t sink = nv - 1, one = nv - 2, zero = nv - 3;
   const size_t n = seq.size();
   // vop[vptr[v] .. vptr[v + 1]): the ops of value v
@@ -298,24 +298,34 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv) {
     const uint32_t run = ready[v] - pos[v];
     const bool last = ready[v] == vptr[v + 1] && divides(v);
     Task t{v, pos[v], std::min(run - (last ? 1u : 0u), kTaskOps), false};
-    t.div = last && t.ops + 1 == run;
+    t.div = last && t.ops + 1 == run && t.ops < kTaskOps;
     return t;
   };
   std::vector<uint32_t> out[kTaskWarps];
   uint32_t idle[kTaskWarps] = {};
-  uint32_t lane_words[32][kTaskWords];
+  struct Words {
+    uint32_t dst, flags, pair[kTaskOps][2];
+  };
+  Words lanes[32];
   auto put = [&](uint32_t w) {
-    for (int h = 0; h < 2; ++h)
-      for (int l = 0; l < 32; ++l)
-        for (int j = 0; j < 4; ++j) out[w].push_back(lane_words[l][4 * h + j]);
+    std::vector<uint32_t>& o = out[w];
+    if (compact) {
+      for (const Words& x : lanes) {
+        o.push_back(x.dst | (x.flags << 16));
+        for (const auto& p : x.pair) o.push_back(p[0] | (p[1] << 16));
+      }
+      return;
+    }
+    for (const Words& x : lanes) o.insert(o.end(), {x.dst, x.flags, x.pair[0][0], x.pair[0][1]});
+    for (const Words& x : lanes) o.insert(o.end(), {x.pair[1][0], x.pair[1][1], x.pair[2][0], x.pair[2][1]});
   };
   auto put_idle = [&](uint32_t w, uint32_t barriers) {
-    for (auto& l : lane_words) {
-      std::fill(std::begin(l), std::end(l), 0u);
-      l[0] = kTaskIdle;
-      l[1] = barriers;
-    }
-    put(w);
+    do {  // the count takes the first update's words
+      const uint32_t k = std::min(barriers, 0xffffu);
+      for (Words& x : lanes) x = Words{0, kTaskIdle, {{k, 0}, {0, 0}, {0, 0}}};
+      put(w);
+      barriers -= k;
+    } while (barriers);
   };
   auto flush = [&](uint32_t w) {
     if (idle[w]) put_idle(w, idle[w]);
@@ -324,7 +334,7 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv) {
   TaskStream S;
   // One row's tasks onto the warps; `cta`: a CTA barrier follows.
   auto emit = [&](const std::vector<Task>& row, bool cta) {
-    for (uint32_t w = 0; w < kTaskWarps; ++w) {
+    for (uint32_t w = 0; w < warps; ++w) {
       if (32 * w >= row.size()) {
         idle[w] += cta;
         continue;
@@ -337,28 +347,30 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv) {
         most = std::max(most, row[t0 + l].ops);
         any_div |= row[t0 + l].div;
       }
+      const uint32_t common =
+          (most > 1 ? kTaskMore : 0u) | (any_div ? kTaskDivAny : 0u) | (cta ? kTaskCta : 0u);
       for (uint32_t l = 0; l < 32; ++l) {
-        uint32_t* x = lane_words[l];
-        x[0] = sink | (most > 1 ? kTaskMore : 0u) | (cta ? kTaskCta : 0u);
-        x[1] = one | (any_div ? kTaskDivAny : 0u);
-        for (uint32_t j = 0; j < kTaskOps; ++j) {
-          x[2 + 2 * j] = zero;
-          x[3 + 2 * j] = one;
+        Words& x = lanes[l];
+        x = Words{sink, common, {{zero, one}, {zero, one}, {zero, one}}};
+        if (l >= nt) {
+          x.pair[kTaskOps - 1][0] = any_div ? one : zero;  // what the lane divides by, unused
+          x.pair[kTaskOps - 1][1] = any_div ? zero : one;
+          continue;
         }
-        if (l >= nt) continue;
         const Task& t = row[t0 + l];
-        x[0] = (x[0] & ~kTaskIndex) | t.v;
+        x.dst = t.v;
         for (uint32_t j = 0; j < t.ops; ++j) {
           const SeqOp& o = seq[vop[t.lo + j]];
-          x[2 + 2 * j] = o.a;
-          x[3 + 2 * j] = o.b;
-          if (o.kind == kOpSubNz) x[0] |= kTaskNz;
+          x.pair[j][0] = o.a;
+          x.pair[j][1] = o.b;
+          if (o.kind == kOpSubNz) x.flags |= kTaskNz;
         }
         if (t.div) {
           const SeqOp& o = seq[vop[t.lo + t.ops]];
-          x[0] |= kTaskDiv;
-          x[1] = o.a | kTaskDivAny | (o.kind == kOpDivGrowth ? kTaskGrowth : 0u) |
-                 (o.kind == kOpDivScaled ? kTaskScaled : 0u);
+          x.flags |= kTaskDiv | (o.kind == kOpDivGrowth ? kTaskGrowth : 0u) |
+                     (o.kind == kOpDivScaled ? kTaskScaled : 0u);
+          x.pair[kTaskOps - 1][0] = o.a;
+          x.pair[kTaskOps - 1][1] = one;
         }
       }
       put(w);
@@ -372,7 +384,7 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv) {
     row.clear();
     later.clear();
     const int top = queue.front().first;
-    while (!queue.empty() && row.size() < 32 * kTaskWarps) {
+    while (!queue.empty() && row.size() < 32 * warps) {
       std::pop_heap(queue.begin(), queue.end());
       const uint32_t v = queue.back().second;
       const int path = queue.back().first;
@@ -414,14 +426,12 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv) {
   }
   if (!prev.empty()) emit(prev, true);
   size_t total = 0;
-  for (uint32_t w = 0; w < kTaskWarps; ++w) {
+  for (uint32_t w = 0; w < warps; ++w) {
     flush(w);
-    constexpr size_t kChunk = 32 * kTaskWords;
-    const size_t have = out[w].size() / kChunk;
-    const size_t want = (have + kTaskUnroll - 1) / kTaskUnroll * kTaskUnroll + kTaskUnroll;
-    for (size_t c = have; c < want; ++c) put_idle(w, 0u);
+    const size_t chunk = 32 * task_words(compact);
+    for (uint32_t c = 0; c < kTaskRing; ++c) put_idle(w, 0u);
     total += out[w].size();
-    S.off[w + 1] = uint32_t(total / kChunk);
+    S.off[w + 1] = uint32_t(total / chunk);
   }
   S.words.reserve(total);
   for (auto& o : out) {
@@ -433,17 +443,18 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv) {
 
 }  // namespace
 
-BlockPrograms compile_block(const Programs& P) {
+BlockPrograms compile_block(const Programs& P, uint32_t warps) {
   BlockPrograms B;
+  B.compact = P.nv < 65536;
   const std::vector<SeqOp> a = unpack(P.a_seq), b = unpack(P.b_seq);
-  B.a = pack_tasks(a, P.nv);
-  B.b = pack_tasks(b, P.nv);
+  B.a = pack_tasks(a, P.nv, warps, B.compact);
+  B.b = pack_tasks(b, P.nv, warps, B.compact);
   // the forward substitution alone (program A's solve ops), for the mixed
   // form's refinement corrections on the finished factors
   std::vector<SeqOp> f;
   for (const SeqOp& s : a)
     if (s.kind == kOpSubNz) f.push_back(s);
-  B.f = pack_tasks(f, P.nv);
+  B.f = pack_tasks(f, P.nv, warps, B.compact);
   // the longest dependence chain of single ops
   std::vector<uint32_t> level(P.nv, 0);
   for (const SeqOp& s : a) {

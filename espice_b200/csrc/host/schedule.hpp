@@ -48,9 +48,9 @@ struct Programs {
 
 // A block-lane program as each warp's stream of chunks, a chunk the 32 tasks
 // (common.h) its lanes run between two barriers: warp w's chunks are
-// off[w] .. off[w + 1] (in chunks of 32 * kTaskWords words), a multiple of
-// kTaskUnroll and then kTaskUnroll that are only read ahead.
-constexpr uint32_t kTaskWarps = 8;
+// off[w] .. off[w + 1] (in chunks of 32 * task_words words), the last
+// kTaskRing of them only read ahead.
+constexpr uint32_t kTaskWarps = 8;  // a block lane's CTA has at most this many
 struct TaskStream {
   std::vector<uint32_t> words;
   uint32_t off[kTaskWarps + 1] = {};
@@ -63,6 +63,7 @@ struct TaskStream {
 struct BlockPrograms {
   TaskStream a, b, f;
   uint32_t a_levels = 0;
+  bool compact = true;
 };
 
 // Every op reads final operands and every value's updates keep their
@@ -70,8 +71,8 @@ struct BlockPrograms {
 // sparse triangular solves.
 Programs compile_tape(const SparseLu& lu);
 
-// The block lanes' task streams.
-BlockPrograms compile_block(const Programs& P);
+// The block lanes' task streams for a CTA of `warps` warps (at most kTaskWarps).
+BlockPrograms compile_block(const Programs& P, uint32_t warps);
 
 constexpr uint32_t kRow = 32;
 

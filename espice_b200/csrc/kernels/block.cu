@@ -98,47 +98,50 @@ struct BlockMem {
   double* a64;  // nnz: the assembled matrix in FP64 (mixed form only)
   V* v;         // tape values | y | 0.0 | 1.0 | sink
   V* y;
+  uint32_t ring;  // the CTA's ring of task words (shared address)
 };
 
 // base: the working set (its hot part when split); cold: the CTA's slab
 // for a split layout's cold part.
 template <typename V>
-__device__ __forceinline__ BlockMem<V> block_carve(const BlockDev& D, unsigned char* base, unsigned char* cold) {
+__device__ __forceinline__ BlockMem<V> block_carve(const BlockDev& D, unsigned char* base, unsigned char* cold,
+                                                  unsigned char* ring = nullptr) {
   BlockMem<V> b;
-  unsigned char* cbase = D.split ? cold : base;
+  b.ring = ring ? static_cast<uint32_t>(__cvta_generic_to_shared(ring)) : 0u;
+  unsigned char* mid = D.split == 2 ? cold : base;
+  unsigned char* far = D.split ? cold : base;
   b.m.base = reinterpret_cast<double*>(base);
-  b.m.x = reinterpret_cast<double*>(base + D.o_x);
-  b.m.xo = reinterpret_cast<double*>(cbase + D.o_xo);
-  b.m.rhs = reinterpret_cast<double*>(base + D.o_rhs);
-  b.m.diag = reinterpret_cast<double*>(base + D.o_diag);
-  b.m.st = reinterpret_cast<double*>(cbase + D.o_st);
   b.m.lim = reinterpret_cast<double*>(base + D.o_lim);
-  b.m.v = nullptr;
-  b.m.y = nullptr;
-  b.dx = reinterpret_cast<double*>(base + D.o_dx);
-  b.a64 = reinterpret_cast<double*>(base + D.o_a64);
   b.v = reinterpret_cast<V*>(base + D.o_v);
   b.y = b.v + D.T.ntv;
+  b.m.x = reinterpret_cast<double*>(mid + D.o_x);
+  b.m.rhs = reinterpret_cast<double*>(mid + D.o_rhs);
+  b.m.diag = reinterpret_cast<double*>(mid + D.o_diag);
+  b.dx = reinterpret_cast<double*>(mid + D.o_dx);
+  b.a64 = reinterpret_cast<double*>(mid + D.o_a64);
+  b.m.xo = reinterpret_cast<double*>(far + D.o_xo);
+  b.m.st = reinterpret_cast<double*>(far + D.o_st);
+  b.m.v = nullptr;
+  b.m.y = nullptr;
   return b;
 }
 
-// Assembly as one streamed gather: thread t walks its term stream
-// (D.g_terms[k * kW + t], k < D.g_len) summing staging cells (the constant
-// cells for x[0], 1.0 and +0.0) from +0.0 in each cell's list order (the CSR order: the same bits as
-// the warp lanes' gather and the host factor's pattern copy); a term with
-// kGTermEnd closes a cell, whose destinations come from the thread's cell
+// Assembly as one streamed gather: thread t of warp w walks its term stream
+// (D.g_terms[k * kW + t], k < D.g_len[w]) summing staging cells (the constant
+// cells for x[0], 1.0 and +0.0) from +0.0 in each cell's list order (the CSR
+// order: the same bits as the warp lanes' gather and the host factor's
+// pattern copy); a term with kGTermEnd closes a cell, in every thread of the
+// warp at once, whose destinations come from the thread's cell
 // stream (D.g_cells[c * kW + t]): a pattern slot (its tape value, FP32 in the
 // mixed form which also keeps the FP64 sum, and the diagonal copy for the
-// gates) or a residual row (rhs and y = P(-rhs)). Term words arrive two
-// batches of eight ahead, staging values one batch ahead, cells two ahead.
+// gates) or a residual row (rhs and y = P(-rhs)). Two batches of eight take
+// turns: while one's terms are summed the other's staging values and the
+// term words of the batch after that are in flight (one rotating batch
+// waited for both at its register moves: 51k cycles an assembly of the
+// analog block, two CTAs an SM, against 36k).
 // gmin > 0 adds loadExtras' diagonal and residual terms; gs > 0 the
 // gmin-stepping rung's at the cells that carry a stamp (c.w: 1 on a stamped
 // slot, the column + 1 on a stamped row). Fill-in tape values are zeroed.
-template <typename V, uint32_t kW>
-__device__ __forceinline__ double gather_term(const BlockMem<V>& b, uint32_t w) {
-  return b.m.st[w & ~kGTermEnd];
-}
-
 template <typename V, uint32_t kW>
 __device__ __forceinline__ void gather_store(const BlockDev& D, const BlockMem<V>& b, const uint4& c, double s,
                                              double gmin, double gs) {
@@ -163,48 +166,52 @@ __device__ void block_assemble(const BlockDev& D, const BlockMem<V>& b, double g
   const TopoDev& T = D.T;
   const uint32_t* terms = D.g_terms + tid;
   const uint4* cells = D.g_cells + tid;
-  const uint32_t K = D.g_len, pad = T.n_stage + kGCellZero;
-  // Term words two batches ahead and staging values one batch ahead: every
-  // load of a batch is issued before the stores of the batch before it, so
-  // none waits behind them (the staging cells are only read here).
-  uint32_t w[8], nx[8];
-  double val[8];
+  const uint32_t K = D.g_len[tid >> 5];  // a multiple of 2 kGBatch, and 2 kGBatch more to read ahead
+  const double* st = b.m.st;
+  struct Batch {
+    uint32_t w[kGBatch];
+    double v[kGBatch];
+    uint32_t ends;
+  };
+  auto words = [&](Batch& x, uint32_t k) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    w[j] = uint32_t(j) < K ? __ldg(terms + size_t(j) * kW) : pad;
-    nx[j] = uint32_t(8 + j) < K ? __ldg(terms + size_t(8 + j) * kW) : pad;
-  }
+    for (uint32_t j = 0; j < kGBatch; ++j) x.w[j] = __ldg(terms + size_t(k + j) * kW);
+  };
+  auto values = [&](Batch& x) {
+    x.ends = 0;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) val[j] = gather_term<V, kW>(b, w[j]);
-  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-  uint4 cell = D.g_ncells > 0 ? __ldg(cells) : none;
-  uint4 cell1 = D.g_ncells > 1 ? __ldg(cells + kW) : none;
-  uint32_t c_next = 2;
+    for (uint32_t j = 0; j < kGBatch; ++j) {
+      x.v[j] = st[x.w[j] & ~kGTermEnd];
+      x.ends |= (x.w[j] >> 31) << j;
+    }
+  };
+  uint4 cell = __ldg(cells), next = __ldg(cells + kW);
+  cells += 2 * kW;
   double s = 0.0;
-  for (uint32_t k0 = 0; k0 < K; k0 += 8) {
-    uint32_t nnx[8];
-    double nv[8];
+  auto sum = [&](const Batch& x) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) nnx[j] = k0 + 16 + j < K ? __ldg(terms + size_t(k0 + 16 + j) * kW) : pad;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) nv[j] = gather_term<V, kW>(b, nx[j]);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      s = __dadd_rn(s, val[j]);
-      if (w[j] & kGTermEnd) {
+    for (uint32_t j = 0; j < kGBatch; ++j) {
+      s = __dadd_rn(s, x.v[j]);
+      if (x.ends >> j & 1u) {
         gather_store<V, kW>(D, b, cell, s, gmin, gs);
         s = 0.0;
-        cell = cell1;
-        cell1 = c_next < D.g_ncells ? __ldg(cells + size_t(c_next) * kW) : none;
-        ++c_next;
+        cell = next;
+        next = __ldg(cells);
+        cells += kW;
       }
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      w[j] = nx[j];
-      nx[j] = nnx[j];
-      val[j] = nv[j];
-    }
+  };
+  Batch p, q;
+  words(p, 0);
+  words(q, kGBatch);
+  values(p);
+  for (uint32_t k = 0; k < K; k += 2 * kGBatch) {
+    words(p, k + 2 * kGBatch);
+    values(q);
+    sum(p);
+    words(q, k + 3 * kGBatch);
+    values(p);
+    sum(q);
   }
   for (uint32_t j = tid; j < T.n_fill; j += kW) b.v[T.fill[j]] = V(0);
 }
@@ -212,28 +219,37 @@ __device__ void block_assemble(const BlockDev& D, const BlockMem<V>& b, double g
 // One of the programs over the lane's values; this thread's pivot-test
 // failures. Ends in a CTA barrier (a program without tasks has none).
 template <typename V>
-__device__ __forceinline__ bool block_program(const BlockDev& D, const BlockProgram& p, V* v) {
-  const uint32_t w = threadIdx.x >> 5, first = p.off[w], chunks = p.off[w + 1] - first - kTaskUnroll;
-  return (D.in_smem ? run_tasks<V, true>(p.words, first, chunks, v) : run_tasks<V, false>(p.words, first, chunks, v)) !=
-         0;
+__device__ __forceinline__ bool block_program(const BlockDev& D, const BlockProgram& p, const BlockMem<V>& b) {
+  const uint32_t w = threadIdx.x >> 5, first = p.off[w], chunks = p.off[w + 1] - first - kTaskRing;
+  uint32_t bad;
+  if (D.compact)
+    bad = D.in_smem ? run_tasks<V, true, true>(p.words, first, chunks, b.ring, b.v)
+                    : run_tasks<V, false, true>(p.words, first, chunks, b.ring, b.v);
+  else
+    bad = D.in_smem ? run_tasks<V, true, false>(p.words, first, chunks, b.ring, b.v)
+                    : run_tasks<V, false, false>(p.words, first, chunks, b.ring, b.v);
+  return bad != 0;
 }
 
-// Refactor + forward solve (program A), then the lane kernels' peel tests on
+// Refactor + forward solve (program A) with the lane kernels' peel tests on
 // the finished tape values (lane_kernels.zig Bodies.refactor and
 // LaneSolver.wideMultipliers). CTA-uniform verdict.
 template <typename V, uint32_t kW>
-__device__ bool block_refactor(const BlockDev& D, V* v, int tid) {
+__device__ bool block_refactor(const BlockDev& D, const BlockMem<V>& b, int tid) {
   const TopoDev& T = D.T;
-  bool bad = block_program(D, D.a, v);
-  const uint32_t l0 = T.nu + T.n;
-  for (uint32_t s = tid; s < T.nu; s += kW)
-    if (!(fabs(v[s]) < inf_of(v[s]))) bad = true;
-  for (uint32_t k = tid; k < T.n; k += kW) {
-    const V d = v[T.nu + k];
-    if (d == V(0) || !(fabs(d) < inf_of(d))) bad = true;
+  bool bad = block_program(D, D.a, b);
+  const V* v = b.v;
+  // the L entries were tested where they were divided; U and the diagonal
+  // lie side by side, read 16 bytes at a time
+  constexpr uint32_t kPer = 16 / sizeof(V);
+  const uint32_t m = T.nu + T.n;
+  for (uint32_t s = tid * kPer; s < m; s += kW * kPer) {
+    V x[kPer];
+    *reinterpret_cast<uint4*>(x) = *reinterpret_cast<const uint4*>(v + s);
+#pragma unroll
+    for (uint32_t j = 0; j < kPer; ++j)
+      bad |= s + j < m && (!task_finite(x[j]) || (s + j >= T.nu && x[j] == V(0)));
   }
-  for (uint32_t s = tid; s < T.nl; s += kW)
-    if (!T.l_scaled[s] && !(fabs(v[l0 + s]) <= V(1e3))) bad = true;
   return __syncthreads_or(bad) != 0;
 }
 
@@ -260,8 +276,8 @@ __device__ uint32_t block_refine(const BlockDev& D, const BlockMem<float>& b, ui
     rmax = block_max_abs<kW>(rmax, red);
     bmax = block_max_abs<kW>(bmax, red);
     if (!(rmax > D.refine_tol * bmax) || it >= D.refine_max) break;
-    block_program(D, D.f, b.v);
-    block_program(D, D.b, b.v);
+    block_program(D, D.f, b);
+    block_program(D, D.b, b);
     for (uint32_t j = tid; j < T.n; j += kW) {
       const uint32_t i = T.qcol[j];
       b.dx[i] = __dadd_rn(b.dx[i], double(b.y[j]));
@@ -311,7 +327,8 @@ __device__ __forceinline__ void phase_mark(unsigned long long* prof, uint32_t ph
 // dc_solve_lane step for step, reductions across the CTA.
 template <typename V, bool kHasB3, uint32_t kW, bool kLadder = false>
 __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& o, unsigned char* base,
-                           unsigned char* cold, uint64_t* red, uint32_t lane, const LadderDev* ld = nullptr) {
+                           unsigned char* cold, unsigned char* ring, uint64_t* red, uint32_t lane,
+                           const LadderDev* ld = nullptr) {
   constexpr bool kMixed = sizeof(V) == 4;
   const TopoDev& T = D.T;
   const int tid = threadIdx.x;
@@ -320,7 +337,7 @@ __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& 
   if (!(status == kRunning || resuming)) return;
 
   const uint32_t n = T.n;
-  const BlockMem<V> b = block_carve<V>(D, base, cold);
+  const BlockMem<V> b = block_carve<V>(D, base, cold, ring);
   const LaneMem& m = b.m;
   const double* rec = L.rec + size_t(lane) * T.rec_size;
   for (uint32_t i = tid; i < n; i += kW) m.x[i] = L.x[size_t(lane) * n + i];
@@ -384,7 +401,7 @@ __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& 
       }
       const bool host_mode = (flags & 2u) != 0;
       bool bad = true;
-      if (!host_mode) bad = block_refactor<V, kW>(D, b.v, tid);
+      if (!host_mode) bad = block_refactor<V, kW>(D, b, tid);
       phase_mark(D.prof, kBlockPhaseRefactor, t0);
       if (bad) {
         // Pause: the host factors this lane with its own FP64 direct solver.
@@ -407,7 +424,7 @@ __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& 
         }
         return;
       }
-      block_program(D, D.b, b.v);
+      block_program(D, D.b, b);
       for (uint32_t j = tid; j < n; j += kW) b.dx[T.qcol[j]] = double(b.y[j]);
       __syncthreads();
       phase_mark(D.prof, kBlockPhaseSolve, t0);
@@ -477,25 +494,26 @@ __device__ void block_lane(const BlockDev& D, const LaneDev& L, const LaneOpts& 
 // Persistent grid: each CTA takes lanes blockIdx.x, + gridDim.x, ...; its
 // working set in dynamic shared memory, split between shared memory and its
 // slab of D.slab, or all in its slab. Dynamic shared memory: the working set
-// (its hot part when split; nothing when all in the slab).
-// Two CTAs an SM by registers (the BSIM3 instantiation spills a few words
-// of its evaluation for it), as many as shared memory then allows.
+// (its hot part when split; nothing when all in the slab), behind the ring of
+// task words.
+// 512 threads an SM by registers (128 each: the BSIM3 instantiation spills a
+// few words of its evaluation for it), as shared memory then allows.
 template <typename V, bool kHasB3, uint32_t kW, bool kLadder>
-__global__ void __launch_bounds__(kW, 2) dc_block_kernel(BlockDev D, LaneDev L, LaneOpts o) {
+__global__ void __launch_bounds__(kW, 512 / kW) dc_block_kernel(BlockDev D, LaneDev L, LaneOpts o) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t red[kW / 32];
   unsigned char* own = D.slab + size_t(blockIdx.x) * (D.split ? D.cold_bytes : D.lane_bytes);
-  unsigned char* base = D.in_smem ? smem_raw : own;
+  unsigned char* base = D.in_smem ? smem_raw + D.ring_bytes : own;
   for (uint32_t lane = blockIdx.x; lane < L.n_lanes; lane += gridDim.x) {
     if constexpr (!kLadder) {
-      block_lane<V, kHasB3, kW>(D, L, o, base, own, red, lane);
+      block_lane<V, kHasB3, kW>(D, L, o, base, own, smem_raw, red, lane);
     } else {
       // an operating-point lane runs Newton until the ladder is done or the
       // lane pauses for a host factor (a singular host factor ends a run)
       for (;;) {
         const uint32_t st = *(volatile uint32_t*)(L.status + lane);
         if (st == kRunning || (L.resume && st == kNeedSolve)) {
-          block_lane<V, kHasB3, kW, true>(D, L, o, base, own, red, lane, L.ladder + lane);
+          block_lane<V, kHasB3, kW, true>(D, L, o, base, own, smem_raw, red, lane, L.ladder + lane);
           __syncthreads();
           if (*(volatile uint32_t*)(L.status + lane) == kNeedSolve) break;
         } else if (!(st == kSingular && L.ladder[lane].rung != kRungDone)) {
@@ -537,31 +555,10 @@ __global__ void __launch_bounds__(kW, 2) dc_block_group_kernel(const BlockDev* _
       L = Ls[w.x];
     }
     __syncthreads();
-    block_lane<V, kHasB3, kW>(D, L, o, D.in_smem ? smem_raw : own_slab, own_slab, red, w.y, nullptr);
+    block_lane<V, kHasB3, kW>(D, L, o, D.in_smem ? smem_raw + D.ring_bytes : own_slab, own_slab, smem_raw,
+                                   red, w.y, nullptr);
     __syncthreads();
   }
-}
-
-template <typename V, bool kHasB3, uint32_t kW>
-cudaError_t launch_group_t(const BlockDev* Ds, const LaneDev* Ls, const uint2* items, uint32_t n_items,
-                           uint32_t* next, const LaneOpts& o, unsigned char* slab, size_t slab_stride, size_t smem,
-                           uint32_t grid, cudaStream_t s) {
-  auto* k = dc_block_group_kernel<V, kHasB3, kW>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(next, 0, sizeof(uint32_t), s);
-  if (e != cudaSuccess) return e;
-  k<<<grid, kW, smem, s>>>(Ds, Ls, items, n_items, next, o, slab, slab_stride);
-  return cudaGetLastError();
-}
-
-template <typename V, bool kHasB3, uint32_t kW>
-int group_occupancy_t(size_t smem) {
-  int per_sm = 0;
-  auto* k = dc_block_group_kernel<V, kHasB3, kW>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, int(kW), smem);
-  return per_sm;
 }
 
 // The lead lane's first Jacobian in pattern order (its device evaluation at
@@ -585,30 +582,39 @@ __global__ void __launch_bounds__(kW) block_lead_kernel(BlockDev D, LaneDev L, u
   gather_pattern<kW>(T, b.m, out, tid);
 }
 
+// The DC kernel of a CTA width.
+template <typename V, bool kHasB3>
+auto dc_kernel(uint32_t threads) {
+  return threads == kBlockNarrow ? dc_block_kernel<V, kHasB3, kBlockNarrow, false>
+                                 : dc_block_kernel<V, kHasB3, kBlockThreads, false>;
+}
+
 template <typename V, bool kHasB3>
 cudaError_t launch_t(const BlockDev& D, const LaneDev& L, const LaneOpts& o, cudaStream_t s) {
   // operating-point lanes: the FP64 form with the ladder between runs
-  auto* k = dc_block_kernel<V, kHasB3, kBlockThreads, false>;
+  auto* k = dc_kernel<V, kHasB3>(D.threads);
   if (o.ladder) {
-    if constexpr (sizeof(V) == 8)
+    if constexpr (sizeof(V) == 8) {
+      if (D.threads != kBlockThreads) return cudaErrorNotSupported;
       k = dc_block_kernel<V, kHasB3, kBlockThreads, true>;
-    else
+    } else {
       return cudaErrorNotSupported;
+    }
   }
-  const size_t smem = (D.in_smem ? D.lane_bytes : 0);
+  const size_t smem = D.ring_bytes + (D.in_smem ? D.lane_bytes : 0);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   const uint32_t grid = D.grid < L.n_lanes ? D.grid : L.n_lanes;
-  k<<<grid > 0 ? grid : 1, kBlockThreads, smem, s>>>(D, L, o);
+  k<<<grid > 0 ? grid : 1, D.threads, smem, s>>>(D, L, o);
   return cudaGetLastError();
 }
 
 template <typename V, bool kHasB3>
-int occupancy_t(size_t smem) {
+int occupancy_t(uint32_t threads, size_t smem) {
   int per_sm = 0;
-  auto* k = dc_block_kernel<V, kHasB3, kBlockThreads, false>;
+  auto* k = dc_kernel<V, kHasB3>(threads);
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, int(kBlockThreads), smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, int(threads), smem);
   return per_sm;
 }
 
@@ -748,11 +754,11 @@ __device__ int block_tran_newton(const BlockDev& D, const BlockMem<V>& b, const 
       const double scale = fmin(fmax(from_bits(xm), from_bits(fm) * gd), 1e18);
       limit = !(1e3 * scale > kXPlausible) ? kXPlausible : 1e3 * scale;
     }
-    if (block_refactor<V, kW>(D, b.v, tid)) {
+    if (block_refactor<V, kW>(D, b, tid)) {
       iters = iter + 1;
       return 2;
     }
-    block_program(D, D.b, b.v);
+    block_program(D, D.b, b);
     for (uint32_t j = tid; j < n; j += kW) b.dx[T.qcol[j]] = double(b.y[j]);
     __syncthreads();
     if constexpr (kMixed) refinements += block_refine_step<kW>(D, b, o, red, tid);
@@ -815,12 +821,12 @@ __host__ __device__ inline size_t tran_block_slab_doubles(const TopoDev& T) {
 // predictor, LTE control, order promotion and source breakpoints.
 template <typename V, bool kHasB3, uint32_t kW>
 __device__ void block_tran_lane(const BlockDev& D, const LaneDev& L, const TranDev& P, const LaneOpts& o,
-                                unsigned char* base, unsigned char* cold, double* tslab,
+                                unsigned char* base, unsigned char* cold, unsigned char* ring, double* tslab,
                                 uint64_t* red, uint32_t lane) {
   const TopoDev& T = D.T;
   const int tid = threadIdx.x;
   const uint32_t n = T.n, nq = T.n_qt;
-  const BlockMem<V> b = block_carve<V>(D, base, cold);
+  const BlockMem<V> b = block_carve<V>(D, base, cold, ring);
   uint32_t refinements = 0;
   const LaneMem& m = b.m;
   double* cur = tslab;
@@ -1109,10 +1115,10 @@ __global__ void __launch_bounds__(kW, 2) tran_block_kernel(BlockDev D, LaneDev L
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t red[kW / 32];
   unsigned char* own = D.slab + size_t(blockIdx.x) * (D.split ? D.cold_bytes : D.lane_bytes);
-  unsigned char* base = D.in_smem ? smem_raw : own;
+  unsigned char* base = D.in_smem ? smem_raw + D.ring_bytes : own;
   double* ts = tslab + size_t(blockIdx.x) * tslab_stride;
   for (uint32_t lane = blockIdx.x; lane < L.n_lanes; lane += gridDim.x) {
-    block_tran_lane<V, kHasB3, kW>(D, L, P, o, base, own, ts, red, lane);
+    block_tran_lane<V, kHasB3, kW>(D, L, P, o, base, own, smem_raw, ts, red, lane);
     __syncthreads();
   }
 }
@@ -1121,7 +1127,7 @@ template <typename V, bool kHasB3>
 cudaError_t launch_tran_t(const BlockDev& D, const LaneDev& L, const TranDev& P, const LaneOpts& o, double* tslab,
                           size_t tslab_stride, cudaStream_t s) {
   auto* k = tran_block_kernel<V, kHasB3, kBlockThreads>;
-  const size_t smem = (D.in_smem ? D.lane_bytes : 0);
+  const size_t smem = D.ring_bytes + (D.in_smem ? D.lane_bytes : 0);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   const uint32_t grid = D.grid < L.n_lanes ? D.grid : L.n_lanes;
@@ -1151,8 +1157,8 @@ cudaError_t launch_tran_block(const BlockDev& D, const LaneDev& L, const TranDev
   ESL_BLOCK_DISPATCH(launch_tran_t, D, L, P, o, tslab, stride, s);
 }
 
-int block_occupancy(bool mixed, bool has_b3, size_t smem) {
-  ESL_BLOCK_DISPATCH(occupancy_t, smem);
+int block_occupancy(bool mixed, bool has_b3, uint32_t threads, size_t smem) {
+  ESL_BLOCK_DISPATCH(occupancy_t, threads, smem);
 }
 
 cudaError_t launch_dc_block_group(const BlockDev* d_Ds, const LaneDev* d_Ls, const uint2* d_items, uint32_t n_items,

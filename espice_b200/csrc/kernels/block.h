@@ -13,6 +13,8 @@ namespace esl {
 
 // Threads of a block lane's CTA (its program rows are this wide).
 constexpr uint32_t kBlockThreads = 256;
+// Threads of the narrow form, for more lanes an SM (DC lanes).
+constexpr uint32_t kBlockNarrow = 128;
 // The block lanes' assembly streams (see block_assemble): a term word is a
 // staging index, with kGTermEnd on a cell's last term. Three cells past the
 // device stamps hold constants, so every term is a plain load: n_stage +
@@ -24,6 +26,7 @@ constexpr uint32_t kBlockThreads = 256;
 constexpr uint32_t kGTermEnd = 0x80000000u;
 constexpr uint32_t kGCellZero = 0, kGCellOne = 1, kGCellX0 = 2, kGConstCells = 3;
 constexpr uint32_t kGCellRow = 0x80000000u;
+constexpr uint32_t kGBatch = 8;  // terms a thread takes at a time, two batches in turn
 
 // A task program (host/schedule.hpp TaskStream): its words, and each warp's
 // chunks.
@@ -37,21 +40,24 @@ struct BlockDev {
   // Programs A (refactor + forward solve), B (back solve) and F (forward
   // solve alone).
   BlockProgram a, b, f;
-  // The assembly: term stream [g_len][kBlockThreads], cell stream
-  // [g_ncells][kBlockThreads] (uint4).
+  uint32_t compact;     // the programs' word form (common.h)
+  uint32_t ring_bytes;  // the CTA's ring of task words, first in its dynamic shared memory
+  // The assembly: term stream [k][threads], warp w's first g_len[w] summed
+  // (block_assemble), cell stream [c][threads] (uint4).
   const uint32_t* g_terms;
   const uint4* g_cells;
-  uint32_t g_len, g_ncells;
-  // A lane's working set, byte offsets: the hot part x, rhs, diag, dx (FP64,
-  // n each), limited images, the FP64 matrix (mixed form: nnz), the value
-  // space v (FP64, or FP32 in the mixed form); then the cold part xo (n) and
-  // the staging cells. Split: the cold part lives apart, in the CTA's slab
-  // (its offsets from there), so that more CTAs fit an SM's shared memory.
+  uint32_t g_len[kBlockThreads / 32];
+  // A lane's working set, byte offsets: limited images, the value space v
+  // (FP64, or FP32 in the mixed form), x, rhs, diag, dx (FP64, n each), the
+  // FP64 matrix (mixed form: nnz), xo (n) and the staging cells. Split: a
+  // tail of it lives apart, in the CTA's slab (its offsets from there), so
+  // that more CTAs fit an SM's shared memory.
   uint32_t o_x, o_xo, o_rhs, o_diag, o_dx, o_st, o_lim, o_a64, o_v;
   uint32_t lane_bytes;  // the working set (split: its hot part), 16-byte aligned
   uint32_t in_smem;     // 1: (the hot part) in the CTA's shared memory; 0: all in its slab of `slab`
-  uint32_t split;       // 1: the cold part in the CTA's slab, cold_bytes each
+  uint32_t split;       // 1: xo and the staging cells in the CTA's slab; 2: all from x on; cold_bytes each
   uint32_t cold_bytes;
+  uint32_t threads;     // of a CTA (kBlockThreads or kBlockNarrow)
   uint32_t grid;        // CTAs of a launch (persistent)
   unsigned char* slab;  // per CTA: the working set (in_smem 0) or its cold part (split), and the lead assembly's scratch
   // Mixed form: refinement stops at max |res| <= refine_tol * max |rhs| or
@@ -84,8 +90,8 @@ enum BlockPhase : uint32_t {
 // values with FP64 refinement; has_b3: the BSIM3 instantiation.
 cudaError_t launch_dc_block(const BlockDev& D, const LaneDev& L, const LaneOpts& o, bool mixed, bool has_b3,
                             cudaStream_t s);
-// CTAs per SM of the DC kernel at this precision and dynamic shared memory.
-int block_occupancy(bool mixed, bool has_b3, size_t smem);
+// CTAs per SM of the DC kernel at this precision, CTA width and dynamic shared memory.
+int block_occupancy(bool mixed, bool has_b3, uint32_t threads, size_t smem);
 // Uneven batching: the lanes of several topologies (device arrays of their
 // BlockDev and LaneDev) in one persistent launch over work items (topology,
 // lane), taken from the counter d_next in order; smem: the largest working

@@ -28,31 +28,45 @@ __device__ __forceinline__ Dual dmul(Dual a, Dual b) {
 }
 // a * c, c a constant
 __device__ __forceinline__ Dual dscl(Dual a, double c) { return {a.v * c, a.g * c, a.d * c, a.b * c}; }
-__device__ __forceinline__ Dual ddiv(Dual a, Dual b) {
-  const double q = div_rn(a.v, b.v);
-  return {q, div_rn(a.g - q * b.g, b.v), div_rn(a.d - q * b.d, b.v), div_rn(a.b - q * b.b, b.v)};
+// The quotients of one dual division share their divisor (models.cuh
+// Divisor). The divisions and functions are calls: inlined, the chain is some
+// sixty of them, and its instructions alone outgrow the SM's instruction
+// caches (analog block, mixed, four CTAs an SM: 152k cycles an evaluation
+// inlined, 134k called).
+static __device__ __noinline__ Dual ddiv(Dual a, Dual b) {
+  const Divisor by(b.v);
+  const double q = by.quot(a.v);
+  double g = a.g - q * b.g, d = a.d - q * b.d, e = a.b - q * b.b;
+  by.quot3(g, d, e);
+  return {q, g, d, e};
 }
 // a / c, c a constant
-__device__ __forceinline__ Dual ddivk(Dual a, double c) {
-  return {div_rn(a.v, c), div_rn(a.g, c), div_rn(a.d, c), div_rn(a.b, c)};
+static __device__ __noinline__ Dual ddivk(Dual a, double c) {
+  const Divisor by(c);
+  const double q = by.quot(a.v);
+  by.quot3(a.g, a.d, a.b);
+  return {q, a.g, a.d, a.b};
 }
 // c / b, c a constant
-__device__ __forceinline__ Dual dkdiv(double c, Dual b) {
-  const double q = div_rn(c, b.v);
-  const double s = div_rn(-q, b.v);
+static __device__ __noinline__ Dual dkdiv(double c, Dual b) {
+  const Divisor by(b.v);
+  const double q = by.quot(c);
+  const double s = by.quot(-q);
   return {q, s * b.g, s * b.d, s * b.b};
 }
-__device__ __forceinline__ Dual dsqrt(Dual a) {
+static __device__ __noinline__ Dual dsqrt(Dual a) {
   const double s = sqrt(a.v);
   const double h = div_rn(0.5, s);
   return {s, a.g * h, a.d * h, a.b * h};
 }
-__device__ __forceinline__ Dual dexp(Dual a) {
+static __device__ __noinline__ Dual dexp(Dual a) {
   const double e = esl_exp(a.v);
   return {e, a.g * e, a.d * e, a.b * e};
 }
-__device__ __forceinline__ Dual dlog(Dual a) {
-  return {esl_log(a.v), div_rn(a.g, a.v), div_rn(a.d, a.v), div_rn(a.b, a.v)};
+static __device__ __noinline__ Dual dlog(Dual a) {
+  const Divisor by(a.v);
+  by.quot3(a.g, a.d, a.b);
+  return {esl_log(a.v), a.g, a.d, a.b};
 }
 // a + c and c - a, c a constant
 __device__ __forceinline__ Dual daddk(Dual a, double c) { return {a.v + c, a.g, a.d, a.b}; }

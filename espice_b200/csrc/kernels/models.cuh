@@ -26,6 +26,56 @@ __device__ __forceinline__ double div_rn(double a, double b) {
   return __ddiv_rn(a, b);
 }
 
+// Exponents within 2^-511 .. 2^511 (finite, normal, quotients too).
+__device__ __forceinline__ bool mid_range(double x) {
+  return (static_cast<uint32_t>(__double2hiint(x)) & 0x7fffffffu) - 0x20000000u < 0x3fe00000u;
+}
+
+// Quotients by one divisor, each correctly rounded (bitwise div_rn). The
+// reciprocal is taken once, correctly rounded; a quotient is then the product
+// and two residual corrections (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. R&D 34, 1990,
+// theorem 8.3: with a correctly rounded reciprocal, correcting a quotient
+// that is within one ulp by its exact residual rounds correctly). A
+// division alone is a chain of about 115 cycles with a branch, so four of
+// them do not overlap; four of these do, in about 60 cycles beyond the
+// reciprocal. Operands outside mid_range take div_rn; a zero dividend keeps
+// the product's signed zero.
+struct Divisor {
+  double b, r;
+  bool mid;
+  __device__ __forceinline__ explicit Divisor(double d) {
+    b = d;
+    r = __drcp_rn(d);
+    mid = mid_range(d);
+  }
+  __device__ __forceinline__ bool takes(double a) const { return mid && (a == 0.0 || mid_range(a)); }
+  // a / b for an `a` this takes
+  __device__ __forceinline__ double near(double a) const {
+    const double q0 = __dmul_rn(a, r);
+    const double q1 = __fma_rn(__fma_rn(-b, q0, a), r, q0);
+    const double q2 = __fma_rn(__fma_rn(-b, q1, a), r, q1);
+    return a == 0.0 ? q0 : q2;
+  }
+  __device__ __forceinline__ double quot(double a) const {
+    double q = near(a);
+    if (!takes(a)) q = div_rn(a, b);
+    return q;
+  }
+  __device__ __forceinline__ void quot3(double& x, double& y, double& z) const {
+    const double p = near(x), q = near(y), r3 = near(z);
+    if (takes(x) && takes(y) && takes(z)) {
+      x = p;
+      y = q;
+      z = r3;
+    } else {
+      x = div_rn(x, b);
+      y = div_rn(y, b);
+      z = div_rn(z, b);
+    }
+  }
+};
+
 struct SimDev {
   double t;          // time (transient)
   double src_scale;  // source-stepping factor

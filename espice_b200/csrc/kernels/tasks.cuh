@@ -4,14 +4,18 @@
 // row to row by barriers.
 //
 // What bounds it is the chain of rows, not the arithmetic: a row costs a
-// warp's in-order pass through one chunk (about 340 cycles with three
-// updates, 165 more with a division; B200, all eight warps in step) and the
-// barrier (50). So a row does as much as it can: a value stays in a register
-// over its updates and its division, every operand of a chunk is loaded
-// before the first is used, selects stand in place of branches, and the next
-// chunks' words are already in registers (read kTaskUnroll ahead, straight
-// from L2: a ring in shared memory is 5% faster alone, but its 24 KB cost
-// the second CTA of an SM).
+// warp's in-order pass through one chunk and the barrier. So a row does as
+// much as it can: a value stays in a register over its updates and its
+// division, every operand of a chunk is loaded before the first is used, and
+// selects stand in place of branches. The words stream from L2 through a
+// ring of four chunks a warp by cp.async: loads into registers, three chunks
+// ahead, share the warp's few scoreboards with the operands' loads, which
+// then wait for L2 as well (analog block, mixed, two CTAs an SM: 210k cycles a
+// refactor; one chunk ahead 260k; through the ring 142k).
+//
+// A division tests its pivot as the CPU replay does (growth, or a finite
+// quotient in a row-scaled column), and in a column without row scaling
+// also the L entry it makes against the wide-multiplier bound.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -98,32 +102,68 @@ struct TaskMem<float, false> {
   }
 };
 
-// One lane's task of a chunk (common.h), read past L1: a CTA reads each once.
-struct TaskChunk {
-  uint4 h, u;
-  __device__ __forceinline__ void load(const uint4* p) {
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(h.x), "=r"(h.y), "=r"(h.z), "=r"(h.w)
-                 : "l"(p));
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
-                 : "l"(p + 32));
+__device__ __forceinline__ uint4 task_lds(uint32_t at) {
+  uint4 r;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(at));
+  return r;
+}
+__device__ __forceinline__ void task_copy(uint32_t to, const uint4* from) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+}
+__device__ __forceinline__ void task_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void task_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// One lane's task words (common.h), from a ring slot.
+template <bool kCompact>
+struct TaskLane;
+template <>
+struct TaskLane<true> {
+  static constexpr uint32_t kBytes = 512;  // a chunk
+  uint4 c;
+  __device__ __forceinline__ void load(uint32_t at) { c = task_lds(at); }
+  static __device__ __forceinline__ void copy(uint32_t to, const uint4* from) { task_copy(to, from); }
+  __device__ __forceinline__ uint32_t flags() const { return c.x >> 16; }
+  __device__ __forceinline__ uint32_t dst() const { return c.x & 0xffffu; }
+  __device__ __forceinline__ uint32_t idle() const { return c.y; }
+  __device__ __forceinline__ uint32_t a(int j) const { return (j == 0 ? c.y : j == 1 ? c.z : c.w) & 0xffffu; }
+  __device__ __forceinline__ uint32_t b(int j) const { return (j == 0 ? c.y : j == 1 ? c.z : c.w) >> 16; }
+};
+template <>
+struct TaskLane<false> {
+  static constexpr uint32_t kBytes = 1024;
+  uint4 c, e;
+  __device__ __forceinline__ void load(uint32_t at) {
+    c = task_lds(at);
+    e = task_lds(at + 512);
   }
+  static __device__ __forceinline__ void copy(uint32_t to, const uint4* from) {
+    task_copy(to, from);
+    task_copy(to + 512, from + 32);
+  }
+  __device__ __forceinline__ uint32_t flags() const { return c.y; }
+  __device__ __forceinline__ uint32_t dst() const { return c.x; }
+  __device__ __forceinline__ uint32_t idle() const { return c.z; }
+  __device__ __forceinline__ uint32_t a(int j) const { return j == 0 ? c.z : j == 1 ? e.x : e.z; }
+  __device__ __forceinline__ uint32_t b(int j) const { return j == 0 ? c.w : j == 1 ? e.y : e.w; }
 };
 
-template <typename V, bool kShared>
-__device__ __forceinline__ void run_task(const TaskChunk& c, const TaskMem<V, kShared>& v, uint32_t& bad) {
-  const uint32_t w0 = c.h.x, w1 = c.h.y, dst = w0 & kTaskIndex;
-  if (dst == kTaskIdle) {
-    for (uint32_t k = w1; k; --k) __syncthreads();
+template <typename V, bool kShared, bool kCompact>
+__device__ __forceinline__ void run_task(const TaskLane<kCompact>& c, const TaskMem<V, kShared>& v, uint32_t& bad) {
+  const uint32_t f = c.flags();
+  if (f & kTaskIdle) {
+    for (uint32_t k = c.idle(); k; --k) __syncthreads();
     return;
   }
-  const bool all = !(w0 & kTaskNz);
+  const uint32_t dst = c.dst();
+  const bool all = !(f & kTaskNz), div = f & kTaskDiv;
   V d = v.ld(dst);
-  const V a0 = v.ld(c.h.z), b0 = v.ld(c.h.w), piv = v.ld(w1 & kTaskIndex);
-  if (w0 & kTaskMore) {
-    const V a1 = v.ld(c.u.x), b1 = v.ld(c.u.y), a2 = v.ld(c.u.z), b2 = v.ld(c.u.w);
-    const bool r0 = b0 != V(0) || all, r1 = b1 != V(0) || all, r2 = b2 != V(0) || all;
+  const V a0 = v.ld(c.a(0)), b0 = v.ld(c.b(0)), a2 = v.ld(c.a(2));
+  if (f & kTaskMore) {
+    const V a1 = v.ld(c.a(1)), b1 = v.ld(c.b(1)), b2 = v.ld(c.b(2));
+    const bool r0 = b0 != V(0) || all, r1 = b1 != V(0) || all, r2 = (b2 != V(0) || all) && !div;
     V t = task_msub(d, a0, b0);
     d = r0 ? t : d;
     t = task_msub(d, a1, b1);
@@ -135,40 +175,53 @@ __device__ __forceinline__ void run_task(const TaskChunk& c, const TaskMem<V, kS
     const V t = task_msub(d, a0, b0);
     d = r0 ? t : d;
   }
-  if (w1 & kTaskDivAny) {
-    const V q = task_div(d, piv);
-    const bool shrunk = !(fabs(piv) >= task_growth(piv) * fabs(d)), wild = !task_finite(q);
-    bad |= (uint32_t(shrunk) & (w1 / kTaskGrowth)) | (uint32_t(wild) & (w1 / kTaskScaled));
-    d = (w0 & kTaskDiv) ? q : d;
+  if (f & kTaskDivAny) {
+    const V q = task_div(d, a2);
+    const bool shrunk = !(fabs(a2) >= task_growth(a2) * fabs(d) && fabs(q) <= V(1e3)), wild = !task_finite(q);
+    bad |= (uint32_t(shrunk) & (f / kTaskGrowth)) | (uint32_t(wild) & (f / kTaskScaled));
+    d = div ? q : d;
   }
   v.st(dst, d);
-  if (w0 & kTaskCta) __syncthreads();
+  if (f & kTaskCta) __syncthreads();
   else __syncwarp();
 }
 
-// Runs a warp's `chunks` (a multiple of kTaskUnroll) from `first` of a
-// program's words. Returns bit 0 set when a division of this thread failed
-// its pivot test.
-template <typename V, bool kShared>
-__device__ __noinline__ uint32_t run_tasks(const uint32_t* words, uint32_t first, uint32_t chunks, V* values) {
-  constexpr uint32_t kStep = 8 * kTaskWords;  // uint4 a chunk
-  const uint4* s = reinterpret_cast<const uint4*>(words) + size_t(first) * kStep + (threadIdx.x & 31);
+// Runs a warp's `chunks` from `first` of a program's words, streamed through
+// the warp's part of the ring (shared address): while a chunk runs, the next
+// one's words are on their way into registers and the two after that into
+// the ring. Returns bit 0 set when a division of this thread failed its
+// pivot test.
+template <typename V, bool kShared, bool kCompact>
+__device__ __noinline__ uint32_t run_tasks(const uint32_t* words, uint32_t first, uint32_t chunks, uint32_t ring,
+                                           V* values) {
+  using Lane = TaskLane<kCompact>;
+  constexpr uint32_t kBytes = Lane::kBytes, kStep = kBytes / 16, kSpan = kTaskRing * kBytes;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint4* s = reinterpret_cast<const uint4*>(words) + size_t(first) * kStep + lane;
+  const uint32_t base = ring + (threadIdx.x >> 5) * kSpan + 16 * lane;
   const TaskMem<V, kShared> v(values);
-  static_assert(kTaskUnroll == 3, "three chunks in registers");
-  TaskChunk c0, c1, c2;
-  c0.load(s);
-  c1.load(s + kStep);
-  c2.load(s + 2 * kStep);
-  uint32_t bad = 0;
-  for (uint32_t k = 0; k < chunks; k += kTaskUnroll) {
-    s += kTaskUnroll * kStep;
-    run_task(c0, v, bad);
-    c0.load(s);
-    run_task(c1, v, bad);
-    c1.load(s + kStep);
-    run_task(c2, v, bad);
-    c2.load(s + 2 * kStep);
+#pragma unroll
+  for (uint32_t k = 0; k + 1 < kTaskRing; ++k) {
+    Lane::copy(base + k * kBytes, s);
+    task_commit();
+    s += kStep;
   }
+  uint32_t bad = 0, read = 0, fill = (kTaskRing - 1) * kBytes;
+  Lane c, next;
+  task_wait<kTaskRing - 2>();
+  c.load(base);
+  for (uint32_t k = 0; k < chunks; ++k) {
+    Lane::copy(base + fill, s);
+    task_commit();
+    s += kStep;
+    read = (read + kBytes) & (kSpan - 1);
+    fill = (fill + kBytes) & (kSpan - 1);
+    task_wait<kTaskRing - 2>();
+    next.load(base + read);
+    run_task<V, kShared, kCompact>(c, v, bad);
+    c = next;
+  }
+  task_wait<0>();
   return bad & 1u;
 }
 
