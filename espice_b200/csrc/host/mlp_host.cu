@@ -72,7 +72,8 @@ struct esl_mlp {
   Dev<float> dz, dh, t, loss, xf;
   Dev<__nv_bfloat16> dzb, dzt;
   Dev<int> gerr;
-  Dev<uint32_t> idx;
+  Dev<uint32_t> perm, at;        // training: an epoch's order, the step within it
+  Dev<esl::AdamRate> rates;      // and each step's rate and bias corrections
 
   int32_t fail(int32_t code, const std::string& what) {
     err = what;
@@ -91,14 +92,16 @@ namespace {
     }                                                               \
   } while (0)
 
-__global__ void scale_rows(const float* x, const uint32_t* idx, int rows, int cols, int ld, const float* mu,
-                           const float* sig, __nv_bfloat16* out, float* outf) {
+// (x - mu) / sig of `rows` rows, those of idx when given (the *step'th batch
+// of them), as BF16 with zero padding (out) or FP32 (outf).
+__global__ void scale_rows(const float* x, const uint32_t* idx, const uint32_t* step, int rows, int cols, int ld,
+                           const float* mu, const float* sig, __nv_bfloat16* out, float* outf) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * ld) return;
   const int r = i / ld, c = i % ld;
   float v = 0.0f;
   if (c < cols) {
-    const size_t src = idx ? idx[r] : uint32_t(r);
+    const size_t src = idx ? idx[size_t(*step) * rows + r] : uint32_t(r);
     v = (x[src * cols + c] - mu[c]) / sig[c];
   }
   if (out) out[i] = __float2bfloat16_rn(v);
@@ -137,7 +140,6 @@ int32_t ensure_batch(esl_mlp* m, int rows) {
   MLP_CUDA(m->dzb.ensure(size_t(rows) * wmax));
   MLP_CUDA(m->dzt.ensure(size_t(rows) * wmax));
   MLP_CUDA(m->t.ensure(size_t(rows) * m->n_out));
-  MLP_CUDA(m->idx.ensure(size_t(rows)));
   m->rows = rows;
   return ESL_MLP_OK;
 }
@@ -163,10 +165,10 @@ int32_t backward(esl_mlp* m, int rows) {
   const int L = int(m->layers.size());
   for (int l = L - 1; l >= 0; --l) {
     Layer& ly = *m->layers[l];
-    if (l != L - 1) MLP_CUDA(esl::launch_tanh_backward(m->dh.p, m->z[l]->p, rows, ly.n, ly.n, m->dz.p, m->dzb.p, m->stream));
-    else MLP_CUDA(esl::launch_to_bf16(m->dz.p, rows * ly.n, m->dzb.p, m->stream));
+    const bool last = l == L - 1;
+    MLP_CUDA(esl::launch_layer_grad(last ? m->dz.p : m->dh.p, last ? nullptr : m->z[l]->p, rows, ly.n, m->dz.p,
+                                    m->dzb.p, m->dzt.p, m->stream));
     // dW (n x k) = dZ^T (n x rows) . H (rows x k) = GEMM(dZ^T, H^T)
-    MLP_CUDA(esl::launch_transpose_bf16(m->dzb.p, rows, ly.n, ly.n, m->dzt.p, rows, m->stream));
     MLP_CUDA(esl::launch_transpose_bf16(m->hb[l]->p, rows, ly.k, ly.k, m->ht[l]->p, rows, m->stream));
     MLP_CUDA(esl::launch_gemm_bf16(m->dzt.p, rows, m->ht[l]->p, rows, ly.n, ly.k, rows, nullptr, ly.gw.p, ly.k,
                                    nullptr, 0, 0, m->gerr.p, m->stream));
@@ -282,6 +284,67 @@ int32_t esl_mlp_set_scaling(esl_mlp* m, const float* in_mu, const float* in_sig,
   return ESL_MLP_OK;
 }
 
+// A training run's second stream (the loss beside the gradients), the
+// events that order it, and the step's graph: for the run alone, since the
+// inputs' addresses are in it.
+struct TrainRun {
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  cudaError_t init() {
+    cudaError_t e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+    return e;
+  }
+  ~TrainRun() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    if (side) cudaStreamDestroy(side);
+  }
+};
+
+// One training step's launches on the network's stream: the batch at
+// perm[*at], forward, the gradients, Adam on every tensor, the next step.
+static int32_t train_step(esl_mlp* m, TrainRun& run, const float* d_x, const float* d_y, int B) {
+  cudaStream_t s = m->stream;
+  Layer& last = *m->layers.back();
+  const int kin = m->layers[0]->k;
+  scale_rows<<<(B * kin + 255) / 256, 256, 0, s>>>(d_x, m->perm.p, m->at.p, B, m->n_in, kin, m->d_in_mu.p,
+                                                    m->d_in_sig.p, m->hb[0]->p, nullptr);
+  // targets, standardized: t = (y - out_mu) / out_sig
+  scale_rows<<<(B * m->n_out + 255) / 256, 256, 0, s>>>(d_y, m->perm.p, m->at.p, B, m->n_out, m->n_out, m->d_out_mu.p,
+                                                         m->d_out_sig.p, nullptr, m->t.p);
+  MLP_CUDA(cudaGetLastError());
+  if (int32_t rc = forward(m, B)) return rc;
+  MLP_CUDA(cudaEventRecord(run.fork, s));
+  MLP_CUDA(cudaStreamWaitEvent(run.side, run.fork, 0));
+  MLP_CUDA(esl::launch_mse_loss(m->z.back()->p, m->t.p, B, m->n_out, last.n, m->loss.p, run.side));
+  MLP_CUDA(cudaEventRecord(run.join, run.side));
+  MLP_CUDA(esl::launch_mse_grad(m->z.back()->p, m->t.p, B, m->n_out, last.n, m->dz.p, s));
+  if (int32_t rc = backward(m, B)) return rc;
+  esl::AdamTensors T{};
+  for (auto& ly : m->layers) {
+    if (T.n + 2 > esl::kAdamMax) {
+      MLP_CUDA(esl::launch_adam(T, m->rates.p, m->at.p, s));
+      T.n = 0;
+    }
+    T.t[T.n++] = {ly->w.p, ly->gw.p, ly->mw.p, ly->vw.p, ly->wb.p, ly->wt.p, ly->n, ly->k, 0};
+    T.t[T.n++] = {ly->b.p, ly->gb.p, ly->mb.p, ly->vb.p, nullptr, nullptr, 1, ly->n, 0};
+  }
+  MLP_CUDA(esl::launch_adam(T, m->rates.p, m->at.p, s));
+  MLP_CUDA(cudaStreamWaitEvent(s, run.join, 0));
+  MLP_CUDA(esl::launch_next_step(m->at.p, s));
+  return ESL_MLP_OK;
+}
+
+// The first step is launched as it is; the others replay it as a graph: a
+// step is some two dozen short kernels, and launched one by one they cost
+// the host 18 us each, tensor maps included (512 hidden, batch 256: 460 us a
+// step, 100 as a graph).
 int32_t esl_mlp_train(esl_mlp* m, const float* d_x, const float* d_y, uint32_t n, uint32_t epochs, uint32_t batch,
                       float lr, float lr_end, uint64_t seed, float* loss_out) {
   if (!m || !d_x || !d_y || n == 0 || batch == 0 || batch % 16) return ESL_MLP_INVALID_ARGUMENT;
@@ -296,40 +359,53 @@ int32_t esl_mlp_train(esl_mlp* m, const float* d_x, const float* d_y, uint32_t n
   for (uint32_t i = 0; i < n; ++i) perm[i] = i;
   const uint32_t n_batches = n / batch;
   if (n_batches == 0) return m->fail(ESL_MLP_INVALID_ARGUMENT, "fewer samples than one batch");
-  Layer& last = *m->layers.back();
+  if (epochs == 0) return check_gemm_err(m);
+  MLP_CUDA(m->perm.ensure(n));
+  MLP_CUDA(m->at.ensure(1));
+  MLP_CUDA(m->rates.ensure(n_batches));
+  // beta^t of the steps so far
+  float p1 = 1.0f, p2 = 1.0f;
+  for (int i = 0; i < m->step; ++i) {
+    p1 *= esl::kAdamB1;
+    p2 *= esl::kAdamB2;
+  }
+  TrainRun run;
+  MLP_CUDA(run.init());
+  std::vector<esl::AdamRate> rates(n_batches);
   for (uint32_t ep = 0; ep < epochs; ++ep) {
     // geometric decay from lr to lr_end over the epochs
     const float lr_ep = (lr_end > 0 && epochs > 1)
                             ? lr * std::pow(lr_end / lr, float(ep) / float(epochs - 1))
                             : lr;
     std::shuffle(perm.begin(), perm.end(), rng);
+    for (esl::AdamRate& r : rates) {
+      p1 *= esl::kAdamB1;
+      p2 *= esl::kAdamB2;
+      r = {lr_ep, 1.0f - p1, 1.0f - p2};
+    }
+    m->step += int(n_batches);
+    MLP_CUDA(cudaMemcpyAsync(m->perm.p, perm.data(), size_t(n) * 4, cudaMemcpyHostToDevice, s));
+    MLP_CUDA(cudaMemcpyAsync(m->rates.p, rates.data(), rates.size() * sizeof(esl::AdamRate), cudaMemcpyHostToDevice, s));
+    MLP_CUDA(cudaMemsetAsync(m->at.p, 0, 4, s));
     MLP_CUDA(cudaMemsetAsync(m->loss.p, 0, 4, s));
     for (uint32_t bi = 0; bi < n_batches; ++bi) {
-      MLP_CUDA(cudaMemcpyAsync(m->idx.p, perm.data() + size_t(bi) * batch, batch * 4, cudaMemcpyHostToDevice, s));
-      const int kin = m->layers[0]->k;
-      scale_rows<<<(B * kin + 255) / 256, 256, 0, s>>>(d_x, m->idx.p, B, m->n_in, kin, m->d_in_mu.p, m->d_in_sig.p,
-                                                        m->hb[0]->p, nullptr);
-      // targets, standardized: t = (y - out_mu) / out_sig
-      scale_rows<<<(B * m->n_out + 255) / 256, 256, 0, s>>>(d_y, m->idx.p, B, m->n_out, m->n_out, m->d_out_mu.p,
-                                                             m->d_out_sig.p, nullptr, m->t.p);
-      MLP_CUDA(cudaGetLastError());
-      if (int32_t rc = forward(m, B)) return rc;
-      MLP_CUDA(esl::launch_mse_grad(m->z.back()->p, m->t.p, B, m->n_out, last.n, m->dz.p, m->loss.p, s));
-      if (int32_t rc = backward(m, B)) return rc;
-      ++m->step;
-      for (auto& ly : m->layers) {
-        MLP_CUDA(esl::launch_adam(ly->w.p, ly->gw.p, ly->mw.p, ly->vw.p, ly->n, ly->k, lr_ep, m->step, ly->wb.p,
-                                  ly->wt.p, ly->n, s));
-        MLP_CUDA(esl::launch_adam(ly->b.p, ly->gb.p, ly->mb.p, ly->vb.p, 1, ly->n, lr_ep, m->step, nullptr, nullptr,
-                                  0, s));
+      if (run.exec) {
+        MLP_CUDA(cudaGraphLaunch(run.exec, s));
+        continue;
       }
+      int32_t rc = train_step(m, run, d_x, d_y, B);
+      if (rc) return rc;
+      MLP_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+      rc = train_step(m, run, d_x, d_y, B);
+      const cudaError_t ended = cudaStreamEndCapture(s, &run.graph);
+      if (rc) return rc;
+      MLP_CUDA(ended);
+      MLP_CUDA(cudaGraphInstantiate(&run.exec, run.graph, 0));
     }
-    if (loss_out) {
-      float l = 0;
-      MLP_CUDA(cudaMemcpyAsync(&l, m->loss.p, 4, cudaMemcpyDeviceToHost, s));
-      MLP_CUDA(cudaStreamSynchronize(s));
-      loss_out[ep] = l / float(n_batches);
-    }
+    float l = 0;
+    MLP_CUDA(cudaMemcpyAsync(&l, m->loss.p, 4, cudaMemcpyDeviceToHost, s));
+    MLP_CUDA(cudaStreamSynchronize(s));
+    if (loss_out) loss_out[ep] = l / float(n_batches);
   }
   return check_gemm_err(m);
 }
@@ -345,7 +421,7 @@ int32_t esl_mlp_predict(esl_mlp* m, const float* d_x, uint32_t n, float* d_y) {
   const Layer& last = *m->layers.back();
   for (uint32_t r0 = 0; r0 < n; r0 += chunk) {
     const int rows = int(std::min(chunk, n - r0));
-    scale_rows<<<(rows * kin + 255) / 256, 256, 0, s>>>(d_x + size_t(r0) * m->n_in, nullptr, rows, m->n_in, kin,
+    scale_rows<<<(rows * kin + 255) / 256, 256, 0, s>>>(d_x + size_t(r0) * m->n_in, nullptr, nullptr, rows, m->n_in, kin,
                                                          m->d_in_mu.p, m->d_in_sig.p, m->hb[0]->p, nullptr);
     MLP_CUDA(cudaGetLastError());
     if (int32_t rc = forward(m, rows, false)) return rc;
@@ -367,13 +443,14 @@ int32_t esl_mlp_gradients(esl_mlp* m, const float* d_x, const float* d_y, uint32
   MLP_CUDA(cudaMemsetAsync(m->gerr.p, 0, 4, s));
   MLP_CUDA(cudaMemsetAsync(m->loss.p, 0, 4, s));
   const int kin = m->layers[0]->k;
-  scale_rows<<<(B * kin + 255) / 256, 256, 0, s>>>(d_x, nullptr, B, m->n_in, kin, m->d_in_mu.p, m->d_in_sig.p,
+  scale_rows<<<(B * kin + 255) / 256, 256, 0, s>>>(d_x, nullptr, nullptr, B, m->n_in, kin, m->d_in_mu.p, m->d_in_sig.p,
                                                     m->hb[0]->p, nullptr);
-  scale_rows<<<(B * m->n_out + 255) / 256, 256, 0, s>>>(d_y, nullptr, B, m->n_out, m->n_out, m->d_out_mu.p,
+  scale_rows<<<(B * m->n_out + 255) / 256, 256, 0, s>>>(d_y, nullptr, nullptr, B, m->n_out, m->n_out, m->d_out_mu.p,
                                                          m->d_out_sig.p, nullptr, m->t.p);
   MLP_CUDA(cudaGetLastError());
   if (int32_t rc = forward(m, B)) return rc;
-  MLP_CUDA(esl::launch_mse_grad(m->z.back()->p, m->t.p, B, m->n_out, m->layers.back()->n, m->dz.p, m->loss.p, s));
+  MLP_CUDA(esl::launch_mse_loss(m->z.back()->p, m->t.p, B, m->n_out, m->layers.back()->n, m->loss.p, s));
+  MLP_CUDA(esl::launch_mse_grad(m->z.back()->p, m->t.p, B, m->n_out, m->layers.back()->n, m->dz.p, s));
   if (int32_t rc = backward(m, B)) return rc;
   if (int32_t rc = check_gemm_err(m)) return rc;
   if (loss) MLP_CUDA(cudaMemcpy(loss, m->loss.p, 4, cudaMemcpyDeviceToHost));

@@ -246,19 +246,33 @@ __global__ void __launch_bounds__(kThreads) gemm_bf16_tc(const __grid_constant__
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
 }
 
-// dZ = dH * (1 - H^2) for a tanh layer (H stored as BF16); FP32 out and a
-// BF16 copy for the next GEMMs.
-__global__ void tanh_backward(const float* dh, const __nv_bfloat16* hb, int ldh, const float* zpre, int rows, int cols,
-                              int ld, float* dz, __nv_bfloat16* dzb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * cols) return;
-  const int r = i / cols, c = i % cols;
-  const float t = tanhf(zpre[size_t(r) * ld + c]);
-  const float g = dh[size_t(r) * ld + c] * (1.0f - t * t);
-  dz[size_t(r) * ld + c] = g;
-  dzb[size_t(r) * ld + c] = __float2bfloat16_rn(g);
-  (void)hb;
-  (void)ldh;
+// dZ = dH * (1 - tanh(Z)^2) for a tanh layer (zpre given; dz is dH's buffer
+// turned in place), dZ as it stands for the output layer; its BF16 copy and
+// that copy's transpose, through a 32 x 32 tile, in the same pass.
+__global__ void layer_grad(const float* dh, const float* zpre, int rows, int cols, float* dz, __nv_bfloat16* dzb,
+                           __nv_bfloat16* dzt) {
+  __shared__ __nv_bfloat16 tile[32][34];
+  const int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 32;
+  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
+    const int r = r0 + j;
+    if (r >= rows || c >= cols) continue;
+    const size_t at = size_t(r) * cols + c;
+    float g = dh[at];
+    if (zpre) {
+      const float t = tanhf(zpre[at]);
+      g = g * (1.0f - t * t);
+      dz[at] = g;
+    }
+    const __nv_bfloat16 gb = __float2bfloat16_rn(g);
+    dzb[at] = gb;
+    tile[j][threadIdx.x] = gb;
+  }
+  __syncthreads();
+  const int oc = r0 + threadIdx.x;
+  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
+    const int orow = blockIdx.x * 32 + j;
+    if (orow < cols && oc < rows) dzt[size_t(orow) * rows + oc] = tile[threadIdx.x][j];
+  }
 }
 
 // out (cols x rows, BF16) = in (rows x cols)^T, through a 32 x 32 tile.
@@ -278,53 +292,119 @@ __global__ void transpose_to_bf16(const T* in, int rows, int cols, int ldi, __nv
   }
 }
 
-// db[c] = sum over rows of dz[r][c] (one thread per column; rows is a batch).
+// db[c] = sum over rows of dz[r][c] in row order (one thread per column;
+// rows is a batch), sixteen rows' loads in flight: one at a time the column
+// was 256 round trips to L2.
 __global__ void bias_grad(const float* dz, int rows, int cols, int ld, float* db) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;
+  const float* p = dz + c;
   float s = 0.0f;
-  for (int r = 0; r < rows; ++r) s += dz[size_t(r) * ld + c];
+  int r = 0;
+  for (; r + 16 <= rows; r += 16) {
+    float x[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = p[size_t(r + j) * ld];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) s += x[j];
+  }
+  for (; r < rows; ++r) s += p[size_t(r) * ld];
   db[c] = s;
 }
 
 // MSE gradient over the real output columns: d = 2 (y - t) / (rows * outs).
-__global__ void mse_grad(const float* y, const float* t, int rows, int outs, int ld, float* d, float* loss) {
+__global__ void mse_grad(const float* y, const float* t, int rows, int outs, int ld, float* d) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows * ld) return;
   const int r = i / ld, c = i % ld;
-  float g = 0.0f;
-  if (c < outs) {
-    const float e = y[size_t(r) * ld + c] - t[size_t(r) * outs + c];
-    g = 2.0f * e / float(rows * outs);
-    atomicAdd(loss, e * e / float(rows * outs));
+  d[i] = c < outs ? 2.0f * (y[size_t(r) * ld + c] - t[size_t(r) * outs + c]) / float(rows * outs) : 0.0f;
+}
+
+// The loss the same batch adds to the FP32 accumulator, its terms one after
+// another: adding a term moves the accumulator by the term rounded to its
+// unit in the last place u, so the terms of a chunk are summed as integer
+// multiples of u, in parallel, and u is taken anew for the next chunk. (As
+// an atomic an element, 127,488 of them on one address, a batch's loss took
+// 270 us, three times the rest of its training step; summed in blocks it
+// would lose the accumulator's rounding, 1% of an epoch's loss.)
+constexpr int kLossThreads = 1024, kLossPer = 4;
+__global__ void __launch_bounds__(kLossThreads) mse_loss(const float* y, const float* t, int rows, int outs, int ld,
+                                                         float* loss) {
+  __shared__ long long part[kLossThreads / 32];
+  __shared__ float acc;
+  const int n = rows * outs, tid = threadIdx.x;
+  const float count = float(n);
+  if (tid == 0) acc = *loss;
+  __syncthreads();
+  for (int i0 = 0; i0 < n; i0 += kLossThreads * kLossPer) {
+    float x[kLossPer];
+    float top = 0.0f;
+#pragma unroll
+    for (int j = 0; j < kLossPer; ++j) {
+      const int i = i0 + j * kLossThreads + tid;
+      float e = 0.0f;
+      if (i < n) e = y[size_t(i / outs) * ld + i % outs] - t[i];
+      x[j] = e * e / count;
+      top = fmaxf(top, x[j]);
+    }
+    float a = acc;
+    if (a == 0.0f) {
+      // the first terms: from the largest one's scale
+      for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      if ((tid & 31) == 0) part[tid >> 5] = __float_as_int(top);
+      __syncthreads();
+      for (int w = 0; w < kLossThreads / 32; ++w) a = fmaxf(a, __int_as_float(int(part[w])));
+      __syncthreads();
+    }
+    // u = 2^(exponent - 23), at least 2^-126; a NaN or infinity passes through
+    const int ex = max(1, int((__float_as_uint(a) >> 23) & 255u) - 23);
+    const float u = __int_as_float(ex << 23);
+    long long k = 0;
+    bool wild = !(a < INFINITY);
+#pragma unroll
+    for (int j = 0; j < kLossPer; ++j) {
+      wild |= !(x[j] / u < 4.0e15f);
+      k += __float2ll_rn(x[j] / u);
+    }
+    for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+    if ((tid & 31) == 0) part[tid >> 5] = k;
+    const bool any_wild = __syncthreads_or(wild);
+    if (tid == 0) {
+      long long s = 0;
+      for (int w = 0; w < kLossThreads / 32; ++w) s += part[w];
+      acc = any_wild ? NAN : float(double(acc) + double(s) * double(u));
+    }
+    __syncthreads();
   }
-  d[size_t(r) * ld + c] = g;
+  if (tid == 0) *loss = acc;
 }
 
 // Adam on FP32 master weights; refreshes the BF16 copy (and its transpose
-// when given, for the backward GEMMs).
-__global__ void adam_step(float* w, const float* g, float* m, float* v, int rows, int cols, float lr, float b1,
-                          float b2, float eps, float c1, float c2, __nv_bfloat16* wb, __nv_bfloat16* wt, int ldt) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * cols) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-  w[i] = wi;
-  if (wb) wb[i] = __float2bfloat16_rn(wi);
-  if (wt) {
-    const int r = i / cols, c = i % cols;
-    wt[size_t(c) * ldt + r] = __float2bfloat16_rn(wi);
+// when given, for the backward GEMMs). One launch over every tensor of the
+// network (blocks first .. of each), the step's rate and bias corrections
+// from rates[*step].
+__global__ void adam_step(AdamTensors T, const AdamRate* rates, const uint32_t* step, float b1, float b2, float eps) {
+  int k = 0;
+  while (k + 1 < T.n && blockIdx.x >= T.t[k + 1].first) ++k;
+  const AdamTensor& a = T.t[k];
+  const int i = int(blockIdx.x - a.first) * int(blockDim.x) + int(threadIdx.x);
+  if (i >= a.rows * a.cols) return;
+  const AdamRate q = rates[*step];
+  const float gi = a.g[i];
+  const float mi = b1 * a.m[i] + (1.0f - b1) * gi;
+  const float vi = b2 * a.v[i] + (1.0f - b2) * gi * gi;
+  a.m[i] = mi;
+  a.v[i] = vi;
+  const float wi = a.w[i] - q.lr * (mi / q.c1) / (sqrtf(vi / q.c2) + eps);
+  a.w[i] = wi;
+  if (a.wb) a.wb[i] = __float2bfloat16_rn(wi);
+  if (a.wt) {
+    const int r = i / a.cols, c = i % a.cols;
+    a.wt[size_t(c) * a.rows + r] = __float2bfloat16_rn(wi);
   }
 }
 
-__global__ void to_bf16(const float* in, int n, __nv_bfloat16* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = __float2bfloat16_rn(in[i]);
-}
+__global__ void next_step(uint32_t* step) { ++*step; }
 
 }  // namespace
 
@@ -391,17 +471,10 @@ cudaError_t launch_gemm_bf16(const __nv_bfloat16* a, int lda, const __nv_bfloat1
   return cudaGetLastError();
 }
 
-cudaError_t launch_tanh_backward(const float* dh, const float* zpre, int rows, int cols, int ld, float* dz,
-                                 __nv_bfloat16* dzb, cudaStream_t s) {
-  const int n = rows * cols;
-  tanh_backward<<<(n + 255) / 256, 256, 0, s>>>(dh, nullptr, 0, zpre, rows, cols, ld, dz, dzb);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_transpose_f32(const float* in, int rows, int cols, int ldi, __nv_bfloat16* out, int ldo,
-                                 cudaStream_t s) {
+cudaError_t launch_layer_grad(const float* dh, const float* zpre, int rows, int cols, float* dz, __nv_bfloat16* dzb,
+                              __nv_bfloat16* dzt, cudaStream_t s) {
   dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
-  transpose_to_bf16<float><<<grid, block, 0, s>>>(in, rows, cols, ldi, out, ldo);
+  layer_grad<<<grid, block, 0, s>>>(dh, zpre, rows, cols, dz, dzb, dzt);
   return cudaGetLastError();
 }
 
@@ -417,29 +490,29 @@ cudaError_t launch_bias_grad(const float* dz, int rows, int cols, int ld, float*
   return cudaGetLastError();
 }
 
-cudaError_t launch_mse_grad(const float* y, const float* t, int rows, int outs, int ld, float* d, float* loss,
-                            cudaStream_t s) {
+cudaError_t launch_mse_grad(const float* y, const float* t, int rows, int outs, int ld, float* d, cudaStream_t s) {
   const int n = rows * ld;
-  mse_grad<<<(n + 255) / 256, 256, 0, s>>>(y, t, rows, outs, ld, d, loss);
+  mse_grad<<<(n + 255) / 256, 256, 0, s>>>(y, t, rows, outs, ld, d);
   return cudaGetLastError();
 }
 
-cudaError_t launch_adam(float* w, const float* g, float* m, float* v, int rows, int cols, float lr, int step,
-                        __nv_bfloat16* wb, __nv_bfloat16* wt, int ldt, cudaStream_t s) {
-  const float b1 = 0.9f, b2 = 0.999f;
-  float c1 = 1.0f, c2 = 1.0f;
-  for (int i = 0; i < step; ++i) {
-    c1 *= b1;
-    c2 *= b2;
+cudaError_t launch_mse_loss(const float* y, const float* t, int rows, int outs, int ld, float* loss, cudaStream_t s) {
+  mse_loss<<<1, kLossThreads, 0, s>>>(y, t, rows, outs, ld, loss);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_adam(AdamTensors T, const AdamRate* rates, uint32_t* step, cudaStream_t s) {
+  uint32_t blocks = 0;
+  for (int k = 0; k < T.n; ++k) {
+    T.t[k].first = blocks;
+    blocks += uint32_t((T.t[k].rows * T.t[k].cols + 255) / 256);
   }
-  const int n = rows * cols;
-  adam_step<<<(n + 255) / 256, 256, 0, s>>>(w, g, m, v, rows, cols, lr, b1, b2, 1e-8f, 1.0f - c1, 1.0f - c2, wb, wt,
-                                            ldt);
+  adam_step<<<blocks, 256, 0, s>>>(T, rates, step, kAdamB1, kAdamB2, 1e-8f);
   return cudaGetLastError();
 }
 
-cudaError_t launch_to_bf16(const float* in, int n, __nv_bfloat16* out, cudaStream_t s) {
-  to_bf16<<<(n + 255) / 256, 256, 0, s>>>(in, n, out);
+cudaError_t launch_next_step(uint32_t* step, cudaStream_t s) {
+  next_step<<<1, 1, 0, s>>>(step);
   return cudaGetLastError();
 }
 
