@@ -53,7 +53,7 @@ def stale():
 def _flags(verbose):
     return [NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3",
             "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off",
-            "--split-compile=8", "-Xptxas", "-v" if verbose else "-O3"]
+            "-Xptxas", "-v" if verbose else "-O3"]
 
 
 def build(force=False, verbose=False):

@@ -741,7 +741,7 @@ int32_t upload_tape(esl_ctx* ctx) {
   ctx->warp_ok = false;
   if (P.nv >= 65536) return ESL_OK;
   {
-    // One blob: A ops, B ops, gather depth/off/src/dst, each section
+    // One blob: the tasks of A and B, gather depth/off/src/dst, each section
     // 16-byte aligned.
     GatherSegments G = build_gather_segments(ctx, P);
     std::vector<unsigned char> blob;
@@ -751,8 +751,14 @@ int32_t upload_tape(esl_ctx* ctx) {
       blob.resize((blob.size() + 15) & ~size_t(15), 0);
       return at;
     };
-    T.o_a_ops = put(P.a_ops.data(), P.a_ops.size() * sizeof(Op));
-    T.o_b_ops = put(P.b_ops.data(), P.b_ops.size() * sizeof(Op));
+    // a stream's first chunk beyond its last is read ahead
+    TaskStream A, B;
+    compile_warp(P, A, B);
+    const uint32_t chunk = 32 * task_words(true) * 4;
+    T.a_chunks = A.off[1] - kTaskRing;
+    T.b_chunks = B.off[1] - kTaskRing;
+    T.o_a_tasks = put(A.words.data(), (T.a_chunks + 1) * chunk);
+    T.o_b_tasks = put(B.words.data(), (T.b_chunks + 1) * chunk);
     T.o_g_src = put(G.src.data(), G.src.size() * 4);
     T.o_g_dst = put(G.dst.data(), G.dst.size() * 4);
     uint32_t n_kr = 0;
@@ -766,8 +772,6 @@ int32_t upload_tape(esl_ctx* ctx) {
     ESL_CUDA(upload(ctx->d_prog, blob, s));
     T.prog = ctx->d_prog.as<unsigned char>();
     T.prog_bytes = uint32_t(blob.size());
-    T.a_rows = P.a_rows;
-    T.b_rows = P.b_rows;
     T.g_nseg = G.nseg;
     T.g_seg_blocks = G.seg_len / kGatherBlock;
   }

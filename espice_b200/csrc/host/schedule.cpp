@@ -352,11 +352,7 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv, uint32_t warps
       for (uint32_t l = 0; l < 32; ++l) {
         Words& x = lanes[l];
         x = Words{sink, common, {{zero, one}, {zero, one}, {zero, one}}};
-        if (l >= nt) {
-          x.pair[kTaskOps - 1][0] = any_div ? one : zero;  // what the lane divides by, unused
-          x.pair[kTaskOps - 1][1] = any_div ? zero : one;
-          continue;
-        }
+        if (l >= nt) continue;
         const Task& t = row[t0 + l];
         x.dst = t.v;
         for (uint32_t j = 0; j < t.ops; ++j) {
@@ -442,6 +438,11 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv, uint32_t warps
 }
 
 }  // namespace
+
+void compile_warp(const Programs& P, TaskStream& a, TaskStream& b) {
+  a = pack_tasks(unpack(P.a_seq), P.nv, 1, true);
+  b = pack_tasks(unpack(P.b_seq), P.nv, 1, true);
+}
 
 BlockPrograms compile_block(const Programs& P, uint32_t warps) {
   BlockPrograms B;

@@ -71,6 +71,10 @@ struct BlockPrograms {
 // sparse triangular solves.
 Programs compile_tape(const SparseLu& lu);
 
+// The warp lanes' programs A and B as one warp's compact task stream each
+// (value spaces below 65,536).
+void compile_warp(const Programs& P, TaskStream& a, TaskStream& b);
+
 // The block lanes' task streams for a CTA of `warps` warps (at most kTaskWarps).
 BlockPrograms compile_block(const Programs& P, uint32_t warps);
 

@@ -43,9 +43,8 @@ struct TopoDev {
   uint32_t n_fill;
   // The warp programs live in one 16-byte-aligned blob, staged into each
   // CTA's shared memory: A = refactor + forward solve and B = back solve,
-  // rows of 32 ops over v = [tape values | y | 0.0 | 1.0 | sink], each row
-  // divisions only or multiply-subtracts only (every op word carries its
-  // kind); the assembly as one segmented gather: g_nseg segments of
+  // chunks of 32 compact tasks (common.h) over v = [tape values | y | 0.0 |
+  // 1.0 | sink], each followed by one that is only read ahead; the assembly as one segmented gather: g_nseg segments of
   // kGatherBlock g_seg_blocks terms, thread t summing term k of its column at
   // src[k * 32 + t] (lane-block indices) and, at a segment's end where its
   // destination triple (dst[(3 s + i) * 32 + t]) carries kGatherEnd,
@@ -60,8 +59,8 @@ struct TopoDev {
   // Offsets in bytes.
   const unsigned char* prog;
   uint32_t prog_bytes;
-  uint32_t o_a_ops, o_b_ops, o_g_src, o_g_dst;
-  uint32_t a_rows, b_rows, g_nseg, g_seg_blocks;
+  uint32_t o_a_tasks, o_b_tasks, o_g_src, o_g_dst;
+  uint32_t a_chunks, b_chunks, g_nseg, g_seg_blocks;
   uint32_t o_k_depth, o_k_off, o_k_src, o_k_dst;
   uint32_t n_kr_groups, n_ks_groups;
   // L tape values whose column passed on the row-scaled test (no wide test).

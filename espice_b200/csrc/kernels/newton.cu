@@ -35,6 +35,7 @@
 #include "bsim3.cuh"
 #include "lane_eval.cuh"
 #include "ladder.cuh"
+#include "tasks.cuh"
 #include "tran_core.cuh"
 
 namespace esl {
@@ -199,64 +200,24 @@ __device__ void assemble(const TopoDev& T, uint32_t prog, const LaneMem& m, int 
 }
 
 
-// Runs one warp program over v (shared address vb): rows of 32 ops, each
-// row divisions only or multiply-subtracts only (warp-uniform branches),
-// thread t taking op t, the next row's op fetched while this one runs.
-// Padding ops move 1.0 / 0.0 into the sink. Returns true when a division
-// failed its pivot test (thread-local). Compiled out of line: the loop's
-// own register allocation measured about 1% faster on the transient than
-// inlined into the fused kernels.
-__device__ __noinline__ bool run_rows(uint32_t ops, uint32_t rows, uint32_t vb, int tid) {
-  bool bad = false;
-  if (rows == 0) return false;
-  uint2 op = lds_u2(ops + 8 * tid);
-  for (uint32_t r = 0; r < rows; ++r) {
-    const uint32_t rn = r + 1 < rows ? r + 1 : r;
-    const uint2 next = lds_u2(ops + 8 * (rn * 32 + tid));
-    const uint32_t kind = op.x >> 28;
-    const uint32_t pd = vb + 8 * (op.x & 0x0fffffffu);
-    const uint32_t pa = vb + 8 * (op.y & 0xffffu), pb = vb + 8 * (op.y >> 16);
-    // Two warp-uniform paths (a switch here compiles to an indirect jump
-    // that costs more than the op): the divisions with their checks
-    // predicated on the kind, and the multiply-subtracts (the solves skip a
-    // zero multiplier, the refactor never does).
-    const double a = lds(pa), b = lds(pb);
-    if (kind == kOpDivGrowth || kind == kOpDivScaled || kind == kOpDivY) {
-      // dividend at b (the op's own value; 1.0 on padding)
-      const double q = div_rn(b, a);
-      if (kind == kOpDivGrowth && !(fabs(a) >= __dmul_rn(kGrowth, fabs(b)))) bad = true;
-      if (kind == kOpDivScaled && !(fabs(q) < CUDART_INF)) bad = true;
-      sts(pd, q);
-    } else {
-      const double d = lds(pd);
-      if (kind == kOpFlop || b != 0.0) sts(pd, __dsub_rn(d, __dmul_rn(a, b)));
-    }
-    __syncwarp();
-    op = next;
-  }
-  return bad;
-}
-
 // Refactor on the frozen tape with the forward solve merged in (program A),
-// then the lane kernel's peel tests (lane_kernels.zig Bodies.refactor and
+// and the lane kernel's peel tests (lane_kernels.zig Bodies.refactor and
 // LaneSolver.wideMultipliers): U entries finite, pivots alive, L multipliers
-// within 1 / pivot_tol. y must hold P(-rhs). Warp-uniform verdict.
+// within 1 / pivot_tol (tested where they are divided). y must hold P(-rhs).
+// Warp-uniform verdict. (As rows of one op a thread the ring's program A was
+// 79 rows and 19.0k cycles, B 51 and 11.8k.)
 __device__ bool refactor_forward(const TopoDev& T, uint32_t prog, double* v, int tid) {
-  bool bad = run_rows(prog + T.o_a_ops, T.a_rows, saddr(v), tid);
-  const uint32_t l0 = T.nu + T.n;
-  for (uint32_t s = tid; s < T.nu; s += 32)
-    if (dbits(v[s] - v[s]) != 0) bad = true;
+  bool bad = run_warp_tasks(prog + T.o_a_tasks, T.a_chunks, v) != 0;
+  for (uint32_t s = tid; s < T.nu; s += 32) bad |= !task_finite(v[s]);
   for (uint32_t k = tid; k < T.n; k += 32) {
     const double d = v[T.nu + k];
-    if (d == 0.0 || !(fabs(d) < CUDART_INF)) bad = true;
+    bad |= d == 0.0 || !task_finite(d);
   }
-  for (uint32_t s = tid; s < T.nl; s += 32)
-    if (!T.l_scaled[s] && !(fabs(v[l0 + s]) <= kWide)) bad = true;
   return __any_sync(kFull, bad);
 }
 
-__device__ __forceinline__ void back_solve(const TopoDev& T, uint32_t prog, double* v, int tid) {
-  run_rows(prog + T.o_b_ops, T.b_rows, saddr(v), tid);
+__device__ __forceinline__ void back_solve(const TopoDev& T, uint32_t prog, double* v) {
+  run_warp_tasks(prog + T.o_b_tasks, T.b_chunks, v);
 }
 
 __device__ __forceinline__ void load_y(const TopoDev& T, const double* rhs, double* y, int tid) {
@@ -390,7 +351,7 @@ __device__ void dc_solve_lane(const TopoDev& T, const LaneDev& L, const LaneOpts
         }
         return;
       }
-      back_solve(T, prog, m.v, tid);
+      back_solve(T, prog, m.v);
     }
     have_step = false;
     __syncwarp();
@@ -509,7 +470,7 @@ __global__ void __launch_bounds__(256) lu_replay_kernel(TopoDev T, uint32_t n_la
     load_y(T, r, y, tid);
     __syncwarp();
     const bool bad = refactor_forward(T, prog, v, tid);
-    back_solve(T, prog, v, tid);
+    back_solve(T, prog, v);
     for (uint32_t j = tid; j < T.n; j += 32) dx[size_t(lane) * T.n + T.qcol[j]] = y[j];
     if (tv_out)
       for (uint32_t s = tid; s < T.ntv; s += 32) tv_out[size_t(lane) * T.ntv + s] = v[s];
@@ -1127,7 +1088,7 @@ __device__ int lane_newton(const TopoDev& T, uint32_t prog, const LaneMem& m, co
       iters = iter + 1;
       return 2;
     }
-    back_solve(T, prog, m.v, tid);
+    back_solve(T, prog, m.v);
    }
     have_step = false;
     __syncwarp();

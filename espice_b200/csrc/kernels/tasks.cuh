@@ -1,7 +1,7 @@
-// The block lanes' task programs (host/schedule.cpp pack_tasks) over a
-// lane's value space: every lane of a warp takes one task a chunk, up to
-// kTaskOps updates of one value and its division, and the CTA steps from
-// row to row by barriers.
+// The task programs (host/schedule.cpp pack_tasks) over a lane's value
+// space: every lane of a warp takes one task a chunk, up to kTaskOps updates
+// of one value and its division; a block lane's CTA steps from row to row by
+// barriers, a warp lane is one warp and its rows follow each other.
 //
 // What bounds it is the chain of rows, not the arithmetic: a row costs a
 // warp's in-order pass through one chunk and the barrier. So a row does as
@@ -150,12 +150,16 @@ struct TaskLane<false> {
   __device__ __forceinline__ uint32_t b(int j) const { return j == 0 ? c.w : j == 1 ? e.y : e.w; }
 };
 
-template <typename V, bool kShared, bool kCompact>
+// kCta: the program of a CTA's warps (idle chunks, CTA barriers), else of
+// one warp.
+template <typename V, bool kShared, bool kCompact, bool kCta>
 __device__ __forceinline__ void run_task(const TaskLane<kCompact>& c, const TaskMem<V, kShared>& v, uint32_t& bad) {
   const uint32_t f = c.flags();
-  if (f & kTaskIdle) {
-    for (uint32_t k = c.idle(); k; --k) __syncthreads();
-    return;
+  if constexpr (kCta) {
+    if (f & kTaskIdle) {
+      for (uint32_t k = c.idle(); k; --k) __syncthreads();
+      return;
+    }
   }
   const uint32_t dst = c.dst();
   const bool all = !(f & kTaskNz), div = f & kTaskDiv;
@@ -176,13 +180,17 @@ __device__ __forceinline__ void run_task(const TaskLane<kCompact>& c, const Task
     d = r0 ? t : d;
   }
   if (f & kTaskDivAny) {
-    const V q = task_div(d, a2);
-    const bool shrunk = !(fabs(a2) >= task_growth(a2) * fabs(d) && fabs(q) <= V(1e3)), wild = !task_finite(q);
+    // a lane that does not divide takes 1.0: its other operand may be zero,
+    // and one such lane sends the warp down the division's slow path (the
+    // ring's two programs: 31k cycles, against 25k)
+    const V piv = div ? a2 : V(1);
+    const V q = task_div(d, piv);
+    const bool shrunk = !(fabs(piv) >= task_growth(piv) * fabs(d) && fabs(q) <= V(1e3)), wild = !task_finite(q);
     bad |= (uint32_t(shrunk) & (f / kTaskGrowth)) | (uint32_t(wild) & (f / kTaskScaled));
     d = div ? q : d;
   }
   v.st(dst, d);
-  if (f & kTaskCta) __syncthreads();
+  if (kCta && (f & kTaskCta)) __syncthreads();
   else __syncwarp();
 }
 
@@ -218,10 +226,26 @@ __device__ __noinline__ uint32_t run_tasks(const uint32_t* words, uint32_t first
     fill = (fill + kBytes) & (kSpan - 1);
     task_wait<kTaskRing - 2>();
     next.load(base + read);
-    run_task<V, kShared, kCompact>(c, v, bad);
+    run_task<V, kShared, kCompact, true>(c, v, bad);
     c = next;
   }
   task_wait<0>();
+  return bad & 1u;
+}
+
+// Runs one warp's program of `chunks` whose words lie in shared memory
+// (`words`, a shared address), the next chunk's read while this one runs.
+__device__ __noinline__ uint32_t run_warp_tasks(uint32_t words, uint32_t chunks, double* values) {
+  uint32_t at = words + 16 * (threadIdx.x & 31), bad = 0;
+  const TaskMem<double, true> v(values);
+  TaskLane<true> c, next;
+  c.load(at);
+  for (uint32_t k = 0; k < chunks; ++k) {
+    at += TaskLane<true>::kBytes;
+    next.load(at);
+    run_task<double, true, true, false>(c, v, bad);
+    c = next;
+  }
   return bad & 1u;
 }
 
