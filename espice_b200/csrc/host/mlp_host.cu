@@ -16,6 +16,7 @@
 #include <memory>
 #include <random>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../../include/espice_mlp.h"
@@ -48,8 +49,10 @@ struct Dev {
 
 struct Layer {
   int k = 0, n = 0;  // padded input and output widths
-  Dev<float> w, b, gw, gb, mw, vw, mb, vb;
-  Dev<__nv_bfloat16> wb, wt;  // BF16 W (n x k) and W^T (k x n)
+  // in the network's arena
+  float *w = nullptr, *b = nullptr, *gw = nullptr, *gb = nullptr;
+  float *mw = nullptr, *vw = nullptr, *mb = nullptr, *vb = nullptr;
+  __nv_bfloat16 *wb = nullptr, *wt = nullptr;  // BF16 W (n x k) and W^T (k x n)
 };
 
 }  // namespace
@@ -60,6 +63,7 @@ struct esl_mlp {
   std::string err;
   int n_in = 0, n_out = 0, k_in = 0, k_out = 0;
   std::vector<std::unique_ptr<Layer>> layers;
+  Dev<unsigned char> arena;
   int step = 0;
   // standardization: x' = (x - in_mu) / in_sig, y = y' * out_sig + out_mu
   std::vector<float> in_mu, in_sig, out_mu, out_sig;
@@ -154,7 +158,7 @@ int32_t forward(esl_mlp* m, int rows, bool keep_z = true) {
     const bool last = l + 1 == L;
     __nv_bfloat16* next = last ? nullptr : m->hb[l + 1]->p;
     float* z = (keep_z || last) ? m->z[l]->p : nullptr;
-    MLP_CUDA(esl::launch_gemm_bf16(m->hb[l]->p, ly.k, ly.wb.p, ly.k, rows, ly.n, ly.k, ly.b.p, z, ly.n, next,
+    MLP_CUDA(esl::launch_gemm_bf16(m->hb[l]->p, ly.k, ly.wb, ly.k, rows, ly.n, ly.k, ly.b, z, ly.n, next,
                                    ly.n, last ? 0 : 1, m->gerr.p, m->stream));
   }
   return ESL_MLP_OK;
@@ -170,12 +174,12 @@ int32_t backward(esl_mlp* m, int rows) {
                                     m->dzb.p, m->dzt.p, m->stream));
     // dW (n x k) = dZ^T (n x rows) . H (rows x k) = GEMM(dZ^T, H^T)
     MLP_CUDA(esl::launch_transpose_bf16(m->hb[l]->p, rows, ly.k, ly.k, m->ht[l]->p, rows, m->stream));
-    MLP_CUDA(esl::launch_gemm_bf16(m->dzt.p, rows, m->ht[l]->p, rows, ly.n, ly.k, rows, nullptr, ly.gw.p, ly.k,
+    MLP_CUDA(esl::launch_gemm_bf16(m->dzt.p, rows, m->ht[l]->p, rows, ly.n, ly.k, rows, nullptr, ly.gw, ly.k,
                                    nullptr, 0, 0, m->gerr.p, m->stream));
-    MLP_CUDA(esl::launch_bias_grad(m->dz.p, rows, ly.n, ly.n, ly.gb.p, m->stream));
+    MLP_CUDA(esl::launch_bias_grad(m->dz.p, rows, ly.n, ly.n, ly.gb, m->stream));
     if (l > 0) {
       // dH_{l-1} (rows x k) = dZ (rows x n) . W (n x k) = GEMM(dZ, W^T)
-      MLP_CUDA(esl::launch_gemm_bf16(m->dzb.p, ly.n, ly.wt.p, ly.n, rows, ly.k, ly.n, nullptr, m->dh.p, ly.k, nullptr,
+      MLP_CUDA(esl::launch_gemm_bf16(m->dzb.p, ly.n, ly.wt, ly.n, rows, ly.k, ly.n, nullptr, m->dh.p, ly.k, nullptr,
                                      0, 0, m->gerr.p, m->stream));
     }
   }
@@ -211,6 +215,7 @@ int32_t esl_mlp_create(int n_in, int n_hidden, int n_layers, int n_out, int devi
   widths.push_back(m->k_in);
   for (int l = 0; l + 1 < n_layers; ++l) widths.push_back(pad16(n_hidden));
   widths.push_back(m->k_out);
+  std::vector<std::vector<float>> weights;
   for (size_t l = 0; l + 1 < widths.size(); ++l) {
     auto ly = std::make_unique<Layer>();
     ly->k = widths[l];
@@ -223,23 +228,41 @@ int32_t esl_mlp_create(int n_in, int n_hidden, int n_layers, int n_out, int devi
     std::vector<float> w(size_t(ly->n) * ly->k, 0.0f);
     for (int r = 0; r < real_n; ++r)
       for (int c = 0; c < real_k; ++c) w[size_t(r) * ly->k + c] = u(rng);
-    const size_t nw = w.size();
-    for (Dev<float>* d : {&ly->w, &ly->gw, &ly->mw, &ly->vw})
-      if (d->ensure(nw) != cudaSuccess) return ESL_MLP_OUT_OF_MEMORY;
-    for (Dev<float>* d : {&ly->b, &ly->gb, &ly->mb, &ly->vb})
-      if (d->ensure(size_t(ly->n)) != cudaSuccess) return ESL_MLP_OUT_OF_MEMORY;
-    if (ly->wb.ensure(nw) != cudaSuccess || ly->wt.ensure(nw) != cudaSuccess) return ESL_MLP_OUT_OF_MEMORY;
-    cudaMemcpy(ly->w.p, w.data(), nw * 4, cudaMemcpyHostToDevice);
-    std::vector<__nv_bfloat16> wb(nw), wt(nw);
-    for (int r = 0; r < ly->n; ++r)
-      for (int c = 0; c < ly->k; ++c) {
-        wb[size_t(r) * ly->k + c] = __float2bfloat16_rn(w[size_t(r) * ly->k + c]);
-        wt[size_t(c) * ly->n + r] = wb[size_t(r) * ly->k + c];
-      }
-    cudaMemcpy(ly->wb.p, wb.data(), nw * 2, cudaMemcpyHostToDevice);
-    cudaMemcpy(ly->wt.p, wt.data(), nw * 2, cudaMemcpyHostToDevice);
+    weights.push_back(std::move(w));
     m->layers.push_back(std::move(ly));
   }
+  // every layer's tensors in one zeroed allocation (14 a layer, with their
+  // fills and frees, took most of a network's life outside its training),
+  // the BF16 copies made on the device
+  size_t bytes = 0;
+  auto place = [&](bool assign) {
+    bytes = 0;
+    auto take = [&](auto*& p, size_t count) {
+      using T = std::remove_reference_t<decltype(*p)>;
+      if (assign) p = reinterpret_cast<T*>(m->arena.p + bytes);
+      bytes += (count * sizeof(T) + 255) & ~size_t(255);
+    };
+    for (auto& ly : m->layers) {
+      const size_t nw = size_t(ly->n) * ly->k;
+      for (float** p : {&ly->w, &ly->gw, &ly->mw, &ly->vw}) take(*p, nw);
+      for (float** p : {&ly->b, &ly->gb, &ly->mb, &ly->vb}) take(*p, size_t(ly->n));
+      take(ly->wb, nw);
+      take(ly->wt, nw);
+    }
+  };
+  place(false);
+  if (m->arena.ensure(bytes) != cudaSuccess) return ESL_MLP_OUT_OF_MEMORY;
+  // the fill runs on the default stream, which the network's does not wait for
+  if (cudaStreamSynchronize(nullptr) != cudaSuccess) return ESL_MLP_DEVICE_FAULT;
+  place(true);
+  for (size_t l = 0; l < m->layers.size(); ++l) {
+    Layer& ly = *m->layers[l];
+    if (cudaMemcpyAsync(ly.w, weights[l].data(), weights[l].size() * 4, cudaMemcpyHostToDevice, m->stream) !=
+            cudaSuccess ||
+        esl::launch_weight_copies(ly.w, ly.n, ly.k, ly.wb, ly.wt, m->stream) != cudaSuccess)
+      return ESL_MLP_DEVICE_FAULT;
+  }
+  if (cudaStreamSynchronize(m->stream) != cudaSuccess) return ESL_MLP_DEVICE_FAULT;
   m->in_mu.assign(n_in, 0.0f);
   m->in_sig.assign(n_in, 1.0f);
   m->out_mu.assign(n_out, 0.0f);
@@ -332,8 +355,8 @@ static int32_t train_step(esl_mlp* m, TrainRun& run, const float* d_x, const flo
       MLP_CUDA(esl::launch_adam(T, m->rates.p, m->at.p, s));
       T.n = 0;
     }
-    T.t[T.n++] = {ly->w.p, ly->gw.p, ly->mw.p, ly->vw.p, ly->wb.p, ly->wt.p, ly->n, ly->k, 0};
-    T.t[T.n++] = {ly->b.p, ly->gb.p, ly->mb.p, ly->vb.p, nullptr, nullptr, 1, ly->n, 0};
+    T.t[T.n++] = {ly->w, ly->gw, ly->mw, ly->vw, ly->wb, ly->wt, ly->n, ly->k, 0};
+    T.t[T.n++] = {ly->b, ly->gb, ly->mb, ly->vb, nullptr, nullptr, 1, ly->n, 0};
   }
   MLP_CUDA(esl::launch_adam(T, m->rates.p, m->at.p, s));
   MLP_CUDA(cudaStreamWaitEvent(s, run.join, 0));
@@ -457,9 +480,9 @@ int32_t esl_mlp_gradients(esl_mlp* m, const float* d_x, const float* d_y, uint32
   if (grads) {
     size_t at = 0;
     for (auto& ly : m->layers) {
-      MLP_CUDA(cudaMemcpy(grads + at, ly->gw.p, size_t(ly->n) * ly->k * 4, cudaMemcpyDeviceToHost));
+      MLP_CUDA(cudaMemcpy(grads + at, ly->gw, size_t(ly->n) * ly->k * 4, cudaMemcpyDeviceToHost));
       at += size_t(ly->n) * ly->k;
-      MLP_CUDA(cudaMemcpy(grads + at, ly->gb.p, size_t(ly->n) * 4, cudaMemcpyDeviceToHost));
+      MLP_CUDA(cudaMemcpy(grads + at, ly->gb, size_t(ly->n) * 4, cudaMemcpyDeviceToHost));
       at += size_t(ly->n);
     }
   }
@@ -482,9 +505,9 @@ int32_t esl_mlp_weights(esl_mlp* m, float* out) {
   MLP_CUDA(cudaStreamSynchronize(m->stream));
   size_t at = 0;
   for (auto& ly : m->layers) {
-    MLP_CUDA(cudaMemcpy(out + at, ly->w.p, size_t(ly->n) * ly->k * 4, cudaMemcpyDeviceToHost));
+    MLP_CUDA(cudaMemcpy(out + at, ly->w, size_t(ly->n) * ly->k * 4, cudaMemcpyDeviceToHost));
     at += size_t(ly->n) * ly->k;
-    MLP_CUDA(cudaMemcpy(out + at, ly->b.p, size_t(ly->n) * 4, cudaMemcpyDeviceToHost));
+    MLP_CUDA(cudaMemcpy(out + at, ly->b, size_t(ly->n) * 4, cudaMemcpyDeviceToHost));
     at += size_t(ly->n);
   }
   return ESL_MLP_OK;

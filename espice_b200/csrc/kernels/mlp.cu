@@ -327,7 +327,7 @@ __global__ void mse_grad(const float* y, const float* t, int rows, int outs, int
 // an atomic an element, 127,488 of them on one address, a batch's loss took
 // 270 us, three times the rest of its training step; summed in blocks it
 // would lose the accumulator's rounding, 1% of an epoch's loss.)
-constexpr int kLossThreads = 1024, kLossPer = 4;
+constexpr int kLossThreads = 1024;
 __global__ void __launch_bounds__(kLossThreads) mse_loss(const float* y, const float* t, int rows, int outs, int ld,
                                                          float* loss) {
   __shared__ long long part[kLossThreads / 32];
@@ -336,20 +336,15 @@ __global__ void __launch_bounds__(kLossThreads) mse_loss(const float* y, const f
   const float count = float(n);
   if (tid == 0) acc = *loss;
   __syncthreads();
-  for (int i0 = 0; i0 < n; i0 += kLossThreads * kLossPer) {
-    float x[kLossPer];
-    float top = 0.0f;
-#pragma unroll
-    for (int j = 0; j < kLossPer; ++j) {
-      const int i = i0 + j * kLossThreads + tid;
-      float e = 0.0f;
-      if (i < n) e = y[size_t(i / outs) * ld + i % outs] - t[i];
-      x[j] = e * e / count;
-      top = fmaxf(top, x[j]);
-    }
+  for (int i0 = 0; i0 < n; i0 += kLossThreads) {
+    const int i = i0 + tid;
+    float e = 0.0f;
+    if (i < n) e = y[size_t(i / outs) * ld + i % outs] - t[i];
+    const float x = e * e / count;
     float a = acc;
     if (a == 0.0f) {
       // the first terms: from the largest one's scale
+      float top = x;
       for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
       if ((tid & 31) == 0) part[tid >> 5] = __float_as_int(top);
       __syncthreads();
@@ -359,13 +354,8 @@ __global__ void __launch_bounds__(kLossThreads) mse_loss(const float* y, const f
     // u = 2^(exponent - 23), at least 2^-126; a NaN or infinity passes through
     const int ex = max(1, int((__float_as_uint(a) >> 23) & 255u) - 23);
     const float u = __int_as_float(ex << 23);
-    long long k = 0;
-    bool wild = !(a < INFINITY);
-#pragma unroll
-    for (int j = 0; j < kLossPer; ++j) {
-      wild |= !(x[j] / u < 4.0e15f);
-      k += __float2ll_rn(x[j] / u);
-    }
+    const bool wild = !(a < INFINITY) || !(x / u < 4.0e15f);
+    long long k = __float2ll_rn(x / u);
     for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
     if ((tid & 31) == 0) part[tid >> 5] = k;
     const bool any_wild = __syncthreads_or(wild);
@@ -508,6 +498,13 @@ cudaError_t launch_adam(AdamTensors T, const AdamRate* rates, uint32_t* step, cu
     blocks += uint32_t((T.t[k].rows * T.t[k].cols + 255) / 256);
   }
   adam_step<<<blocks, 256, 0, s>>>(T, rates, step, kAdamB1, kAdamB2, 1e-8f);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_weight_copies(const float* w, int rows, int cols, __nv_bfloat16* wb, __nv_bfloat16* wt,
+                                 cudaStream_t s) {
+  dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
+  layer_grad<<<grid, block, 0, s>>>(w, nullptr, rows, cols, nullptr, wb, wt);
   return cudaGetLastError();
 }
 

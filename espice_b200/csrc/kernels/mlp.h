@@ -45,6 +45,9 @@ struct AdamTensors {
   AdamTensor t[kAdamMax];
 };
 cudaError_t launch_adam(AdamTensors T, const AdamRate* rates, uint32_t* step, cudaStream_t s);
+// wb, wt: w (rows x cols) as BF16 and its transpose.
+cudaError_t launch_weight_copies(const float* w, int rows, int cols, __nv_bfloat16* wb, __nv_bfloat16* wt,
+                                 cudaStream_t s);
 cudaError_t launch_next_step(uint32_t* step, cudaStream_t s);
 
 }  // namespace esl
