@@ -66,6 +66,8 @@ struct Gen {
   std::vector<int64_t> pos;
   int64_t cur_stage = -1;
   uint32_t n_stages = 0;
+  // factors_out false: the entries no op writes, whose home is A (or zero)
+  std::vector<uint8_t> kept;
 
   explicit Gen(const LuJitInput& i) : in(i) {
     defined.assign(in.nv, 0);
@@ -95,7 +97,8 @@ struct Gen {
   // The home of value v, as an expression for this lane.
   std::string home(uint32_t v) const {
     std::ostringstream h;
-    if (v < in.ntv) h << "tl[" << v << " * N]";
+    if (v < in.ntv && kept[v]) h << "al[" << slot_of[v] << " * N]";
+    else if (v < in.ntv) h << "tl[" << v << " * N]";
     else h << "dx[" << (*in.qcol)[v - in.ntv] << " * N + lane]";
     return h.str();
   }
@@ -121,7 +124,10 @@ struct Gen {
     if (record) {
       uses[v].push_back(u);
     } else if (!constant(v)) {
-      if (defined[v] && !resident[v]) os << "  v" << v << " = __ldcg(&" << home(v) << ");\n";
+      if (defined[v] && !resident[v]) {
+        if (v < in.ntv && kept[v] && slot_of[v] < 0) os << "  v" << v << " = " << zero() << ";\n";
+        else os << "  v" << v << " = __ldcg(&" << home(v) << ");\n";
+      }
       touch(v);
     }
     if (!defined[v]) {
@@ -140,6 +146,10 @@ struct Gen {
            << ", " << pos[v] % kStage << ")" << (in.mixed ? ")" : "");
       else os << zero();  // fill-in (and an entry no slot or op sets)
       os << ";\n";
+      if (!in.factors_out && v < in.ntv && kept[v]) {
+        clean[v] = 1;
+        test(v);
+      }
     }
   }
 
@@ -221,14 +231,25 @@ struct Gen {
     wrote(d);
   }
 
-  // A tape value is final: out to its plane, then the refactor's peel test
-  // on it (a non-finite U entry, a dead or non-finite pivot, an unscaled L
-  // multiplier past 1 / pivot_tol).
+  // A tape value is final: out to its plane (when the factors are wanted),
+  // then the refactor's peel test on it.
   void finish(uint32_t v) {
     if (v >= in.ntv - 1) return;  // the discard entry holds nothing
+    const bool first = !defined[v];
     use(v);
-    os << "  " << home(v) << " = v" << v << ";\n";
-    clean[v] = 1;
+    if (in.factors_out) {
+      os << "  " << home(v) << " = v" << v << ";\n";
+      clean[v] = 1;
+    } else if (first && kept[v]) {
+      return;  // tested as it was loaded
+    }
+    test(v);
+  }
+
+  // The peel test on a final tape value (a non-finite U entry, a dead or
+  // non-finite pivot, an unscaled L multiplier past 1 / pivot_tol).
+  void test(uint32_t v) {
+    if (v >= in.ntv - 1) return;
     if (in.mixed) {  // the interpreted mixed kernel's FP32 tests
       if (v < in.nu) os << "  bad |= !(fabsf(v" << v << ") < kInf);\n";
       else if (v < in.nu + in.n) os << "  bad |= v" << v << " == 0.0f || !(fabsf(v" << v << ") < kInf);\n";
@@ -320,9 +341,17 @@ std::string lu_jit_source(const LuJitInput& in) {
   // The op stream: tape values (U, diagonal, L) are final after their last
   // update in program A (at once when program A never writes them); dx is
   // final after its last update (a y entry no op writes goes out as loaded).
+  // Without the factors an entry no op writes is tested as it is first read,
+  // and one no op reads either is read for its test alone.
+  std::vector<uint8_t> kept(in.nv, 0), read(in.nv, 0);
+  if (!in.factors_out) {
+    for (uint32_t v = 0; v < in.ntv; ++v) kept[v] = last_all[v] < 0;
+    for (uint32_t k = 0; k < in.n_seq; ++k)
+      if ((seq[k].w0 >> 28) != kOpNop) read[seq[k].w1 & 0xffffu] = read[seq[k].w1 >> 16] = 1;
+  }
   auto walk = [&](Gen& g) {
     for (uint32_t v = 0; v + 1 < in.ntv; ++v)
-      if (last_a[v] < 0) {
+      if (last_a[v] < 0 && !(kept[v] && read[v])) {
         g.finish(v);
         g.settle();
       }
@@ -346,8 +375,10 @@ std::string lu_jit_source(const LuJitInput& in) {
   };
   // pass 1: the loaded values' first-use order
   Gen first(in);
+  first.kept = kept;
   walk(first);
   Gen g(in);
+  g.kept = kept;
   g.record = false;
   g.order = first.order;
   g.pos = first.pos;

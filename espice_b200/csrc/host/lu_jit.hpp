@@ -26,6 +26,10 @@ struct LuJitInput {
   // register budget, in values: beyond it the final tape values needed
   // farthest ahead are let go and re-read from their plane at next use
   uint32_t resident_values = 48;
+  // false: the factors stay on the lane (dx and the verdict alone go out); an
+  // entry the ops never write is read again from A when let go, and only
+  // those they do write, and the back solve needs, go to `tv`
+  bool factors_out = true;
   // the mixed form: FP32 factors and solves, then FP64 refinement on the
   // residual over the pattern (col_ptr, row_idx), kernel `lu_tape_mixed`
   bool mixed = false;
@@ -37,7 +41,8 @@ struct LuJitInput {
 // [entry][lane] planes, every tape value a local variable, each op one
 // statement in the given order; the tape values go to their plane `tv`
 // (the caller's, or scratch) as they become final and come back from it
-// when their next use is far off.
+// when their next use is far off. A caller that wants no factors gets the
+// form without their stores (factors_out).
 std::string lu_jit_source(const LuJitInput& in);
 
 struct LuJitKernels {

@@ -1,0 +1,141 @@
+"""The task programs at the edges of their forms (B200): one warp's stream, a
+CTA's of 256 and of 128 threads, compact and wide words, shared memory and
+the slab. Every form runs the same operations in the same order, so the
+lanes agree bit for bit.
+
+- A lane of a batch large enough for the narrow CTAs equals the same lane of
+  a small batch (wide CTAs), FP64 and mixed.
+- FP64 block lanes equal the warp lanes.
+- A value space past the compact words' 65,536 equals the oracle.
+- Training: a step replayed as a graph equals one launched by itself.
+"""
+
+import numpy as np
+import pytest
+
+from espice_b200 import decks, lanes, mlp
+from espice_b200.circuit import Circuit
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def ladder(sections):
+    """A resistor ladder with a diode at its end: sections + 3 unknowns."""
+    c = Circuit()
+    c.V("vin", "n0", "0", dc=1.0)
+    for k in range(sections):
+        c.R(f"r{k}", f"n{k}", f"n{k + 1}", 100.0 + k)
+        c.R(f"g{k}", f"n{k + 1}", "0", 1e4)
+    c.D("d0", f"n{sections}", "0", is_=1e-14, n=1.0, rs=10.0)
+    fr = c.freeze()
+    return fr, [fr.slot("vin", "dc")], lambda n: np.linspace(0.5, 3.0, n).reshape(-1, 1)
+
+
+def mesh(size):
+    fr, slots = decks.mesh_gates(size)
+    return fr, slots, lambda n: np.linspace(0.8, 1.8, n).reshape(-1, 1)
+
+
+def grid(_):
+    fr, slots, _ = decks.grid_diodes(seed=1)
+    return fr, slots, lambda n: np.linspace(0.0, 5.0, n).reshape(-1, 1)
+
+
+def solve(fr, slots, values, precision, path):
+    ctx = lanes.DcLanes(fr)
+    ctx.set_mode(precision=precision, path=path)
+    ctx.set_lanes(slots, values)
+    x, it, st, stats = ctx.solve(x0=np.zeros(fr.n))
+    ctx.close()
+    return x.view(np.uint64), it, st
+
+
+@pytest.mark.parametrize("precision", [lanes.PREC_FP64, lanes.PREC_MIXED])
+@pytest.mark.parametrize("deck,size", [(ladder, 1), (ladder, 31), (ladder, 130), (grid, 0), (mesh, 50), (mesh, 200),
+                                       (mesh, 400)])
+def test_narrow_ctas_equal_wide(deck, size, precision):
+    fr, slots, values = deck(size)
+    # 1,200 lanes: more than any form holds at once on wide CTAs
+    big = values(1200)
+    pick = np.r_[0:3, 593:596, 1197:1200]
+    a = solve(fr, slots, big, precision, lanes.PATH_BLOCK)
+    b = solve(fr, slots, big[pick], precision, lanes.PATH_BLOCK)
+    for u, v in zip(a, b):
+        assert np.array_equal(u[pick], v)
+
+
+@pytest.mark.parametrize("deck,size", [(ladder, 1), (ladder, 28), (ladder, 29), (ladder, 61), (grid, 0), (mesh, 50)])
+def test_block_lanes_equal_warp_lanes(deck, size):
+    fr, slots, values = deck(size)
+    v = values(17)
+    a = solve(fr, slots, v, lanes.PREC_FP64, lanes.PATH_WARP)
+    b = solve(fr, slots, v, lanes.PREC_FP64, lanes.PATH_BLOCK)
+    for u, w in zip(a, b):
+        assert np.array_equal(u, w)
+
+
+def test_wide_words_equal_the_oracle():
+    """A mesh of 2,500 unknowns: past 65,536 values."""
+    fr, slots, values = mesh(2500)
+    v = values(2)
+    ctx = lanes.DcLanes(fr)
+    ctx.set_mode(precision=lanes.PREC_FP64, path=lanes.PATH_BLOCK)
+    ctx.set_lanes(slots, v)
+    x, it, st, _ = ctx.solve(x0=np.zeros(fr.n))
+    assert ctx.block_info()["ntv"] + fr.n + 3 >= 65536
+    ctx.close()
+    xo, ito, cv = oracle.dc_points(fr, slots, v, warm=np.zeros(fr.n))
+    assert np.array_equal(st == lanes.LANE_CONVERGED, cv.astype(bool)) and np.array_equal(it, ito)
+    assert np.array_equal(x.view(np.uint64), xo.view(np.uint64))
+
+
+@pytest.mark.parametrize("epochs", [1, 2, 3, 5])
+def test_graph_steps_equal_single_steps(epochs):
+    """Equal rows (any order the same batch): a run of several steps, all but
+    the first replayed, ends in the weights of as many runs of one."""
+    import torch
+    x = torch.full((16, 5), 0.3, device="cuda") * torch.arange(1, 6, device="cuda")
+    y = torch.full((16, 19), 0.7, device="cuda") - 0.1 * torch.arange(19, device="cuda")
+    torch.cuda.synchronize()
+    one, many = (mlp.Mlp(5, 32, 3, 19, seed=4) for _ in range(2))
+    la = many.train(x.data_ptr(), y.data_ptr(), 16, epochs=epochs, batch=16, lr=1e-2)
+    lb = [one.train(x.data_ptr(), y.data_ptr(), 16, epochs=1, batch=16, lr=1e-2)[0] for _ in range(epochs)]
+    assert np.array_equal(la, np.array(lb, np.float32))
+    for (wa, ba), (wb, bb) in zip(many.weights(), one.weights()):
+        assert np.array_equal(wa, wb) and np.array_equal(ba, bb)
+    one.close()
+    many.close()
+
+
+@pytest.mark.parametrize("deck", ["ring", "grid"])
+def test_compiled_lu_without_the_factors(deck):
+    """dx and the verdicts with and without the factors' planes, a dead pivot
+    and a tiny matrix among the lanes."""
+    import torch
+    fr = decks.ring_oscillator(lanes=2)[0] if deck == "ring" else decks.grid_diodes(seed=1)[0]
+    cp, ri = lanes.pattern(fr)
+    rng = np.random.default_rng(3)
+    lead = rng.uniform(0.5, 2.0, len(ri)) * rng.choice((-1.0, 1.0), len(ri))
+    diag = np.array([np.searchsorted(ri[cp[j]:cp[j + 1]], j) + cp[j] for j in range(fr.n)])
+    lead[diag] += 8.0
+    n = 131
+    vals = lead[:, None] * rng.uniform(0.8, 1.2, (len(ri), n))
+    vals[diag[3], 5] = 0.0
+    vals[:, 7] *= 1e-9
+    vals[diag[2], 9] = np.inf
+    a = torch.tensor(vals, device="cuda")
+    rhs = torch.tensor(rng.normal(size=(fr.n, n)), device="cuda")
+    dx = [torch.zeros((fr.n, n), dtype=torch.float64, device="cuda") for _ in range(2)]
+    bad = [torch.zeros(n, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    ctx = lanes.DcLanes(fr)
+    torch.cuda.synchronize()
+    ctx.lu_lanes_compiled(lead, a.data_ptr(), rhs.data_ptr(), dx[0].data_ptr(), bad[0].data_ptr(), n)
+    tv = torch.zeros((ctx.tape_size()[2], n), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx.lu_lanes_compiled(lead, a.data_ptr(), rhs.data_ptr(), dx[1].data_ptr(), bad[1].data_ptr(), n, tv.data_ptr())
+    ctx.close()
+    b = [v.cpu().numpy() for v in bad]
+    assert np.array_equal(b[0], b[1]) and b[0].any() and not b[0].all()
+    x = [v.cpu().numpy()[:, b[0] == 0].view(np.uint64) for v in dx]
+    assert np.array_equal(x[0], x[1])
