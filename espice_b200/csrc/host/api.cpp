@@ -266,6 +266,7 @@ struct esl_ctx {
   DevBuf d_tran_state, d_tran_save;    // paused transient lanes' state
   esl_stats last_peels{};              // the last call's peel counts (esl_peel_stats)
   uint64_t last_tran_refinements = 0;  // the last block transient's FP64 corrections (mixed)
+  bool have_seq = false;
   uint32_t n_seq_a = 0, n_seq = 0, seq_warps = 0;  // lane-interleaved op list
   uint32_t n_seq_f = 0, mixed_warps = 0;            // its forward-only tail, the mixed kernel's warps
   LuJitKernels lu_jit;                               // the tape-compiled lane LU of the current tape
@@ -733,6 +734,7 @@ int32_t upload_tape(esl_ctx* ctx) {
   T.pinv = ctx->d_pinv.as<uint32_t>();
   T.qcol = ctx->d_q.as<uint32_t>();
   for (BlockTables& t : ctx->block) t.have = false;  // a new tape needs its own block programs
+  ctx->have_seq = false;        // its own op list
   lu_jit_release(ctx->lu_jit);  // and its own compiled LU
   ctx->lu_jit_state = 0;
   lu_jit_release(ctx->lu_jit_dx);
@@ -796,25 +798,24 @@ int32_t upload_tape(esl_ctx* ctx) {
   ctx->tran_lanes_eff = T.prog_bytes + tran_bytes > room
                             ? 0
                             : std::max<uint32_t>(1, std::min<uint32_t>(8, uint32_t((room - T.prog_bytes) / tran_bytes)));
-  // The sequential op list of the lane-interleaved kernel: the programs'
-  // real ops in row order (padding writes the sink, nv - 1).
-  {
-    std::vector<Op> seq = lane_sequence(P, ctx->n_seq_a, ctx->n_seq, ctx->n_seq_f);
-    ESL_CUDA(upload(ctx->d_seq, seq, s));
-    ctx->mixed_warps = 0;
-    for (uint32_t w = 8; w >= 1; --w)
-      if (lu_lanes_mixed_smem(T, ctx->n_seq + ctx->n_seq_f, w) <= room) {
-        ctx->mixed_warps = w;
-        break;
-      }
-    ctx->seq_warps = 0;
-    for (uint32_t w = 8; w >= 1; --w)
-      if (lu_lanes_smem(T, ctx->n_seq, w) <= room) {
-        ctx->seq_warps = w;
-        break;
-      }
-  }
   ctx->warp_ok = true;
+  return ESL_OK;
+}
+
+// The op list of the lane-interleaved kernels, at their first call on a tape
+// (packing the rows it follows took longer than all else of a tape's set-up).
+int32_t ensure_sequence(esl_ctx* ctx) {
+  if (ctx->have_seq) return ESL_OK;
+  pack_op_rows(ctx->prog);
+  const std::vector<Op> seq = lane_sequence(ctx->prog, ctx->n_seq_a, ctx->n_seq, ctx->n_seq_f);
+  ESL_CUDA(upload(ctx->d_seq, seq, ctx->stream));
+  const size_t room = size_t(227) * 1024;
+  ctx->mixed_warps = ctx->seq_warps = 0;
+  for (uint32_t w = 8; w >= 1 && !ctx->mixed_warps; --w)
+    if (lu_lanes_mixed_smem(ctx->topo, ctx->n_seq + ctx->n_seq_f, w) <= room) ctx->mixed_warps = w;
+  for (uint32_t w = 8; w >= 1 && !ctx->seq_warps; --w)
+    if (lu_lanes_smem(ctx->topo, ctx->n_seq, w) <= room) ctx->seq_warps = w;
+  ctx->have_seq = true;
   return ESL_OK;
 }
 
@@ -2211,6 +2212,7 @@ int32_t esl_compile_tape(uint32_t n, const uint32_t* col_ptr, const uint32_t* ro
   lu.keep_min = kGrowthLimit;
   if (!lu.factor(lead, kPivotTol)) return ESL_NOT_ELIGIBLE;
   Programs P = compile_tape(lu);
+  pack_op_rows(P);
   info->nu = P.nu;
   info->nl = P.nl;
   info->ntv = P.ntv;
@@ -2286,6 +2288,7 @@ int32_t esl_lu_lanes_device(esl_ctx* ctx, const double* lead, uint32_t n_lanes, 
     if (int32_t rc = build_tape_from(ctx, lead)) return rc;
   }
   if (int32_t rc = warp_only(ctx)) return rc;
+  if (int32_t rc = ensure_sequence(ctx)) return rc;
   if (ctx->seq_warps == 0) return ctx->fail(ESL_NOT_ELIGIBLE, "a warp's interleaved lane values exceed shared memory");
   ESL_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
   ESL_CUDA(launch_lu_lanes(ctx->topo, ctx->d_seq.as<uint2>(), ctx->n_seq_a, ctx->n_seq, n_lanes, d_a, d_rhs, d_tv,
@@ -2402,6 +2405,7 @@ int32_t esl_lu_lanes_mixed_device(esl_ctx* ctx, const double* lead, uint32_t n_l
     if (int32_t rc = build_tape_from(ctx, lead)) return rc;
   }
   if (int32_t rc = warp_only(ctx)) return rc;
+  if (int32_t rc = ensure_sequence(ctx)) return rc;
   if (ctx->mixed_warps == 0) return ctx->fail(ESL_NOT_ELIGIBLE, "a warp's interleaved lane values exceed shared memory");
   ESL_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
   ESL_CUDA(launch_lu_lanes_mixed(ctx->topo, ctx->d_seq.as<uint2>(), ctx->n_seq_a, ctx->n_seq, ctx->n_seq_f, n_lanes,

@@ -121,6 +121,25 @@ void pack(const std::vector<SeqOp>& seq, uint32_t space, std::vector<Op>& rows, 
 
 }  // namespace
 
+namespace {
+
+// Ops on the longest dependence chain (each op after the last write of the
+// values it reads and of its destination).
+uint32_t longest_chain(const std::vector<SeqOp>& seq, uint32_t nv) {
+  std::vector<uint32_t> level(nv, 0);
+  uint32_t top = 0;
+  for (const SeqOp& s : seq) {
+    uint32_t l = level[s.dst];
+    for (uint32_t x : {s.a, s.b})
+      if (x != kNone) l = std::max(l, level[x]);
+    level[s.dst] = l + 1;
+    top = std::max(top, l + 1);
+  }
+  return top;
+}
+
+}  // namespace
+
 Programs compile_tape(const SparseLu& lu) {
   Programs P;
   const Csc& A = *lu.a;
@@ -166,7 +185,7 @@ Programs compile_tape(const SparseLu& lu) {
     P.a_list.push_back(encode(s.kind, s.dst, s.a, s.b));
     P.a_seq.push_back(Op4{s.dst | (s.kind << 28), s.a == kNone ? 0u : s.a, s.b == kNone ? 0u : s.b, 0u});
   }
-  if (P.nv < 65536) pack(a, P.nv, P.a_ops, P.a_rows, P.a_levels);
+  if (P.nv < 65536) P.a_levels = longest_chain(a, P.nv);
   P.a_nops = uint32_t(a.size());
 
   std::vector<uint8_t> written(P.ntv, 0);
@@ -188,7 +207,7 @@ Programs compile_tape(const SparseLu& lu) {
     P.b_list.push_back(encode(s.kind, s.dst, s.a, s.b));
     P.b_seq.push_back(Op4{s.dst | (s.kind << 28), s.a, s.b, 0u});
   }
-  if (P.nv < 65536) pack(b, P.nv, P.b_ops, P.b_rows, P.b_levels);
+  if (P.nv < 65536) P.b_levels = longest_chain(b, P.nv);
   P.b_nops = uint32_t(b.size());
   return P;
 }
@@ -439,6 +458,13 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv, uint32_t warps
 
 }  // namespace
 
+void pack_op_rows(Programs& P) {
+  if (P.nv >= 65536 || !P.a_ops.empty() || !P.b_ops.empty()) return;
+  uint32_t levels = 0;
+  pack(unpack(P.a_seq), P.nv, P.a_ops, P.a_rows, levels);
+  pack(unpack(P.b_seq), P.nv, P.b_ops, P.b_rows, levels);
+}
+
 void compile_warp(const Programs& P, TaskStream& a, TaskStream& b) {
   a = pack_tasks(unpack(P.a_seq), P.nv, 1, true);
   b = pack_tasks(unpack(P.b_seq), P.nv, 1, true);
@@ -456,15 +482,7 @@ BlockPrograms compile_block(const Programs& P, uint32_t warps) {
   for (const SeqOp& s : a)
     if (s.kind == kOpSubNz) f.push_back(s);
   B.f = pack_tasks(f, P.nv, warps, B.compact);
-  // the longest dependence chain of single ops
-  std::vector<uint32_t> level(P.nv, 0);
-  for (const SeqOp& s : a) {
-    uint32_t l = level[s.dst];
-    for (uint32_t x : {s.a, s.b})
-      if (x != kNone) l = std::max(l, level[x]);
-    level[s.dst] = l + 1;
-    B.a_levels = std::max(B.a_levels, l + 1);
-  }
+  B.a_levels = longest_chain(a, P.nv);
   return B;
 }
 

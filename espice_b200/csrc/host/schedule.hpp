@@ -70,6 +70,9 @@ struct BlockPrograms {
 // sequential order, so the programs are bitwise the column replay and the
 // sparse triangular solves.
 Programs compile_tape(const SparseLu& lu);
+// The rows of 32 single ops (a_ops, b_ops and their counts; value spaces
+// below 65,536), which the interpreted lane LU and esl_compile_tape take.
+void pack_op_rows(Programs& P);
 
 // The warp lanes' programs A and B as one warp's compact task stream each
 // (value spaces below 65,536).
