@@ -212,7 +212,7 @@ cudaError_t upload(DevBuf& b, const std::vector<T>& v, cudaStream_t s) {
 struct BlockTables {
   bool have = false;
   BlockPrograms prog;
-  uint32_t g_len[kBlockThreads / 32] = {}, g_terms = 0, g_ncells = 0;
+  uint32_t g_len[kBlockBroad / 32] = {}, g_terms = 0, g_ncells = 0;
   DevBuf d_a, d_b, d_f, d_terms, d_cells;
 };
 
@@ -254,7 +254,7 @@ struct esl_ctx {
   uint32_t refine_max = 6;
   double refine_skip = 0.0;  // mixed: steps above this many tolerances go unrefined (0: none)
   bool profile = false;  // block lanes: accumulate the phase cycles (esl_solve_mode.profile)
-  BlockTables block[2];  // CTAs of kBlockThreads, of kBlockNarrow threads
+  BlockTables block[3];  // CTAs of kBlockThreads, kBlockNarrow, kBlockBroad threads
   DevBuf d_slab, d_refine, d_prof;
   SparseLu lead;
   Programs prog;
@@ -897,9 +897,11 @@ void build_block_gather(const esl_ctx* ctx, uint32_t W, std::vector<uint32_t>& t
 
 constexpr size_t kBlockSmemRoom = size_t(227) * 1024 - 256;
 
+uint32_t block_width(uint32_t threads) { return threads == kBlockNarrow ? 1u : threads == kBlockBroad ? 2u : 0u; }
+
 // The block lanes' tables of the current tape for CTAs of `threads`.
 int32_t ensure_block(esl_ctx* ctx, uint32_t threads) {
-  BlockTables& t = ctx->block[threads == kBlockNarrow];
+  BlockTables& t = ctx->block[block_width(threads)];
   if (t.have) return ESL_OK;
   cudaStream_t s = ctx->stream;
   t.prog = compile_block(ctx->prog, threads / 32);
@@ -980,13 +982,21 @@ int block_place(const TopoDev& T, bool mixed, uint32_t threads, BlockDev& D) {
 // rows are a chain of latencies that issues on a quarter of the cycles, so
 // four narrow lanes on an SM take less than twice the time of two wide ones
 // (analog block, mixed, 12,288 points: 78.9 -> 64.7 ms when this came in);
-// with fewer lanes the wide CTA's lane is the faster one.
-int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D, bool narrow_ok = false) {
+// with fewer lanes the wide CTA's lane is the faster one. The broad CTA for
+// slab lanes that have an SM each: their rows wait for L2, and sixteen warps
+// take half the rows (2,000-unknown digital block: 1,113 -> 620; working
+// sets in shared memory are smaller, their rows are chains that 256 threads
+// already hold).
+int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D, bool narrow_ok = false,
+                   bool broad_ok = false) {
   const TopoDev& T = ctx->topo;
   D = BlockDev{};
   uint32_t threads = kBlockThreads;
   int best = block_place(T, mixed, threads, D);
-  if (narrow_ok && n_lanes > uint32_t(ctx->sms) * uint32_t(best)) {
+  if (broad_ok && !D.in_smem && n_lanes <= uint32_t(ctx->sms)) {
+    threads = kBlockBroad;
+    best = block_place(T, mixed, threads, D);
+  } else if (narrow_ok && n_lanes > uint32_t(ctx->sms) * uint32_t(best)) {
     BlockDev N{};
     const int narrow = block_place(T, mixed, kBlockNarrow, N);
     if (N.in_smem && narrow > best) {
@@ -996,7 +1006,7 @@ int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D, bool
     }
   }
   if (int32_t rc = ensure_block(ctx, threads)) return rc;
-  const BlockTables& B = ctx->block[threads == kBlockNarrow];
+  const BlockTables& B = ctx->block[block_width(threads)];
   D.T = T;
   D.threads = threads;
   auto program = [](BlockProgram& p, const DevBuf& d, const TaskStream& t) {
@@ -1394,7 +1404,7 @@ int32_t dc_solve(esl_ctx* ctx, const esl_newton_opts* opts, double* d_x, int col
   const bool mixed = ctx->precision == ESL_PREC_MIXED && !d_rung;
   BlockDev D{};
   if (block) {
-    if (int32_t rc = block_view(ctx, mixed, N, D, !d_rung)) return rc;
+    if (int32_t rc = block_view(ctx, mixed, N, D, !d_rung, !d_rung)) return rc;
     if (D.refine_out) ESL_CUDA(cudaMemsetAsync(D.refine_out, 0, size_t(N) * 4, s));
     if (D.prof) ESL_CUDA(cudaMemsetAsync(D.prof, 0, kBlockPhases * sizeof(unsigned long long), s));
   }
@@ -1633,7 +1643,7 @@ int32_t run_tran_block(esl_ctx* ctx, LaneDev L, TranDev P, const LaneOpts& lo) {
   if (P.meas) return ctx->fail(ESL_NOT_ELIGIBLE, "the block transient lanes stream no measure cards");
   const bool mixed = ctx->precision == ESL_PREC_MIXED;
   BlockDev D{};
-  if (int32_t rc = block_view(ctx, mixed, N, D)) return rc;
+  if (int32_t rc = block_view(ctx, mixed, N, D, false, true)) return rc;
   if (mixed) ESL_CUDA(cudaMemsetAsync(D.refine_out, 0, size_t(N) * 4, s));
   ESL_CUDA(ctx->d_tran_slab.ensure(size_t(D.grid) * tran_block_slab(ctx->topo) * 8));
   ESL_CUDA(ctx->d_x_good.ensure(size_t(N) * ctx->topo.n * 8));

@@ -50,7 +50,7 @@ struct Programs {
 // (common.h) its lanes run between two barriers: warp w's chunks are
 // off[w] .. off[w + 1] (in chunks of 32 * task_words words), the last
 // kTaskRing of them only read ahead.
-constexpr uint32_t kTaskWarps = 8;  // a block lane's CTA has at most this many
+constexpr uint32_t kTaskWarps = 16;  // a block lane's CTA has at most this many
 struct TaskStream {
   std::vector<uint32_t> words;
   uint32_t off[kTaskWarps + 1] = {};

@@ -585,8 +585,9 @@ __global__ void __launch_bounds__(kW) block_lead_kernel(BlockDev D, LaneDev L, u
 // The DC kernel of a CTA width.
 template <typename V, bool kHasB3>
 auto dc_kernel(uint32_t threads) {
-  return threads == kBlockNarrow ? dc_block_kernel<V, kHasB3, kBlockNarrow, false>
-                                 : dc_block_kernel<V, kHasB3, kBlockThreads, false>;
+  return threads == kBlockNarrow  ? dc_block_kernel<V, kHasB3, kBlockNarrow, false>
+         : threads == kBlockBroad ? dc_block_kernel<V, kHasB3, kBlockBroad, false>
+                                  : dc_block_kernel<V, kHasB3, kBlockThreads, false>;
 }
 
 template <typename V, bool kHasB3>
@@ -1110,7 +1111,7 @@ __device__ void block_tran_lane(const BlockDev& D, const LaneDev& L, const TranD
 // set placed as the DC block lanes place it (shared memory, split or slab),
 // the run state in the CTA's part of tslab.
 template <typename V, bool kHasB3, uint32_t kW>
-__global__ void __launch_bounds__(kW, 2) tran_block_kernel(BlockDev D, LaneDev L, TranDev P, LaneOpts o,
+__global__ void __launch_bounds__(kW, 512 / kW) tran_block_kernel(BlockDev D, LaneDev L, TranDev P, LaneOpts o,
                                                           double* tslab, size_t tslab_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint64_t red[kW / 32];
@@ -1126,12 +1127,13 @@ __global__ void __launch_bounds__(kW, 2) tran_block_kernel(BlockDev D, LaneDev L
 template <typename V, bool kHasB3>
 cudaError_t launch_tran_t(const BlockDev& D, const LaneDev& L, const TranDev& P, const LaneOpts& o, double* tslab,
                           size_t tslab_stride, cudaStream_t s) {
-  auto* k = tran_block_kernel<V, kHasB3, kBlockThreads>;
+  auto* k = D.threads == kBlockBroad ? tran_block_kernel<V, kHasB3, kBlockBroad>
+                                     : tran_block_kernel<V, kHasB3, kBlockThreads>;
   const size_t smem = D.ring_bytes + (D.in_smem ? D.lane_bytes : 0);
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   const uint32_t grid = D.grid < L.n_lanes ? D.grid : L.n_lanes;
-  k<<<grid > 0 ? grid : 1, kBlockThreads, smem, s>>>(D, L, P, o, tslab, tslab_stride);
+  k<<<grid > 0 ? grid : 1, D.threads, smem, s>>>(D, L, P, o, tslab, tslab_stride);
   return cudaGetLastError();
 }
 

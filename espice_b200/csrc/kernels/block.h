@@ -15,6 +15,8 @@ namespace esl {
 constexpr uint32_t kBlockThreads = 256;
 // Threads of the narrow form, for more lanes an SM (DC lanes).
 constexpr uint32_t kBlockNarrow = 128;
+// Threads of the broad form, for lanes that have an SM each.
+constexpr uint32_t kBlockBroad = 512;
 // The block lanes' assembly streams (see block_assemble): a term word is a
 // staging index, with kGTermEnd on a cell's last term. Three cells past the
 // device stamps hold constants, so every term is a plain load: n_stage +
@@ -32,7 +34,7 @@ constexpr uint32_t kGBatch = 8;  // terms a thread takes at a time, two batches 
 // chunks.
 struct BlockProgram {
   const uint32_t* words;
-  uint32_t off[kBlockThreads / 32 + 1];
+  uint32_t off[kBlockBroad / 32 + 1];
 };
 
 struct BlockDev {
@@ -46,7 +48,7 @@ struct BlockDev {
   // (block_assemble), cell stream [c][threads] (uint4).
   const uint32_t* g_terms;
   const uint4* g_cells;
-  uint32_t g_len[kBlockThreads / 32];
+  uint32_t g_len[kBlockBroad / 32];
   // A lane's working set, byte offsets: limited images, the value space v
   // (FP64, or FP32 in the mixed form), x, rhs, diag, dx (FP64, n each), the
   // FP64 matrix (mixed form: nnz), xo (n) and the staging cells. Split: a
@@ -57,7 +59,7 @@ struct BlockDev {
   uint32_t in_smem;     // 1: (the hot part) in the CTA's shared memory; 0: all in its slab of `slab`
   uint32_t split;       // 1: xo and the staging cells in the CTA's slab; 2: all from x on; cold_bytes each
   uint32_t cold_bytes;
-  uint32_t threads;     // of a CTA (kBlockThreads or kBlockNarrow)
+  uint32_t threads;     // of a CTA (kBlockThreads, kBlockNarrow or kBlockBroad)
   uint32_t grid;        // CTAs of a launch (persistent)
   unsigned char* slab;  // per CTA: the working set (in_smem 0) or its cold part (split), and the lead assembly's scratch
   // Mixed form: refinement stops at max |res| <= refine_tol * max |rhs| or
