@@ -707,6 +707,14 @@ std::string compiled_lu_source(uint32_t nnz, const SparseLu& lu, const Programs&
   in.factors_out = factors_out;
   in.col_ptr = &lu.a->col_ptr;
   in.row_idx = &lu.a->row_idx;
+  // A tape of at most 256 values keeps most of them in 112 registers' worth
+  // of two CTAs an SM: its traffic falls by more than the halved warps cost
+  // (131,072 lanes, ring's 226 values: with the factors 123 -> 100 us,
+  // without 106 -> 82; the grid's 789 values: 938 -> 1,151).
+  if (!mixed && P.ntv + P.n <= 256) {
+    in.resident_values = 112;
+    in.min_blocks = 2;
+  }
   if (mixed) in.resident_values = 48;  // the refinement loop needs the registers (more spilled)
   if (resident) in.resident_values = resident;
   return lu_jit_source(in);

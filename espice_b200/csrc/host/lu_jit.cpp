@@ -28,12 +28,10 @@ namespace esl {
 
 namespace {
 
-// 128 threads, at least 4 CTAs per SM: 128 registers a thread, 16 warps
-// per SM. On the B200 this beat the unbounded form (about 240 registers,
-// 8 warps) by 20% on the ring's tape and the grid's, and an L2 prefetch of
+// 128 threads; four CTAs an SM (128 registers a thread, 16 warps) unless the
+// tape is small enough to stay in registers (min_blocks). An L2 prefetch of
 // every A row at the start gained nothing.
 constexpr uint32_t kThreads = 128;
-constexpr uint32_t kMinBlocks = 4;
 // The A and rhs entries a lane reads arrive through shared memory in
 // stages of kStage entries in first-use order, two stages in flight
 // (cp.async into a per-thread double buffer: 2 x 24 x 128 x 8 B = 48 KB a
@@ -404,12 +402,12 @@ std::string lu_jit_source(const LuJitInput& in) {
      << "}\n"
      << "#endif\n";
   if (in.mixed)
-    os << "extern \"C\" __global__ void __launch_bounds__(" << kThreads << ", " << kMinBlocks << ") lu_tape_mixed(\n"
+    os << "extern \"C\" __global__ void __launch_bounds__(" << kThreads << ", " << in.min_blocks << ") lu_tape_mixed(\n"
        << "    const double* __restrict__ a, const double* __restrict__ rhs, float* __restrict__ tv,\n"
        << "    double* __restrict__ dx, unsigned char* __restrict__ bad_out, unsigned char* __restrict__ refine_out,\n"
        << "    unsigned n_lanes) {\n";
   else
-    os << "extern \"C\" __global__ void __launch_bounds__(" << kThreads << ", " << kMinBlocks << ") lu_tape(\n"
+    os << "extern \"C\" __global__ void __launch_bounds__(" << kThreads << ", " << in.min_blocks << ") lu_tape(\n"
        << "    const double* __restrict__ a, const double* __restrict__ rhs, double* __restrict__ tv,\n"
        << "    double* __restrict__ dx, unsigned char* __restrict__ bad_out, unsigned n_lanes) {\n";
   os

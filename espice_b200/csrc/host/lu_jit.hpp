@@ -26,6 +26,7 @@ struct LuJitInput {
   // register budget, in values: beyond it the final tape values needed
   // farthest ahead are let go and re-read from their plane at next use
   uint32_t resident_values = 48;
+  uint32_t min_blocks = 4;  // CTAs of 128 threads an SM the registers are bounded for
   // false: the factors stay on the lane (dx and the verdict alone go out); an
   // entry the ops never write is read again from A when let go, and only
   // those they do write, and the back solve needs, go to `tv`
