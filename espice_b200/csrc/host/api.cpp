@@ -261,11 +261,12 @@ struct esl_ctx {
 
   DevBuf d_nodes[kMaxBatches], d_rhs_ptr, d_rhs_src, d_a_ptr, d_a_src, d_slot_row, d_cur;
   DevBuf d_q_ptr, d_q_src, d_c_ptr, d_c_src, d_probes, d_tran_t, d_tran_v, d_tran_n, d_tran_stats;
-  DevBuf d_amap, d_fill, d_prog, d_l_scaled, d_pinv, d_q, d_seq, d_sweep_values, d_meas, d_next_lane;
+  DevBuf d_amap, d_fill, d_prog, d_l_scaled, d_pinv, d_q, d_seq, d_tasks, d_sweep_values, d_meas, d_next_lane;
   DevBuf d_sweep_state, d_sweep_rows;  // paused sweep lanes' state
   DevBuf d_tran_state, d_tran_save;    // paused transient lanes' state
   esl_stats last_peels{};              // the last call's peel counts (esl_peel_stats)
   uint64_t last_tran_refinements = 0;  // the last block transient's FP64 corrections (mixed)
+  uint32_t warp_bytes = 0;  // what decides whether a lane is a warp lane (upload_tape)
   bool have_seq = false;
   uint32_t n_seq_a = 0, n_seq = 0, seq_warps = 0;  // lane-interleaved op list
   uint32_t n_seq_f = 0, mixed_warps = 0;            // its forward-only tail, the mixed kernel's warps
@@ -755,6 +756,7 @@ int32_t upload_tape(esl_ctx* ctx) {
   // the block lanes only.
   ctx->warp_ok = false;
   if (P.nv >= 65536) return ESL_OK;
+  size_t most_lane = 0;
   {
     // One blob: the tasks of A and B, gather depth/off/src/dst, each section
     // 16-byte aligned.
@@ -766,14 +768,12 @@ int32_t upload_tape(esl_ctx* ctx) {
       blob.resize((blob.size() + 15) & ~size_t(15), 0);
       return at;
     };
-    // a stream's first chunk beyond its last is read ahead
     TaskStream A, B;
     compile_warp(P, A, B);
     const uint32_t chunk = 32 * task_words(true) * 4;
     T.a_chunks = A.off[1] - kTaskRing;
     T.b_chunks = B.off[1] - kTaskRing;
-    T.o_a_tasks = put(A.words.data(), (T.a_chunks + 1) * chunk);
-    T.o_b_tasks = put(B.words.data(), (T.b_chunks + 1) * chunk);
+    T.tasks = nullptr;
     T.o_g_src = put(G.src.data(), G.src.size() * 4);
     T.o_g_dst = put(G.dst.data(), G.dst.size() * 4);
     uint32_t n_kr = 0;
@@ -784,6 +784,26 @@ int32_t upload_tape(esl_ctx* ctx) {
     T.o_k_dst = put(K.dst.data(), K.dst.size() * 4);
     T.n_kr_groups = n_kr;
     T.n_ks_groups = uint32_t(K.depth.size()) - n_kr;
+    const size_t gathers = blob.size();
+    // The tasks' words (a stream's first chunk beyond its last is read ahead)
+    // beside the gathers when that leaves room for the largest lane there is,
+    // a transient one with every measure card; else in global memory, with a
+    // ring of 2 KB a warp.
+    const size_t nt = lane_layout(T.n, T.ntv, T.n_stage, T.nlim).total + 9 * size_t(T.n) + 5 * size_t(T.n_qt) +
+                      9 * size_t(T.n_src) + 2 + kMeasDoubles * kMaxMeas;
+    if (blob.size() + size_t(T.a_chunks + T.b_chunks + 2) * chunk + nt * 8 <= size_t(227) * 1024) {
+      T.o_a_tasks = put(A.words.data(), (T.a_chunks + 1) * chunk);
+      T.o_b_tasks = put(B.words.data(), (T.b_chunks + 1) * chunk);
+    } else {
+      T.b_first = A.off[1];
+      T.o_ring = uint32_t(blob.size());
+      blob.resize(blob.size() + task_ring_bytes(8, true), 0);
+      A.words.insert(A.words.end(), B.words.begin(), B.words.end());
+      ESL_CUDA(upload(ctx->d_tasks, A.words, s));
+      T.tasks = ctx->d_tasks.as<uint32_t>();
+    }
+    ctx->warp_bytes = uint32_t(gathers);
+    most_lane = nt * 8;
     ESL_CUDA(upload(ctx->d_prog, blob, s));
     T.prog = ctx->d_prog.as<unsigned char>();
     T.prog_bytes = uint32_t(blob.size());
@@ -794,7 +814,22 @@ int32_t upload_tape(esl_ctx* ctx) {
   // Every CTA stages the programs; as many lanes per CTA as fit beside them.
   const size_t lane_bytes = size_t(T.smem_doubles) * 8;
   const size_t room = size_t(227) * 1024;
-  if (T.prog_bytes + lane_bytes > room) return ESL_OK;
+  // Which circuits are warp lanes is decided on the programs as rows of 32
+  // single ops beside the gathers (the tasks need no more room than that), so
+  // that a call's route does not hang on how they are packed. The rows are
+  // packed only when their bounds leave it open: a full row takes 32 ops, and
+  // of two rows that are not full the longest path to the end gets shorter.
+  const size_t least = (P.a_nops + 31) / 32 + (P.b_nops + 31) / 32;
+  const size_t most = least + 2 * (size_t(P.a_levels) + P.b_levels);
+  constexpr size_t kRowBytes = 32 * sizeof(Op);
+  if (ctx->warp_bytes + least * kRowBytes + lane_bytes > room) return ESL_OK;
+  if (ctx->warp_bytes + most * kRowBytes + most_lane <= room) {
+    ctx->warp_bytes += uint32_t(most * kRowBytes);
+  } else {
+    pack_op_rows(P);
+    ctx->warp_bytes += uint32_t((P.a_ops.size() + P.b_ops.size()) * sizeof(Op));
+    if (ctx->warp_bytes + lane_bytes > room) return ESL_OK;
+  }
   ctx->lanes_eff = std::max<uint32_t>(1, std::min<uint32_t>(8, uint32_t((room - T.prog_bytes) / lane_bytes)));
   // Transient lanes add the accepted points, the charge rings and dynamic
   // currents over the rows and the LTE states: cur | prev | q[4] | ip over
@@ -803,7 +838,7 @@ int32_t upload_tape(esl_ctx* ctx) {
   // per source).
   T.tran_doubles = (T.smem_doubles + 7 * T.n + 5 * T.n_qt + 9 * T.n_src + 1) & ~1u;
   const size_t tran_bytes = size_t(T.tran_doubles) * 8;
-  ctx->tran_lanes_eff = T.prog_bytes + tran_bytes > room
+  ctx->tran_lanes_eff = ctx->warp_bytes + tran_bytes > room
                             ? 0
                             : std::max<uint32_t>(1, std::min<uint32_t>(8, uint32_t((room - T.prog_bytes) / tran_bytes)));
   ctx->warp_ok = true;
@@ -1774,7 +1809,7 @@ int32_t esl_dc_sweep_device(esl_ctx* ctx, const esl_slot* slot, const double* va
   if (int32_t rc = warp_only(ctx)) return rc;
   const TopoDev& T = ctx->topo;
   const size_t lane_bytes = size_t(sweep_doubles(T)) * 8, room = size_t(227) * 1024;
-  if (T.prog_bytes + lane_bytes > room) return ctx->fail(ESL_NOT_ELIGIBLE, "a sweep lane exceeds a CTA's shared memory");
+  if (ctx->warp_bytes + lane_bytes > room) return ctx->fail(ESL_NOT_ELIGIBLE, "a sweep lane exceeds a CTA's shared memory");
   const uint32_t fit = std::max<uint32_t>(1, std::min<uint32_t>(8, uint32_t((room - T.prog_bytes) / lane_bytes)));
   ESL_CUDA(ctx->d_sweep_values.ensure(size_t(n_pts) * 8));
   ESL_CUDA(cudaMemcpyAsync(ctx->d_sweep_values.p, values, size_t(n_pts) * 8, cudaMemcpyHostToDevice, s));
@@ -1848,7 +1883,7 @@ int32_t esl_tran_meas_device(esl_ctx* ctx, const esl_tran_opts* opts, const esl_
   if (int32_t rc = warp_only(ctx)) return rc;
   const TopoDev& T = ctx->topo;
   const size_t lane_bytes = (size_t(T.tran_doubles) + size_t(kMeasDoubles) * n_meas) * 8, room = size_t(227) * 1024;
-  if (T.prog_bytes + lane_bytes > room) return ctx->fail(ESL_NOT_ELIGIBLE, "a transient lane exceeds a CTA's shared memory");
+  if (ctx->warp_bytes + lane_bytes > room) return ctx->fail(ESL_NOT_ELIGIBLE, "a transient lane exceeds a CTA's shared memory");
   const uint32_t fit = std::max<uint32_t>(1, std::min<uint32_t>(8, uint32_t((room - T.prog_bytes) / lane_bytes)));
   cudaStream_t s = ctx->stream;
   ESL_CUDA(ctx->d_meas.ensure(size_t(n_meas) * sizeof(esl_measure)));

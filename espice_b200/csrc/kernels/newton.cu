@@ -200,6 +200,14 @@ __device__ void assemble(const TopoDev& T, uint32_t prog, const LaneMem& m, int 
 }
 
 
+// Program A or B on the warp's lane: its words in the CTA's shared memory, or
+// streamed through the warp's ring when they are too long for it.
+__device__ __forceinline__ bool warp_program(const TopoDev& T, uint32_t prog, bool b, double* v) {
+  const uint32_t chunks = b ? T.b_chunks : T.a_chunks;
+  if (T.tasks) return run_tasks<double, true, true, false>(T.tasks, b ? T.b_first : 0u, chunks, prog + T.o_ring, v) != 0;
+  return run_warp_tasks(prog + (b ? T.o_b_tasks : T.o_a_tasks), chunks, v) != 0;
+}
+
 // Refactor on the frozen tape with the forward solve merged in (program A),
 // and the lane kernel's peel tests (lane_kernels.zig Bodies.refactor and
 // LaneSolver.wideMultipliers): U entries finite, pivots alive, L multipliers
@@ -207,7 +215,7 @@ __device__ void assemble(const TopoDev& T, uint32_t prog, const LaneMem& m, int 
 // Warp-uniform verdict. (As rows of one op a thread the ring's program A was
 // 79 rows and 19.0k cycles, B 51 and 11.8k.)
 __device__ bool refactor_forward(const TopoDev& T, uint32_t prog, double* v, int tid) {
-  bool bad = run_warp_tasks(prog + T.o_a_tasks, T.a_chunks, v) != 0;
+  bool bad = warp_program(T, prog, false, v);
   for (uint32_t s = tid; s < T.nu; s += 32) bad |= !task_finite(v[s]);
   for (uint32_t k = tid; k < T.n; k += 32) {
     const double d = v[T.nu + k];
@@ -217,7 +225,7 @@ __device__ bool refactor_forward(const TopoDev& T, uint32_t prog, double* v, int
 }
 
 __device__ __forceinline__ void back_solve(const TopoDev& T, uint32_t prog, double* v) {
-  run_warp_tasks(prog + T.o_b_tasks, T.b_chunks, v);
+  warp_program(T, prog, true, v);
 }
 
 __device__ __forceinline__ void load_y(const TopoDev& T, const double* rhs, double* y, int tid) {

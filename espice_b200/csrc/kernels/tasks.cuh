@@ -199,7 +199,7 @@ __device__ __forceinline__ void run_task(const TaskLane<kCompact>& c, const Task
 // one's words are on their way into registers and the two after that into
 // the ring. Returns bit 0 set when a division of this thread failed its
 // pivot test.
-template <typename V, bool kShared, bool kCompact>
+template <typename V, bool kShared, bool kCompact, bool kCta = true>
 __device__ __noinline__ uint32_t run_tasks(const uint32_t* words, uint32_t first, uint32_t chunks, uint32_t ring,
                                            V* values) {
   using Lane = TaskLane<kCompact>;
@@ -226,7 +226,7 @@ __device__ __noinline__ uint32_t run_tasks(const uint32_t* words, uint32_t first
     fill = (fill + kBytes) & (kSpan - 1);
     task_wait<kTaskRing - 2>();
     next.load(base + read);
-    run_task<V, kShared, kCompact, true>(c, v, bad);
+    run_task<V, kShared, kCompact, kCta>(c, v, bad);
     c = next;
   }
   task_wait<0>();

@@ -5,7 +5,7 @@ lanes agree bit for bit.
 
 - A lane of a batch large enough for the narrow CTAs equals the same lane of
   a small batch (wide CTAs), FP64 and mixed.
-- FP64 block lanes equal the warp lanes.
+- FP64 block lanes equal the warp lanes (the largest ones' words streamed).
 - A value space past the compact words' 65,536 equals the oracle.
 - Training: a step replayed as a graph equals one launched by itself.
 """
@@ -65,7 +65,8 @@ def test_narrow_ctas_equal_wide(deck, size, precision):
         assert np.array_equal(u[pick], v)
 
 
-@pytest.mark.parametrize("deck,size", [(ladder, 1), (ladder, 28), (ladder, 29), (ladder, 61), (grid, 0), (mesh, 50)])
+@pytest.mark.parametrize("deck,size", [(ladder, 1), (ladder, 28), (ladder, 29), (ladder, 61), (grid, 0), (mesh, 50),
+                                       (mesh, 110), (mesh, 140)])
 def test_block_lanes_equal_warp_lanes(deck, size):
     fr, slots, values = deck(size)
     v = values(17)
