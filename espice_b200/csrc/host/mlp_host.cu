@@ -33,17 +33,18 @@ struct Dev {
   ~Dev() {
     if (p) cudaFree(p);
   }
-  cudaError_t ensure(size_t count) {
+  // At least `count` elements, zeroed when new. The fill is ordered on `s`, the
+  // stream that uses the buffer: one on the default stream would wait there
+  // for whatever is queued and could land on what `s` has written since.
+  cudaError_t ensure(size_t count, cudaStream_t s) {
     if (count <= n) return cudaSuccess;
     if (p) cudaFree(p);
     p = nullptr;
     n = 0;
     cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-    if (e == cudaSuccess) {
-      n = count;
-      cudaMemset(p, 0, count * sizeof(T));
-    }
-    return e;
+    if (e != cudaSuccess) return e;
+    n = count;
+    return cudaMemsetAsync(p, 0, count * sizeof(T), s);
   }
 };
 
@@ -129,21 +130,21 @@ int32_t ensure_batch(esl_mlp* m, int rows) {
   for (size_t l = 0; l < L; ++l) {
     auto h = std::make_unique<Dev<__nv_bfloat16>>();
     auto ht = std::make_unique<Dev<__nv_bfloat16>>();
-    MLP_CUDA(h->ensure(size_t(rows) * m->layers[l]->k));
-    MLP_CUDA(ht->ensure(size_t(rows) * m->layers[l]->k));
+    MLP_CUDA(h->ensure(size_t(rows) * m->layers[l]->k, m->stream));
+    MLP_CUDA(ht->ensure(size_t(rows) * m->layers[l]->k, m->stream));
     m->hb.push_back(std::move(h));
     m->ht.push_back(std::move(ht));
     auto zz = std::make_unique<Dev<float>>();
-    MLP_CUDA(zz->ensure(size_t(rows) * m->layers[l]->n));
+    MLP_CUDA(zz->ensure(size_t(rows) * m->layers[l]->n, m->stream));
     m->z.push_back(std::move(zz));
   }
   int wmax = 0;
   for (auto& l : m->layers) wmax = std::max({wmax, l->k, l->n});
-  MLP_CUDA(m->dz.ensure(size_t(rows) * wmax));
-  MLP_CUDA(m->dh.ensure(size_t(rows) * wmax));
-  MLP_CUDA(m->dzb.ensure(size_t(rows) * wmax));
-  MLP_CUDA(m->dzt.ensure(size_t(rows) * wmax));
-  MLP_CUDA(m->t.ensure(size_t(rows) * m->n_out));
+  MLP_CUDA(m->dz.ensure(size_t(rows) * wmax, m->stream));
+  MLP_CUDA(m->dh.ensure(size_t(rows) * wmax, m->stream));
+  MLP_CUDA(m->dzb.ensure(size_t(rows) * wmax, m->stream));
+  MLP_CUDA(m->dzt.ensure(size_t(rows) * wmax, m->stream));
+  MLP_CUDA(m->t.ensure(size_t(rows) * m->n_out, m->stream));
   m->rows = rows;
   return ESL_MLP_OK;
 }
@@ -251,9 +252,7 @@ int32_t esl_mlp_create(int n_in, int n_hidden, int n_layers, int n_out, int devi
     }
   };
   place(false);
-  if (m->arena.ensure(bytes) != cudaSuccess) return ESL_MLP_OUT_OF_MEMORY;
-  // the fill runs on the default stream, which the network's does not wait for
-  if (cudaStreamSynchronize(nullptr) != cudaSuccess) return ESL_MLP_DEVICE_FAULT;
+  if (m->arena.ensure(bytes, m->stream) != cudaSuccess) return ESL_MLP_OUT_OF_MEMORY;
   place(true);
   for (size_t l = 0; l < m->layers.size(); ++l) {
     Layer& ly = *m->layers[l];
@@ -267,7 +266,7 @@ int32_t esl_mlp_create(int n_in, int n_hidden, int n_layers, int n_out, int devi
   m->in_sig.assign(n_in, 1.0f);
   m->out_mu.assign(n_out, 0.0f);
   m->out_sig.assign(n_out, 1.0f);
-  if (m->gerr.ensure(1) != cudaSuccess) return ESL_MLP_OUT_OF_MEMORY;
+  if (m->gerr.ensure(1, m->stream) != cudaSuccess) return ESL_MLP_OUT_OF_MEMORY;
   if (int32_t rc = esl_mlp_set_scaling(m.get(), nullptr, nullptr, nullptr, nullptr)) return rc;
   *out = m.release();
   return ESL_MLP_OK;
@@ -296,14 +295,17 @@ int32_t esl_mlp_set_scaling(esl_mlp* m, const float* in_mu, const float* in_sig,
     if (!(v > 0)) return m->fail(ESL_MLP_INVALID_ARGUMENT, "input scales must be positive");
   for (float v : m->out_sig)
     if (!(v > 0)) return m->fail(ESL_MLP_INVALID_ARGUMENT, "output scales must be positive");
-  MLP_CUDA(m->d_in_mu.ensure(m->n_in));
-  MLP_CUDA(m->d_in_sig.ensure(m->n_in));
-  MLP_CUDA(m->d_out_mu.ensure(m->n_out));
-  MLP_CUDA(m->d_out_sig.ensure(m->n_out));
-  MLP_CUDA(cudaMemcpy(m->d_in_mu.p, m->in_mu.data(), m->n_in * 4, cudaMemcpyHostToDevice));
-  MLP_CUDA(cudaMemcpy(m->d_in_sig.p, m->in_sig.data(), m->n_in * 4, cudaMemcpyHostToDevice));
-  MLP_CUDA(cudaMemcpy(m->d_out_mu.p, m->out_mu.data(), m->n_out * 4, cudaMemcpyHostToDevice));
-  MLP_CUDA(cudaMemcpy(m->d_out_sig.p, m->out_sig.data(), m->n_out * 4, cudaMemcpyHostToDevice));
+  MLP_CUDA(m->d_in_mu.ensure(m->n_in, m->stream));
+  MLP_CUDA(m->d_in_sig.ensure(m->n_in, m->stream));
+  MLP_CUDA(m->d_out_mu.ensure(m->n_out, m->stream));
+  MLP_CUDA(m->d_out_sig.ensure(m->n_out, m->stream));
+  MLP_CUDA(cudaMemcpyAsync(m->d_in_mu.p, m->in_mu.data(), m->n_in * 4, cudaMemcpyHostToDevice, m->stream));
+  MLP_CUDA(cudaMemcpyAsync(m->d_in_sig.p, m->in_sig.data(), m->n_in * 4, cudaMemcpyHostToDevice, m->stream));
+  MLP_CUDA(cudaMemcpyAsync(m->d_out_mu.p, m->out_mu.data(), m->n_out * 4, cudaMemcpyHostToDevice, m->stream));
+  MLP_CUDA(cudaMemcpyAsync(m->d_out_sig.p, m->out_sig.data(), m->n_out * 4, cudaMemcpyHostToDevice, m->stream));
+  // what the caller has queued on the default stream is done when this
+  // returns, as after a blocking copy
+  MLP_CUDA(cudaStreamSynchronize(nullptr));
   return ESL_MLP_OK;
 }
 
@@ -374,7 +376,7 @@ int32_t esl_mlp_train(esl_mlp* m, const float* d_x, const float* d_y, uint32_t n
   cudaSetDevice(m->device);
   const int B = int(batch);
   if (int32_t rc = ensure_batch(m, B)) return rc;
-  MLP_CUDA(m->loss.ensure(1));
+  MLP_CUDA(m->loss.ensure(1, m->stream));
   cudaStream_t s = m->stream;
   MLP_CUDA(cudaMemsetAsync(m->gerr.p, 0, 4, s));
   std::mt19937_64 rng(seed);
@@ -383,9 +385,9 @@ int32_t esl_mlp_train(esl_mlp* m, const float* d_x, const float* d_y, uint32_t n
   const uint32_t n_batches = n / batch;
   if (n_batches == 0) return m->fail(ESL_MLP_INVALID_ARGUMENT, "fewer samples than one batch");
   if (epochs == 0) return check_gemm_err(m);
-  MLP_CUDA(m->perm.ensure(n));
-  MLP_CUDA(m->at.ensure(1));
-  MLP_CUDA(m->rates.ensure(n_batches));
+  MLP_CUDA(m->perm.ensure(n, m->stream));
+  MLP_CUDA(m->at.ensure(1, m->stream));
+  MLP_CUDA(m->rates.ensure(n_batches, m->stream));
   // beta^t of the steps so far
   float p1 = 1.0f, p2 = 1.0f;
   for (int i = 0; i < m->step; ++i) {
@@ -461,7 +463,7 @@ int32_t esl_mlp_gradients(esl_mlp* m, const float* d_x, const float* d_y, uint32
   cudaSetDevice(m->device);
   const int B = int(n);
   if (int32_t rc = ensure_batch(m, B)) return rc;
-  MLP_CUDA(m->loss.ensure(1));
+  MLP_CUDA(m->loss.ensure(1, m->stream));
   cudaStream_t s = m->stream;
   MLP_CUDA(cudaMemsetAsync(m->gerr.p, 0, 4, s));
   MLP_CUDA(cudaMemsetAsync(m->loss.p, 0, 4, s));

@@ -116,6 +116,32 @@ def test_training_fits_a_smooth_map():
     net.close()
 
 
+@pytest.mark.parametrize("passes", [4, 12, 24, 48])
+def test_training_beside_work_on_the_default_stream(passes):
+    """A run's new buffers are made ready on the network's own stream: work
+    queued on the default stream (about a third of a millisecond a pass; it
+    ends before, within and after the 64 steps) changes no weight."""
+    torch = _torch()
+    big = torch.ones(1 << 28, device="cuda")
+    g = torch.Generator().manual_seed(2)
+    x = torch.randn(16384, 16, generator=g).cuda()
+    y = torch.randn(16384, 64, generator=g).cuda()
+
+    def run(queued):
+        net = mlp.Mlp(16, 64, 3, 64, seed=3)
+        torch.cuda.synchronize()
+        for _ in range(queued):
+            big.mul_(1.0)
+        loss = net.train(x.data_ptr(), y.data_ptr(), len(x), epochs=1, batch=256, lr=1e-3)
+        torch.cuda.synchronize()
+        weights = np.concatenate([a.ravel() for layer in net.weights() for a in layer])
+        net.close()
+        return loss, weights
+
+    (la, wa), (lb, wb) = run(passes), run(0)
+    assert np.array_equal(la, lb) and np.array_equal(wa.view(np.uint32), wb.view(np.uint32))
+
+
 def test_gemm_wait_runs_out_and_stores_nothing():
     torch = _torch()
     M, N, K = 256, 128, 192
