@@ -327,42 +327,55 @@ __global__ void mse_grad(const float* y, const float* t, int rows, int outs, int
 // an atomic an element, 127,488 of them on one address, a batch's loss took
 // 270 us, three times the rest of its training step; summed in blocks it
 // would lose the accumulator's rounding, 1% of an epoch's loss.)
+// A chunk whose terms lie far above the accumulator (its first ones, above
+// zero, among them) takes u from its largest term, beside which the others
+// round as they would behind it; an infinite term or a NaN goes into the sum
+// as it is.
 constexpr int kLossThreads = 1024;
 __global__ void __launch_bounds__(kLossThreads) mse_loss(const float* y, const float* t, int rows, int outs, int ld,
                                                          float* loss) {
   __shared__ long long part[kLossThreads / 32];
+  __shared__ uint32_t tops[kLossThreads / 32];
   __shared__ float acc;
   const int n = rows * outs, tid = threadIdx.x;
   const float count = float(n);
   if (tid == 0) acc = *loss;
   __syncthreads();
+  // u = 2^(exponent - 23), at least 2^-126
+  auto unit = [](float a) { return __int_as_float(max(1, int((__float_as_uint(a) >> 23) & 255u) - 23) << 23); };
   for (int i0 = 0; i0 < n; i0 += kLossThreads) {
     const int i = i0 + tid;
     float e = 0.0f;
     if (i < n) e = y[size_t(i / outs) * ld + i % outs] - t[i];
     const float x = e * e / count;
-    float a = acc;
-    if (a == 0.0f) {
-      // the first terms: from the largest one's scale
-      float top = x;
-      for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-      if ((tid & 31) == 0) part[tid >> 5] = __float_as_int(top);
+    const float a = acc;
+    float u = unit(a);
+    // 2^52: 1,024 terms below it sum in 64 bits
+    const bool far = a == 0.0f || !(a < INFINITY) || !(x / u < 0x1p52f);
+    if (__syncthreads_or(far)) {
+      // by their bits terms order as numbers, infinity and then NaN on top
+      const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(x) & 0x7fffffffu);
+      if ((tid & 31) == 0) tops[tid >> 5] = top;
       __syncthreads();
-      for (int w = 0; w < kLossThreads / 32; ++w) a = fmaxf(a, __int_as_float(int(part[w])));
-      __syncthreads();
+      uint32_t m = 0;
+      for (int w = 0; w < kLossThreads / 32; ++w) m = max(m, tops[w]);
+      const float most = __uint_as_float(m);
+      if (!(a < INFINITY) || !(most < INFINITY)) {
+        __syncthreads();  // every thread has read acc and tops
+        if (tid == 0) acc = a + most;
+        __syncthreads();
+        continue;
+      }
+      u = unit(fmaxf(a, most));
     }
-    // u = 2^(exponent - 23), at least 2^-126; a NaN or infinity passes through
-    const int ex = max(1, int((__float_as_uint(a) >> 23) & 255u) - 23);
-    const float u = __int_as_float(ex << 23);
-    const bool wild = !(a < INFINITY) || !(x / u < 4.0e15f);
     long long k = __float2ll_rn(x / u);
     for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
     if ((tid & 31) == 0) part[tid >> 5] = k;
-    const bool any_wild = __syncthreads_or(wild);
+    __syncthreads();
     if (tid == 0) {
       long long s = 0;
       for (int w = 0; w < kLossThreads / 32; ++w) s += part[w];
-      acc = any_wild ? NAN : float(double(acc) + double(s) * double(u));
+      acc = float(double(a) + double(s) * double(u));
     }
     __syncthreads();
   }

@@ -116,6 +116,48 @@ def test_training_fits_a_smooth_map():
     net.close()
 
 
+@pytest.mark.parametrize("errors,want", [
+    ([(0, 2064, 1e-6), (1500, 1501, 1.0)], None),         # far above the sum before its chunk
+    ([(1024, 2064, 1e-9), (2050, 2064, 1e3)], None),      # a first chunk without error, then a rise
+    ([(0, 2064, 1e-18), (2000, 2001, 1e18)], None),       # near the ends of the range
+    ([(0, 1, 1e3), (1, 2064, 1e-3)], None),
+    ([(0, 2064, 0.25)], None),
+    ([], None),
+    ([(0, 2064, 0.25), (3, 4, np.inf)], np.inf),
+    ([(2063, 2064, np.inf)], np.inf),
+    ([(0, 2064, 0.25), (1100, 1101, 1e25)], np.inf),      # its square past FP32
+    ([(0, 2064, 0.25), (7, 8, np.inf), (1999, 2000, np.nan)], np.nan),
+    ([(0, 2064, 0.25), (5, 6, np.nan)], np.nan),
+])
+def test_loss_of_uneven_errors(errors, want):
+    """The loss against its FP32 terms summed in FP64, where they are finite:
+    2,064 roundings to nearest of a sum of one sign, 2^-24 of it each; an
+    infinite term gives infinity, a NaN gives NaN."""
+    torch = _torch()
+    rows, n_out = 16, 129
+    net = mlp.Mlp(4, 16, 2, n_out, seed=9)
+    x = torch.linspace(-1.0, 1.0, rows * 4, device="cuda").reshape(rows, 4).contiguous()
+    y = torch.zeros(rows, n_out, device="cuda")
+    torch.cuda.synchronize()
+    net.predict(x.data_ptr(), rows, y.data_ptr())
+    t = y.cpu().numpy().ravel().copy()
+    out = t.copy()
+    for lo, hi, e in errors:
+        t[lo:hi] += np.float32(e)
+    dt = torch.tensor(t, device="cuda")
+    torch.cuda.synchronize()
+    loss, _ = net.gradients(x.data_ptr(), dt.data_ptr(), rows)
+    net.close()
+    with np.errstate(over="ignore", invalid="ignore"):
+        e = out - t
+        terms = e * e / np.float32(rows * n_out)
+    if want is None:
+        ref = float(np.sum(terms.astype(np.float64)))
+        assert abs(loss - ref) <= rows * n_out * 2.0 ** -24 * ref
+    else:
+        assert np.array_equal(np.float32(loss), np.float32(want), equal_nan=True)
+
+
 @pytest.mark.parametrize("passes", [4, 12, 24, 48])
 def test_training_beside_work_on_the_default_stream(passes):
     """A run's new buffers are made ready on the network's own stream: work
