@@ -721,6 +721,26 @@ std::string compiled_lu_source(uint32_t nnz, const SparseLu& lu, const Programs&
   return lu_jit_source(in);
 }
 
+// Warp lanes of lane_bytes a CTA holds beside the staged programs, each with
+// its ring when the task words stream (and one lane even without).
+uint32_t warp_fit(const esl_ctx* ctx, size_t lane_bytes) {
+  const size_t room = size_t(227) * 1024, ring = ctx->topo.tasks ? task_ring_bytes(1, true) : 0;
+  const size_t beside = room - std::min<size_t>(room, ctx->topo.prog_bytes);
+  return uint32_t(std::clamp<size_t>(beside / (lane_bytes + ring), 1, 8));
+}
+
+// The topology as a launch of `lanes` such lanes a CTA sees it: streamed task
+// words come through rings behind the staged programs, unless a single lane
+// leaves no room for its own.
+TopoDev warp_view(const esl_ctx* ctx, size_t lane_bytes, uint32_t lanes) {
+  TopoDev T = ctx->topo;
+  const uint32_t ring = task_ring_bytes(lanes, true);
+  if (T.tasks && T.prog_bytes + ring + lanes * lane_bytes <= size_t(227) * 1024) T.ring_bytes = ring;
+  return T;
+}
+
+size_t dc_lane_bytes(const esl_ctx* ctx) { return size_t(ctx->topo.smem_doubles) * 8; }
+
 // The lead lane's pivot tape, compiled and uploaded.
 int32_t upload_tape(esl_ctx* ctx) {
   cudaStream_t s = ctx->stream;
@@ -788,7 +808,7 @@ int32_t upload_tape(esl_ctx* ctx) {
     // The tasks' words (a stream's first chunk beyond its last is read ahead)
     // beside the gathers when that leaves room for the largest lane there is,
     // a transient one with every measure card; else in global memory, with a
-    // ring of 2 KB a warp.
+    // ring in the CTA for each lane that leaves room for one (warp_view).
     const size_t nt = lane_layout(T.n, T.ntv, T.n_stage, T.nlim).total + 9 * size_t(T.n) + 5 * size_t(T.n_qt) +
                       9 * size_t(T.n_src) + 2 + kMeasDoubles * kMaxMeas;
     if (blob.size() + size_t(T.a_chunks + T.b_chunks + 2) * chunk + nt * 8 <= size_t(227) * 1024) {
@@ -796,8 +816,6 @@ int32_t upload_tape(esl_ctx* ctx) {
       T.o_b_tasks = put(B.words.data(), (T.b_chunks + 1) * chunk);
     } else {
       T.b_first = A.off[1];
-      T.o_ring = uint32_t(blob.size());
-      blob.resize(blob.size() + task_ring_bytes(8, true), 0);
       A.words.insert(A.words.end(), B.words.begin(), B.words.end());
       ESL_CUDA(upload(ctx->d_tasks, A.words, s));
       T.tasks = ctx->d_tasks.as<uint32_t>();
@@ -807,6 +825,7 @@ int32_t upload_tape(esl_ctx* ctx) {
     ESL_CUDA(upload(ctx->d_prog, blob, s));
     T.prog = ctx->d_prog.as<unsigned char>();
     T.prog_bytes = uint32_t(blob.size());
+    T.ring_bytes = 0;
     T.g_nseg = G.nseg;
     T.g_seg_blocks = G.seg_len / kGatherBlock;
   }
@@ -815,8 +834,10 @@ int32_t upload_tape(esl_ctx* ctx) {
   const size_t lane_bytes = size_t(T.smem_doubles) * 8;
   const size_t room = size_t(227) * 1024;
   // Which circuits are warp lanes is decided on the programs as rows of 32
-  // single ops beside the gathers (the tasks need no more room than that), so
-  // that a call's route does not hang on how they are packed. The rows are
+  // single ops beside the gathers, so that a call's route does not hang on
+  // how they are packed. (The words of a small tape's tasks can take more room
+  // than its rows; they lie in shared memory only where every lane has room
+  // beside them, and a lane beside the gathers alone needs no ring.) The rows are
   // packed only when their bounds leave it open: a full row takes 32 ops, and
   // of two rows that are not full the longest path to the end gets shorter.
   const size_t least = (P.a_nops + 31) / 32 + (P.b_nops + 31) / 32;
@@ -830,7 +851,7 @@ int32_t upload_tape(esl_ctx* ctx) {
     ctx->warp_bytes += uint32_t((P.a_ops.size() + P.b_ops.size()) * sizeof(Op));
     if (ctx->warp_bytes + lane_bytes > room) return ESL_OK;
   }
-  ctx->lanes_eff = std::max<uint32_t>(1, std::min<uint32_t>(8, uint32_t((room - T.prog_bytes) / lane_bytes)));
+  ctx->lanes_eff = warp_fit(ctx, lane_bytes);
   // Transient lanes add the accepted points, the charge rings and dynamic
   // currents over the rows and the LTE states: cur | prev | q[4] | ip over
   // n, then q[4] | ip over n_qt, then the V and I sources' values at the
@@ -838,9 +859,7 @@ int32_t upload_tape(esl_ctx* ctx) {
   // per source).
   T.tran_doubles = (T.smem_doubles + 7 * T.n + 5 * T.n_qt + 9 * T.n_src + 1) & ~1u;
   const size_t tran_bytes = size_t(T.tran_doubles) * 8;
-  ctx->tran_lanes_eff = ctx->warp_bytes + tran_bytes > room
-                            ? 0
-                            : std::max<uint32_t>(1, std::min<uint32_t>(8, uint32_t((room - T.prog_bytes) / tran_bytes)));
+  ctx->tran_lanes_eff = ctx->warp_bytes + tran_bytes > room ? 0 : warp_fit(ctx, tran_bytes);
   ctx->warp_ok = true;
   return ESL_OK;
 }
@@ -1134,6 +1153,12 @@ uint32_t lanes_per_cta(const esl_ctx* ctx, uint32_t n_lanes, uint32_t fit) {
   uint32_t want = ctx->lanes_per_block;
   if (want == 0) want = (n_lanes + uint32_t(ctx->sms) - 1) / uint32_t(ctx->sms);
   return std::max<uint32_t>(1, std::min<uint32_t>(want, fit));
+}
+
+// The warp lanes' DC launch over the context's lanes.
+cudaError_t launch_warp_dc(const esl_ctx* ctx, const LaneDev& L, const LaneOpts& o, cudaStream_t s) {
+  const uint32_t lanes = lanes_per_cta(ctx, ctx->n_lanes, ctx->lanes_eff);
+  return launch_dc_newton(warp_view(ctx, dc_lane_bytes(ctx), lanes), L, o, lanes, s);
 }
 
 LaneDev lane_view(esl_ctx* ctx, uint32_t resume) {
@@ -1454,7 +1479,7 @@ int32_t dc_solve(esl_ctx* ctx, const esl_newton_opts* opts, double* d_x, int col
   const bool b3 = topo_has_b3(ctx->topo);
   auto launch = [&](const LaneDev& LL) {
     return block ? launch_dc_block(D, LL, o, mixed, b3, s)
-                 : launch_dc_newton(ctx->topo, LL, o, lanes_per_cta(ctx, N, ctx->lanes_eff), s);
+                 : launch_warp_dc(ctx, LL, o, s);
   };
   ESL_CUDA(cudaEventRecord(ctx->ev0, s));
   ESL_CUDA(launch(L));
@@ -1594,7 +1619,7 @@ int32_t esl_dc_solve_device_static(esl_ctx* ctx, const esl_newton_opts* opts, do
   cudaStream_t s = ctx->stream;
   if (cudaError_t e = launch_lane_init(ctx->topo, L, cold != 0, opts->init_fix != 0, s))
     return cuda(e, "lane_init_kernel");
-  if (cudaError_t e = launch_dc_newton(ctx->topo, L, o, lanes_per_cta(ctx, N, ctx->lanes_eff), s)) return cuda(e, "dc_newton_kernel");
+  if (cudaError_t e = launch_warp_dc(ctx, L, o, s)) return cuda(e, "dc_newton_kernel");
   uint32_t paused = 0;
   if (cudaError_t e = cudaMemcpyAsync(&paused, L.n_paused, 4, cudaMemcpyDeviceToHost, s))
     return cuda(e, "read paused-lane count");
@@ -1728,8 +1753,9 @@ int32_t run_tran(esl_ctx* ctx, LaneDev L, TranDev P, const LaneOpts& lo, uint32_
   std::memset(&ctx->last_peels, 0, sizeof(ctx->last_peels));
   ESL_CUDA(ctx->d_next_lane.ensure(sizeof(uint32_t)));
   P.next_lane = ctx->d_next_lane.as<uint32_t>();
+  const TopoDev T = warp_view(ctx, (size_t(ctx->topo.tran_doubles) + size_t(kMeasDoubles) * P.n_meas) * 8, lpb);
   ESL_CUDA(cudaEventRecord(ctx->ev0, s));
-  ESL_CUDA(launch_tran(ctx->topo, L, P, lo, lpb, s));
+  ESL_CUDA(launch_tran(T, L, P, lo, lpb, s));
   ctx->last_peels.launches = 1;
   for (;;) {
     bool any = false;
@@ -1737,7 +1763,7 @@ int32_t run_tran(esl_ctx* ctx, LaneDev L, TranDev P, const LaneOpts& lo, uint32_
     if (!any) break;
     LaneDev R = L;
     R.resume = 1;
-    ESL_CUDA(launch_tran(ctx->topo, R, P, lo, lpb, s));
+    ESL_CUDA(launch_tran(T, R, P, lo, lpb, s));
     ++ctx->last_peels.launches;
   }
   ESL_CUDA(cudaEventRecord(ctx->ev1, s));
@@ -1810,7 +1836,7 @@ int32_t esl_dc_sweep_device(esl_ctx* ctx, const esl_slot* slot, const double* va
   const TopoDev& T = ctx->topo;
   const size_t lane_bytes = size_t(sweep_doubles(T)) * 8, room = size_t(227) * 1024;
   if (ctx->warp_bytes + lane_bytes > room) return ctx->fail(ESL_NOT_ELIGIBLE, "a sweep lane exceeds a CTA's shared memory");
-  const uint32_t fit = std::max<uint32_t>(1, std::min<uint32_t>(8, uint32_t((room - T.prog_bytes) / lane_bytes)));
+  const uint32_t fit = warp_fit(ctx, lane_bytes);
   ESL_CUDA(ctx->d_sweep_values.ensure(size_t(n_pts) * 8));
   ESL_CUDA(cudaMemcpyAsync(ctx->d_sweep_values.p, values, size_t(n_pts) * 8, cudaMemcpyHostToDevice, s));
   SweepDev P{};
@@ -1844,7 +1870,8 @@ int32_t esl_dc_sweep_device(esl_ctx* ctx, const esl_slot* slot, const double* va
   const uint32_t lpb = lanes_per_cta(ctx, N, fit);
   ESL_CUDA(cudaEventRecord(ctx->ev0, s));
   std::memset(&ctx->last_peels, 0, sizeof(ctx->last_peels));
-  ESL_CUDA(launch_sweep(T, L, P, o, lpb, s));
+  const TopoDev V = warp_view(ctx, lane_bytes, lpb);
+  ESL_CUDA(launch_sweep(V, L, P, o, lpb, s));
   ctx->last_peels.launches = 1;
   for (;;) {
     bool any = false;
@@ -1852,7 +1879,7 @@ int32_t esl_dc_sweep_device(esl_ctx* ctx, const esl_slot* slot, const double* va
     if (!any) break;
     LaneDev R = L;
     R.resume = 1;
-    ESL_CUDA(launch_sweep(T, R, P, o, lpb, s));
+    ESL_CUDA(launch_sweep(V, R, P, o, lpb, s));
     ++ctx->last_peels.launches;
   }
   ESL_CUDA(cudaEventRecord(ctx->ev1, s));
@@ -1884,7 +1911,7 @@ int32_t esl_tran_meas_device(esl_ctx* ctx, const esl_tran_opts* opts, const esl_
   const TopoDev& T = ctx->topo;
   const size_t lane_bytes = (size_t(T.tran_doubles) + size_t(kMeasDoubles) * n_meas) * 8, room = size_t(227) * 1024;
   if (ctx->warp_bytes + lane_bytes > room) return ctx->fail(ESL_NOT_ELIGIBLE, "a transient lane exceeds a CTA's shared memory");
-  const uint32_t fit = std::max<uint32_t>(1, std::min<uint32_t>(8, uint32_t((room - T.prog_bytes) / lane_bytes)));
+  const uint32_t fit = warp_fit(ctx, lane_bytes);
   cudaStream_t s = ctx->stream;
   ESL_CUDA(ctx->d_meas.ensure(size_t(n_meas) * sizeof(esl_measure)));
   ESL_CUDA(cudaMemcpyAsync(ctx->d_meas.p, meas, size_t(n_meas) * sizeof(esl_measure), cudaMemcpyHostToDevice, s));
@@ -2071,10 +2098,10 @@ int32_t esl_group_dc_solve_device(esl_ctx* const* ctxs, uint32_t n_ctx, const es
   for (uint32_t c = 0; c < n_ctx; ++c) {
     esl_ctx* x = ctxs[c];
     if (int32_t rc = warp_only(x)) return rc;
-    topos[c] = x->topo;
     lpb[c] = lanes_per_cta(x, x->n_lanes, x->lanes_eff);
+    topos[c] = warp_view(x, dc_lane_bytes(x), lpb[c]);
     max_lpb = std::max(max_lpb, lpb[c]);
-    smem = std::max(smem, size_t(x->topo.prog_bytes) + size_t(lpb[c]) * x->topo.smem_doubles * 8);
+    smem = std::max(smem, size_t(topos[c].prog_bytes) + topos[c].ring_bytes + size_t(lpb[c]) * dc_lane_bytes(x));
     for (uint32_t f = 0; f < x->n_lanes; f += lpb[c]) {
       cta_ctx.push_back(c);
       cta_first.push_back(f);
@@ -2109,7 +2136,7 @@ int32_t esl_group_dc_solve_device(esl_ctx* const* ctxs, uint32_t n_ctx, const es
       if (!any) break;
       LaneDev R = lanes[c];
       R.resume = 1;
-      ESL_CUDA(launch_dc_newton(x->topo, R, o, lanes_per_cta(x, x->n_lanes, x->lanes_eff), x->stream));
+      ESL_CUDA(launch_warp_dc(x, R, o, x->stream));
       ++launches;
     }
     ESL_CUDA(cudaStreamSynchronize(x->stream));
@@ -2487,7 +2514,9 @@ int32_t esl_lu_replay_device(esl_ctx* ctx, const double* lead, uint32_t n_lanes,
   }
   if (int32_t rc = warp_only(ctx)) return rc;
   ESL_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
-  ESL_CUDA(launch_lu_replay(ctx->topo, n_lanes, d_a, d_rhs, d_tv, d_dx, d_bad, lanes_per_cta(ctx, n_lanes, ctx->lanes_eff), ctx->stream));
+  const uint32_t per_cta = lanes_per_cta(ctx, n_lanes, ctx->lanes_eff);
+  ESL_CUDA(launch_lu_replay(warp_view(ctx, dc_lane_bytes(ctx), per_cta), n_lanes, d_a, d_rhs, d_tv, d_dx, d_bad, per_cta,
+                            ctx->stream));
   ESL_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
   ESL_CUDA(cudaEventSynchronize(ctx->ev1));
   if (ms) cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1);

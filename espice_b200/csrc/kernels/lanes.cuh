@@ -62,9 +62,10 @@ struct TopoDev {
   uint32_t o_a_tasks, o_b_tasks, o_g_src, o_g_dst;
   uint32_t a_chunks, b_chunks, g_nseg, g_seg_blocks;
   // Tasks too long for the blob: their words in global memory (A's, then
-  // B's from b_first chunks on), each warp's ring at o_ring of the blob.
+  // B's from b_first chunks on), and the rings of a CTA's warps (a launch's
+  // own number of them, or none), between the blob and the lanes.
   const uint32_t* tasks;
-  uint32_t b_first, o_ring;
+  uint32_t b_first, ring_bytes;
   uint32_t o_k_depth, o_k_off, o_k_src, o_k_dst;
   uint32_t n_kr_groups, n_ks_groups;
   // L tape values whose column passed on the row-scaled test (no wide test).

@@ -81,13 +81,13 @@ __device__ __forceinline__ double warp_fmax(double v) {
 
 
 // Copies the program blob into the CTA's shared memory (every thread takes
-// part) and returns the lanes' area that follows it.
+// part) and returns the lanes' area that follows it and the rings.
 __device__ __forceinline__ double* stage_programs(const TopoDev& T, unsigned char* smem) {
   const uint4* src = reinterpret_cast<const uint4*>(T.prog);
   uint4* dst = reinterpret_cast<uint4*>(smem);
   for (uint32_t i = threadIdx.x; i < T.prog_bytes / 16; i += blockDim.x) dst[i] = src[i];
   __syncthreads();
-  return reinterpret_cast<double*>(smem + T.prog_bytes);
+  return reinterpret_cast<double*>(smem + T.prog_bytes + T.ring_bytes);
 }
 
 
@@ -201,10 +201,15 @@ __device__ void assemble(const TopoDev& T, uint32_t prog, const LaneMem& m, int 
 
 
 // Program A or B on the warp's lane: its words in the CTA's shared memory, or
-// streamed through the warp's ring when they are too long for it.
+// streamed through the warp's ring when they are too long for it, or read
+// where they lie when the lane leaves no room for a ring.
 __device__ __forceinline__ bool warp_program(const TopoDev& T, uint32_t prog, bool b, double* v) {
   const uint32_t chunks = b ? T.b_chunks : T.a_chunks;
-  if (T.tasks) return run_tasks<double, true, true, false>(T.tasks, b ? T.b_first : 0u, chunks, prog + T.o_ring, v) != 0;
+  if (T.tasks) {
+    const uint32_t first = b ? T.b_first : 0u;
+    if (T.ring_bytes) return run_tasks<double, true, true, false>(T.tasks, first, chunks, prog + T.prog_bytes, v) != 0;
+    return run_far_tasks(T.tasks, first, chunks, v) != 0;
+  }
   return run_warp_tasks(prog + (b ? T.o_b_tasks : T.o_a_tasks), chunks, v) != 0;
 }
 
@@ -537,7 +542,7 @@ bool topo_has_b3(const TopoDev& T) {
 template <bool kHasB3>
 static cudaError_t launch_dc_newton_t(const TopoDev& T, const LaneDev& L, const LaneOpts& o, uint32_t lanes_per_block,
                                       cudaStream_t s) {
-  const size_t smem = T.prog_bytes + lanes_per_block * lane_smem_bytes(T);
+  const size_t smem = T.prog_bytes + T.ring_bytes + lanes_per_block * lane_smem_bytes(T);
   auto* k = o.ladder ? dc_newton_kernel<kHasB3, true> : dc_newton_kernel<kHasB3, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
@@ -565,7 +570,7 @@ cudaError_t launch_assemble(const TopoDev& T, const LaneDev& L, uint32_t lane, d
 cudaError_t launch_lu_replay(const TopoDev& T, uint32_t n_lanes, const double* a, const double* rhs, double* tv,
                              double* dx, uint8_t* bad, uint32_t lanes_per_block, cudaStream_t s) {
   const size_t per = size_t(T.nv + T.n + 1) * sizeof(double);
-  const size_t smem = T.prog_bytes + lanes_per_block * per;
+  const size_t smem = T.prog_bytes + T.ring_bytes + lanes_per_block * per;
   cudaError_t e = cudaFuncSetAttribute(lu_replay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
   lu_replay_kernel<<<persistent_grid(lu_replay_kernel, n_lanes, lanes_per_block, smem), 32 * lanes_per_block, smem,
@@ -2189,7 +2194,7 @@ __global__ void __launch_bounds__(256) sweep_kernel(TopoDev T, LaneDev L, SweepD
 
 cudaError_t launch_sweep(const TopoDev& T, const LaneDev& L, const SweepDev& P, const LaneOpts& o,
                          uint32_t lanes_per_block, cudaStream_t s) {
-  const size_t smem = T.prog_bytes + lanes_per_block * size_t(sweep_doubles(T)) * sizeof(double);
+  const size_t smem = T.prog_bytes + T.ring_bytes + lanes_per_block * size_t(sweep_doubles(T)) * sizeof(double);
   auto* k = topo_has_b3(T) ? sweep_kernel<true> : sweep_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;
@@ -2202,7 +2207,7 @@ cudaError_t launch_sweep(const TopoDev& T, const LaneDev& L, const SweepDev& P, 
 cudaError_t launch_tran(const TopoDev& T, const LaneDev& L, const TranDev& P, const LaneOpts& o,
                         uint32_t lanes_per_block, cudaStream_t s) {
   const size_t smem =
-      T.prog_bytes + lanes_per_block * size_t(T.tran_doubles + kMeasDoubles * P.n_meas) * sizeof(double);
+      T.prog_bytes + T.ring_bytes + lanes_per_block * size_t(T.tran_doubles + kMeasDoubles * P.n_meas) * sizeof(double);
   auto* k = topo_has_b3(T) ? tran_kernel<true> : tran_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return e;

@@ -249,6 +249,23 @@ __device__ __noinline__ uint32_t run_warp_tasks(uint32_t words, uint32_t chunks,
   return bad & 1u;
 }
 
+// The same with the words in global memory and no ring: a warp whose lane
+// takes all of its CTA's shared memory.
+__device__ __noinline__ uint32_t run_far_tasks(const uint32_t* words, uint32_t first, uint32_t chunks, double* values) {
+  const uint4* s = reinterpret_cast<const uint4*>(words) + size_t(first) * 32 + (threadIdx.x & 31);
+  const TaskMem<double, true> v(values);
+  uint32_t bad = 0;
+  TaskLane<true> c, next;
+  c.c = __ldg(s);
+  for (uint32_t k = 0; k < chunks; ++k) {
+    s += 32;
+    next.c = __ldg(s);
+    run_task<double, true, true, false>(c, v, bad);
+    c = next;
+  }
+  return bad & 1u;
+}
+
 }  // namespace
 
 }  // namespace esl

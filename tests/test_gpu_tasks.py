@@ -76,6 +76,64 @@ def test_block_lanes_equal_warp_lanes(deck, size):
         assert np.array_equal(u, w)
 
 
+def crowd(nodes, parts):
+    """A few nodes with thousands of resistors between them: a small tape
+    beside lanes that take all of a CTA's shared memory."""
+    c = Circuit()
+    c.V("vin", "n0", "0", dc=1.0)
+    for k in range(parts):
+        i = k % nodes
+        j = (i + 1 + k // nodes % (nodes - 1)) % nodes
+        c.R(f"r{k}", f"n{i}", f"n{j}" if k % 3 else "0", 100.0 + k % 71)
+    c.D("d0", f"n{nodes - 1}", "0", is_=1e-14, n=1.0, rs=10.0)
+    fr = c.freeze()
+    return fr, [fr.slot("vin", "dc")]
+
+
+@pytest.mark.parametrize("nodes,first,last", [(9, 2460, 2960), (20, 2070, 2400)])
+def test_lanes_that_fill_shared_memory(nodes, first, last):
+    """Every count of parts up to `last` is a warp lane, whether its words lie
+    in shared memory, stream through a ring or are read where they lie; DC
+    solves, alone and in a group, equal the block lanes', sweeps and measured
+    transients run or are refused."""
+    import torch
+    tran = lanes.tran_opts(1e-9, 1e-10, 1e-10)
+    v = np.linspace(0.5, 3.0, 3).reshape(-1, 1)
+    for parts in list(range(first, last, 90)) + [last]:
+        fr, slots = crowd(nodes, parts)
+        a = solve(fr, slots, v, lanes.PREC_FP64, lanes.PATH_WARP)
+        b = solve(fr, slots, v, lanes.PREC_FP64, lanes.PATH_BLOCK)
+        for u, w in zip(a, b):
+            assert np.array_equal(u, w), parts
+        ctx = lanes.DcLanes(fr)
+        ctx.set_mode(precision=lanes.PREC_FP64, path=lanes.PATH_WARP)
+        ctx.set_lanes(slots, v)
+        if parts < last:  # (a sweep's lane is a little larger)
+            pts = np.linspace(0.0, 1.0, 3)
+            x, it, cv, st, _ = ctx.sweep(slots[0], pts)
+            xo, ito, cvo = oracle.dc_sweep(fr, slots[0], pts)
+            assert (st == lanes.SWEEP_DONE).all() and np.array_equal(it[0], ito) and cv.all() and all(cvo)
+            assert np.allclose(x[0], xo, rtol=1e-9, atol=1e-12)
+        for n_meas in (1, 30):
+            try:
+                ctx.tran_meas(tran, [lanes.window(lanes.MEAS_MAX, fr.unknown("n1"))] * n_meas)
+            except lanes.LaneError as e:
+                assert e.code == lanes.ESL_NOT_ELIGIBLE, str(e)
+        x = torch.zeros((2, 3, fr.n), dtype=torch.float64, device="cuda")
+        words = torch.zeros((2, 2, 3), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        other = lanes.DcLanes(fr)
+        other.set_mode(precision=lanes.PREC_FP64, path=lanes.PATH_WARP)
+        other.set_lanes(slots, v)
+        lanes.group_solve_device([ctx, other], [x[k].data_ptr() for k in range(2)],
+                                 [words[0, k].data_ptr() for k in range(2)],
+                                 [words[1, k].data_ptr() for k in range(2)], cold=[False] * 2)
+        ctx.close()
+        other.close()
+        for k in range(2):
+            assert np.array_equal(x[k].cpu().numpy().view(np.uint64), a[0]), parts
+
+
 def test_wide_words_equal_the_oracle():
     """A mesh of 2,500 unknowns: past 65,536 values."""
     fr, slots, values = mesh(2500)
