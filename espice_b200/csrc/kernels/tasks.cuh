@@ -150,6 +150,15 @@ struct TaskLane<false> {
   __device__ __forceinline__ uint32_t b(int j) const { return j == 0 ? c.w : j == 1 ? e.y : e.w; }
 };
 
+// The barrier between two rows of a CTA's program. Its warps come to it from
+// different places of run_task, a warp without tasks in a row from its idle
+// chunk: the PTX barrier counts warps wherever they arrive, __syncthreads()
+// in such code is defined for a CTA of one mind only.
+__device__ __forceinline__ void task_barrier() {
+  __syncwarp();
+  asm volatile("bar.sync 0;" ::: "memory");
+}
+
 // kCta: the program of a CTA's warps (idle chunks, CTA barriers), else of
 // one warp.
 template <typename V, bool kShared, bool kCompact, bool kCta>
@@ -157,7 +166,7 @@ __device__ __forceinline__ void run_task(const TaskLane<kCompact>& c, const Task
   const uint32_t f = c.flags();
   if constexpr (kCta) {
     if (f & kTaskIdle) {
-      for (uint32_t k = c.idle(); k; --k) __syncthreads();
+      for (uint32_t k = c.idle(); k; --k) task_barrier();
       return;
     }
   }
@@ -190,7 +199,7 @@ __device__ __forceinline__ void run_task(const TaskLane<kCompact>& c, const Task
     d = div ? q : d;
   }
   v.st(dst, d);
-  if (kCta && (f & kTaskCta)) __syncthreads();
+  if (kCta && (f & kTaskCta)) task_barrier();
   else __syncwarp();
 }
 
