@@ -125,15 +125,13 @@ namespace {
 
 // Ops on the longest dependence chain (each op after the last write of the
 // values it reads and of its destination).
-uint32_t longest_chain(const std::vector<SeqOp>& seq, uint32_t nv) {
+uint32_t longest_chain(const std::vector<Op4>& seq, uint32_t nv) {
   std::vector<uint32_t> level(nv, 0);
   uint32_t top = 0;
-  for (const SeqOp& s : seq) {
-    uint32_t l = level[s.dst];
-    for (uint32_t x : {s.a, s.b})
-      if (x != kNone) l = std::max(l, level[x]);
-    level[s.dst] = l + 1;
-    top = std::max(top, l + 1);
+  for (const Op4& o : seq) {
+    const uint32_t v = o.w0 & 0x0fffffffu;
+    level[v] = std::max({level[v], level[o.a], level[o.b]}) + 1;
+    top = std::max(top, level[v]);
   }
   return top;
 }
@@ -181,11 +179,12 @@ Programs compile_tape(const SparseLu& lu) {
     for (uint32_t q = lu.lp[k]; q < lu.lp[k + 1]; ++q) a.push_back({kOpSubNz, y0 + lu.li[q], lx0 + q, y0 + k});
   }
   P.nv = P.ntv + n + 3;
+  P.a_seq.reserve(a.size());
   for (const SeqOp& s : a) {
-    P.a_list.push_back(encode(s.kind, s.dst, s.a, s.b));
-    P.a_seq.push_back(Op4{s.dst | (s.kind << 28), s.a == kNone ? 0u : s.a, s.b == kNone ? 0u : s.b, 0u});
+    if (P.nv < 65536) P.a_list.push_back(encode(s.kind, s.dst, s.a, s.b));
+    P.a_seq.push_back(Op4{s.dst | (s.kind << 28), s.a, s.b, 0u});
   }
-  if (P.nv < 65536) P.a_levels = longest_chain(a, P.nv);
+  if (P.nv < 65536) P.a_levels = longest_chain(P.a_seq, P.nv);
   P.a_nops = uint32_t(a.size());
 
   std::vector<uint8_t> written(P.ntv, 0);
@@ -204,10 +203,10 @@ Programs compile_tape(const SparseLu& lu) {
     for (uint32_t p = lu.up[k]; p < lu.up[k + 1]; ++p) b.push_back({kOpSubNz, y0 + lu.ui[p], p, y0 + k});
   }
   for (const SeqOp& s : b) {
-    P.b_list.push_back(encode(s.kind, s.dst, s.a, s.b));
+    if (P.nv < 65536) P.b_list.push_back(encode(s.kind, s.dst, s.a, s.b));
     P.b_seq.push_back(Op4{s.dst | (s.kind << 28), s.a, s.b, 0u});
   }
-  if (P.nv < 65536) P.b_levels = longest_chain(b, P.nv);
+  if (P.nv < 65536) P.b_levels = longest_chain(P.b_seq, P.nv);
   P.b_nops = uint32_t(b.size());
   return P;
 }
@@ -249,60 +248,85 @@ constexpr int kSlack = 300;
 // alone, and between two such rows no CTA barrier is needed.
 // Against rows of single ops (434 rows for the 498-unknown analog block's
 // refactor, 233 for its back solve) a task keeps its value in a register
-// over its updates and its division: 176 and 101 rows, and 3 loads an update
+// over its updates and its division: 178 and 88 rows, and 3 loads an update
 // in place of 4 accesses.
-TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv, uint32_t warps, bool compact) {
+TaskStream pack_tasks(const std::vector<Op4>& seq, uint32_t nv, uint32_t warps, bool compact) {
   const uint32_t sink = nv - 1, one = nv - 2, zero = nv - 3;
   const size_t n = seq.size();
-  // vop[vptr[v] .. vptr[v + 1]): the ops of value v
-  std::vector<uint32_t> vptr(nv + 1, 0), vop(n), at_op(n);
-  for (const SeqOp& o : seq) ++vptr[o.dst + 1];
+  struct Pair {
+    uint32_t a, b;
+  };
+  auto dst_of = [](const Op4& o) { return o.w0 & 0x0fffffffu; };
+  // ops[vptr[v] .. vptr[v + 1]): the operands of value v's ops; kind[v]: its last op's
+  std::vector<uint32_t> vptr(nv + 1, 0);
+  std::vector<Pair> ops(n);
+  std::vector<uint8_t> kind(nv, kOpNop);
+  for (const Op4& o : seq) ++vptr[dst_of(o) + 1];
   for (uint32_t v = 0; v < nv; ++v) vptr[v + 1] += vptr[v];
-  {
-    std::vector<uint32_t> at(vptr.begin(), vptr.end() - 1);
-    for (size_t i = 0; i < n; ++i) {
-      at_op[i] = at[seq[i].dst];
-      vop[at[seq[i].dst]++] = uint32_t(i);
-    }
+  std::vector<uint32_t> pos(vptr.begin(), vptr.end() - 1);
+  for (const Op4& o : seq) {
+    const uint32_t v = dst_of(o);
+    ops[pos[v]++] = {o.a, o.b};
+    kind[v] = uint8_t(o.w0 >> 28);
   }
-  auto divides = [&](uint32_t v) { return is_div(seq[vop[vptr[v + 1] - 1]].kind); };
-  // cycles from op `pos` of value v to its end
-  auto rest = [&](uint32_t v, uint32_t pos) {
-    const uint32_t left = vptr[v + 1] - pos;
+  auto divides = [&](uint32_t v) { return is_div(kind[v]); };
+  // cycles of value v's last `left` ops
+  auto rest = [&](uint32_t v, uint32_t left) {
     const bool d = divides(v);
     return int(left - (d ? 1u : 0u)) * kCostOp + (d ? kCostDiv : 0);
   };
   // tail[v]: the longest path from v's end to the program's
   std::vector<int> tail(nv, 0);
-  for (size_t i = n; i-- > 0;) {
-    const SeqOp& o = seq[i];
-    const int path = kCostRow + rest(o.dst, at_op[i]) + tail[o.dst];
-    for (uint32_t s : {o.a, o.b})
-      if (s != kNone && s != o.dst) tail[s] = std::max(tail[s], path);
+  {
+    std::vector<uint32_t> left(nv, 0);
+    for (size_t i = n; i-- > 0;) {
+      const Op4& o = seq[i];
+      const uint32_t v = dst_of(o);
+      const int path = kCostRow + rest(v, ++left[v]) + tail[v];
+      for (uint32_t s : {o.a, o.b})
+        if (s != v) tail[s] = std::max(tail[s], path);
+    }
   }
-  std::vector<uint32_t> pos(vptr.begin(), vptr.end() - 1), ready(pos);  // next op; ops before ready[v] can run
-  std::vector<uint8_t> done(nv, 0), queued(nv, 0);
+  std::copy(vptr.begin(), vptr.end() - 1, pos.begin());  // a value's next op
+  std::vector<uint32_t> ready(pos);                      // its ops before ready[v] can run
+  std::vector<uint8_t> done(nv, 0);
   for (uint32_t v = 0; v < nv; ++v) done[v] = vptr[v] == vptr[v + 1];
-  std::vector<std::vector<uint32_t>> waiting(nv);
+  // the values that wait for value s: head[s], next[head[s]], ..
+  std::vector<uint32_t> head(nv, kNone), next(nv, kNone);
   auto advance = [&](uint32_t v) {
     for (; ready[v] < vptr[v + 1]; ++ready[v]) {
-      const SeqOp& o = seq[vop[ready[v]]];
+      const Pair o = ops[ready[v]];
       for (uint32_t s : {o.a, o.b})
-        if (s != kNone && s != v && !done[s]) {
-          waiting[s].push_back(v);
+        if (s != v && !done[s]) {
+          next[v] = head[s];
+          head[s] = v;
           return;
         }
     }
   };
-  std::vector<std::pair<int, uint32_t>> queue;
-  auto push = [&](uint32_t v) {
-    queue.push_back({rest(v, pos[v]) + tail[v], v});
-    std::push_heap(queue.begin(), queue.end());
+  // a task's worth of updates, or all that are left
+  auto full = [&](uint32_t v) { return ready[v] == vptr[v + 1] || ready[v] - pos[v] >= kTaskOps; };
+  // The ready tasks, the longest path on top, and those that wait to be full.
+  // key[v] is value v's place among them, 0 when it has none; an entry that
+  // does not agree with it is stale.
+  std::vector<uint64_t> key(nv, 0), queue, parked;
+  std::vector<uint8_t> is_parked(nv, 0);
+  auto push = [](std::vector<uint64_t>& q, uint64_t k) {
+    q.push_back(k);
+    std::push_heap(q.begin(), q.end());
   };
+  auto pop = [](std::vector<uint64_t>& q) {
+    std::pop_heap(q.begin(), q.end());
+    const uint64_t k = q.back();
+    q.pop_back();
+    return k;
+  };
+  auto path_of = [](uint64_t k) { return int(k >> 32); };
   auto offer = [&](uint32_t v) {
-    if (queued[v] || ready[v] == pos[v]) return;
-    queued[v] = 1;
-    push(v);
+    if (ready[v] == pos[v] || (key[v] && !(is_parked[v] && full(v)))) return;
+    key[v] = uint64_t(uint32_t(rest(v, vptr[v + 1] - pos[v]) + tail[v])) << 32 | v;
+    is_parked[v] = 0;
+    push(queue, key[v]);
   };
   for (uint32_t v = 0; v < nv; ++v)
     if (!done[v]) {
@@ -375,16 +399,16 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv, uint32_t warps
         const Task& t = row[t0 + l];
         x.dst = t.v;
         for (uint32_t j = 0; j < t.ops; ++j) {
-          const SeqOp& o = seq[vop[t.lo + j]];
-          x.pair[j][0] = o.a;
-          x.pair[j][1] = o.b;
-          if (o.kind == kOpSubNz) x.flags |= kTaskNz;
+          x.pair[j][0] = ops[t.lo + j].a;
+          x.pair[j][1] = ops[t.lo + j].b;
         }
+        // a value's updates are of one kind: the solves' before a y entry's
+        // division, the refactor's before an L entry's
+        const uint32_t k = kind[t.v];
+        if (k == kOpSubNz || k == kOpDivY) x.flags |= kTaskNz;
         if (t.div) {
-          const SeqOp& o = seq[vop[t.lo + t.ops]];
-          x.flags |= kTaskDiv | (o.kind == kOpDivGrowth ? kTaskGrowth : 0u) |
-                     (o.kind == kOpDivScaled ? kTaskScaled : 0u);
-          x.pair[kTaskOps - 1][0] = o.a;
+          x.flags |= kTaskDiv | (k == kOpDivGrowth ? kTaskGrowth : 0u) | (k == kOpDivScaled ? kTaskScaled : 0u);
+          x.pair[kTaskOps - 1][0] = ops[t.lo + t.ops].a;
           x.pair[kTaskOps - 1][1] = one;
         }
       }
@@ -393,25 +417,32 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv, uint32_t warps
     ++S.rows;
   };
   std::vector<Task> row, prev;
-  std::vector<uint32_t> later, finished;
+  std::vector<uint32_t> finished;
   size_t left = n;
   while (left) {
     row.clear();
-    later.clear();
-    const int top = queue.front().first;
+    uint64_t top = queue.empty() ? 0 : queue.front();
+    if (!parked.empty()) top = std::max(top, parked.front());
+    const int bar = path_of(top) - kSlack;
+    while (!parked.empty() && path_of(parked.front()) >= bar) {
+      const uint64_t k = pop(parked);
+      const uint32_t v = uint32_t(k);
+      if (key[v] != k || !is_parked[v]) continue;
+      is_parked[v] = 0;
+      push(queue, k);
+    }
     while (!queue.empty() && row.size() < 32 * warps) {
-      std::pop_heap(queue.begin(), queue.end());
-      const uint32_t v = queue.back().second;
-      const int path = queue.back().first;
-      queue.pop_back();
-      if (path < top - kSlack && ready[v] < vptr[v + 1] && ready[v] - pos[v] < kTaskOps) {
-        later.push_back(v);
+      const uint64_t k = pop(queue);
+      const uint32_t v = uint32_t(k);
+      if (key[v] != k || is_parked[v]) continue;
+      if (path_of(k) < bar && !full(v)) {
+        is_parked[v] = 1;
+        push(parked, k);
         continue;
       }
-      queued[v] = 0;
+      key[v] = 0;
       row.push_back(take(v));
     }
-    for (uint32_t v : later) push(v);
     std::sort(row.begin(), row.end(), [&](const Task& x, const Task& y) {
       if (row.size() > 32) {
         if (x.div != y.div) return x.div;
@@ -430,10 +461,11 @@ TaskStream pack_tasks(const std::vector<SeqOp>& seq, uint32_t nv, uint32_t warps
     }
     for (uint32_t v : finished) done[v] = 1;
     for (uint32_t v : finished) {
-      const std::vector<uint32_t> w = std::move(waiting[v]);
-      for (uint32_t x : w) {
+      for (uint32_t x = head[v]; x != kNone;) {
+        const uint32_t after = next[x];
         advance(x);
         offer(x);
+        x = after;
       }
     }
     for (const Task& t : row) offer(t.v);
@@ -466,23 +498,22 @@ void pack_op_rows(Programs& P) {
 }
 
 void compile_warp(const Programs& P, TaskStream& a, TaskStream& b) {
-  a = pack_tasks(unpack(P.a_seq), P.nv, 1, true);
-  b = pack_tasks(unpack(P.b_seq), P.nv, 1, true);
+  a = pack_tasks(P.a_seq, P.nv, 1, true);
+  b = pack_tasks(P.b_seq, P.nv, 1, true);
 }
 
 BlockPrograms compile_block(const Programs& P, uint32_t warps) {
   BlockPrograms B;
   B.compact = P.nv < 65536;
-  const std::vector<SeqOp> a = unpack(P.a_seq), b = unpack(P.b_seq);
-  B.a = pack_tasks(a, P.nv, warps, B.compact);
-  B.b = pack_tasks(b, P.nv, warps, B.compact);
+  B.a = pack_tasks(P.a_seq, P.nv, warps, B.compact);
+  B.b = pack_tasks(P.b_seq, P.nv, warps, B.compact);
   // the forward substitution alone (program A's solve ops), for the mixed
   // form's refinement corrections on the finished factors
-  std::vector<SeqOp> f;
-  for (const SeqOp& s : a)
-    if (s.kind == kOpSubNz) f.push_back(s);
+  std::vector<Op4> f;
+  for (const Op4& s : P.a_seq)
+    if ((s.w0 >> 28) == kOpSubNz) f.push_back(s);
   B.f = pack_tasks(f, P.nv, warps, B.compact);
-  B.a_levels = longest_chain(a, P.nv);
+  B.a_levels = longest_chain(P.a_seq, P.nv);
   return B;
 }
 
