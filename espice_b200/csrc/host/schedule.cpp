@@ -250,6 +250,17 @@ constexpr int kSlack = 300;
 // refactor, 233 for its back solve) a task keeps its value in a register
 // over its updates and its division: 178 and 88 rows, and 3 loads an update
 // in place of 4 accesses.
+// Where the rows are bound by their number and not by the paths through them
+// (a full row's tasks for all the ops make up the longest path), tasks that
+// are full go first and then the columns in their order, whatever their
+// paths: a row's tasks are neighbours in a column, at the same updates, and
+// 32 threads' operands fall into few sectors. Working sets of that size lie
+// in global memory (20,001-unknown digital block, eight warps: 86.0M sectors
+// of loads by longest paths, 25.9M so, in 49,426 and 50,576 rows; 256 lanes,
+// 30 ps: FP64 7,575 -> 2,010 ms, mixed 5,484 -> 1,866; rows of four single ops
+// a thread 5,272 and 3,864). With paths a little longer than the rows the
+// longest ones stay the better order (1,001-unknown mesh, sixteen warps, 162
+// full rows of 319: 0.78 ms against 0.81).
 TaskStream pack_tasks(const std::vector<Op4>& seq, uint32_t nv, uint32_t warps, bool compact) {
   const uint32_t sink = nv - 1, one = nv - 2, zero = nv - 3;
   const size_t n = seq.size();
@@ -304,11 +315,23 @@ TaskStream pack_tasks(const std::vector<Op4>& seq, uint32_t nv, uint32_t warps, 
         }
     }
   };
+  int longest = 0;
+  for (uint32_t v = 0; v < nv; ++v)
+    if (vptr[v] < vptr[v + 1]) longest = std::max(longest, rest(v, vptr[v + 1] - vptr[v]) + tail[v]);
+  const bool near = warps > 1 && n * (kCostRow + kTaskOps * kCostOp) >= size_t(longest) * kTaskOps * 32 * warps;
+  // the values by their first ops' places in the sequence (column by column)
+  std::vector<uint32_t> by_place, place(near ? nv : 0, kNone);
+  for (size_t i = 0; near && i < n; ++i) {
+    const uint32_t v = dst_of(seq[i]);
+    if (place[v] != kNone) continue;
+    place[v] = uint32_t(by_place.size());
+    by_place.push_back(v);
+  }
   // a task's worth of updates, or all that are left
   auto full = [&](uint32_t v) { return ready[v] == vptr[v + 1] || ready[v] - pos[v] >= kTaskOps; };
-  // The ready tasks, the longest path on top, and those that wait to be full.
-  // key[v] is value v's place among them, 0 when it has none; an entry that
-  // does not agree with it is stale.
+  // The ready tasks, the longest path on top (near: the full ones, the first
+  // column), and those that wait to be full. key[v] is value v's place among
+  // them, 0 when it has none; an entry that does not agree with it is stale.
   std::vector<uint64_t> key(nv, 0), queue, parked;
   std::vector<uint8_t> is_parked(nv, 0);
   auto push = [](std::vector<uint64_t>& q, uint64_t k) {
@@ -322,8 +345,16 @@ TaskStream pack_tasks(const std::vector<Op4>& seq, uint32_t nv, uint32_t warps, 
     return k;
   };
   auto path_of = [](uint64_t k) { return int(k >> 32); };
+  auto value_of = [&](uint64_t k) { return near ? by_place[~uint32_t(k)] : uint32_t(k); };
   auto offer = [&](uint32_t v) {
-    if (ready[v] == pos[v] || (key[v] && !(is_parked[v] && full(v)))) return;
+    if (ready[v] == pos[v]) return;
+    if (near) {
+      const uint64_t k = uint64_t(full(v)) << 32 | ~place[v];
+      if (key[v] != k) push(queue, k);
+      key[v] = k;
+      return;
+    }
+    if (key[v] && !(is_parked[v] && full(v))) return;
     key[v] = uint64_t(uint32_t(rest(v, vptr[v + 1] - pos[v]) + tail[v])) << 32 | v;
     is_parked[v] = 0;
     push(queue, key[v]);
@@ -426,16 +457,16 @@ TaskStream pack_tasks(const std::vector<Op4>& seq, uint32_t nv, uint32_t warps, 
     const int bar = path_of(top) - kSlack;
     while (!parked.empty() && path_of(parked.front()) >= bar) {
       const uint64_t k = pop(parked);
-      const uint32_t v = uint32_t(k);
+      const uint32_t v = value_of(k);
       if (key[v] != k || !is_parked[v]) continue;
       is_parked[v] = 0;
       push(queue, k);
     }
     while (!queue.empty() && row.size() < 32 * warps) {
       const uint64_t k = pop(queue);
-      const uint32_t v = uint32_t(k);
+      const uint32_t v = value_of(k);
       if (key[v] != k || is_parked[v]) continue;
-      if (path_of(k) < bar && !full(v)) {
+      if (!near && path_of(k) < bar && !full(v)) {
         is_parked[v] = 1;
         push(parked, k);
         continue;
