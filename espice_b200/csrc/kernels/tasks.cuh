@@ -155,7 +155,6 @@ struct TaskLane<false> {
 // chunk: the PTX barrier counts warps wherever they arrive, __syncthreads()
 // in such code is defined for a CTA of one mind only.
 __device__ __forceinline__ void task_barrier() {
-  __syncwarp();
   asm volatile("bar.sync 0;" ::: "memory");
 }
 
