@@ -211,6 +211,7 @@ cudaError_t upload(DevBuf& b, const std::vector<T>& v, cudaStream_t s) {
 // The block lanes' programs and assembly streams of a tape at one CTA width.
 struct BlockTables {
   bool have = false;
+  uint64_t missed = 0;  // lane iterations of calls that ran at another width for want of these
   BlockPrograms prog;
   uint32_t g_len[kBlockBroad / 32] = {}, g_terms = 0, g_ncells = 0;
   DevBuf d_a, d_b, d_f, d_terms, d_cells;
@@ -762,7 +763,10 @@ int32_t upload_tape(esl_ctx* ctx) {
   T.l_scaled = ctx->d_l_scaled.as<uint8_t>();
   T.pinv = ctx->d_pinv.as<uint32_t>();
   T.qcol = ctx->d_q.as<uint32_t>();
-  for (BlockTables& t : ctx->block) t.have = false;  // a new tape needs its own block programs
+  for (BlockTables& t : ctx->block) {  // a new tape needs its own block programs
+    t.have = false;
+    t.missed = 0;
+  }
   ctx->have_seq = false;        // its own op list
   lu_jit_release(ctx->lu_jit);  // and its own compiled LU
   ctx->lu_jit_state = 0;
@@ -775,64 +779,38 @@ int32_t upload_tape(esl_ctx* ctx) {
   // lane's working set in a CTA's shared memory. A tape beyond them runs on
   // the block lanes only.
   ctx->warp_ok = false;
+  T.tasks = nullptr;
   if (P.nv >= 65536) return ESL_OK;
-  size_t most_lane = 0;
-  {
-    // One blob: the tasks of A and B, gather depth/off/src/dst, each section
-    // 16-byte aligned.
-    GatherSegments G = build_gather_segments(ctx, P);
-    std::vector<unsigned char> blob;
-    auto put = [&blob](const void* p, size_t bytes) {
-      const uint32_t at = uint32_t(blob.size());
-      blob.insert(blob.end(), static_cast<const unsigned char*>(p), static_cast<const unsigned char*>(p) + bytes);
-      blob.resize((blob.size() + 15) & ~size_t(15), 0);
-      return at;
-    };
-    TaskStream A, B;
-    compile_warp(P, A, B);
-    const uint32_t chunk = 32 * task_words(true) * 4;
-    T.a_chunks = A.off[1] - kTaskRing;
-    T.b_chunks = B.off[1] - kTaskRing;
-    T.tasks = nullptr;
-    T.o_g_src = put(G.src.data(), G.src.size() * 4);
-    T.o_g_dst = put(G.dst.data(), G.dst.size() * 4);
-    uint32_t n_kr = 0;
-    GatherProgram K = build_companion_program(ctx, P, n_kr);
-    T.o_k_depth = put(K.depth.data(), K.depth.size() * 4);
-    T.o_k_off = put(K.off.data(), K.off.size() * 4);
-    T.o_k_src = put(K.src.data(), K.src.size() * 4);
-    T.o_k_dst = put(K.dst.data(), K.dst.size() * 4);
-    T.n_kr_groups = n_kr;
-    T.n_ks_groups = uint32_t(K.depth.size()) - n_kr;
-    const size_t gathers = blob.size();
-    // The tasks' words (a stream's first chunk beyond its last is read ahead)
-    // beside the gathers when that leaves room for the largest lane there is,
-    // a transient one with every measure card; else in global memory, with a
-    // ring in the CTA for each lane that leaves room for one (warp_view).
-    const size_t nt = lane_layout(T.n, T.ntv, T.n_stage, T.nlim).total + 9 * size_t(T.n) + 5 * size_t(T.n_qt) +
-                      9 * size_t(T.n_src) + 2 + kMeasDoubles * kMaxMeas;
-    if (blob.size() + size_t(T.a_chunks + T.b_chunks + 2) * chunk + nt * 8 <= size_t(227) * 1024) {
-      T.o_a_tasks = put(A.words.data(), (T.a_chunks + 1) * chunk);
-      T.o_b_tasks = put(B.words.data(), (T.b_chunks + 1) * chunk);
-    } else {
-      T.b_first = A.off[1];
-      A.words.insert(A.words.end(), B.words.begin(), B.words.end());
-      ESL_CUDA(upload(ctx->d_tasks, A.words, s));
-      T.tasks = ctx->d_tasks.as<uint32_t>();
-    }
-    ctx->warp_bytes = uint32_t(gathers);
-    most_lane = nt * 8;
-    ESL_CUDA(upload(ctx->d_prog, blob, s));
-    T.prog = ctx->d_prog.as<unsigned char>();
-    T.prog_bytes = uint32_t(blob.size());
-    T.ring_bytes = 0;
-    T.g_nseg = G.nseg;
-    T.g_seg_blocks = G.seg_len / kGatherBlock;
-  }
   T.smem_doubles = lane_layout(T.n, T.ntv, T.n_stage, T.nlim).total;
   // Every CTA stages the programs; as many lanes per CTA as fit beside them.
   const size_t lane_bytes = size_t(T.smem_doubles) * 8;
   const size_t room = size_t(227) * 1024;
+  if (lane_bytes > room) return ESL_OK;
+  // the largest lane there is, a transient one with every measure card
+  const size_t most_lane = lane_bytes + 8 * (9 * size_t(T.n) + 5 * size_t(T.n_qt) + 9 * size_t(T.n_src) + 2 +
+                                             kMeasDoubles * kMaxMeas);
+  // One blob: gather depth/off/src/dst and the tasks of A and B, each section
+  // 16-byte aligned.
+  std::vector<unsigned char> blob;
+  auto put = [&blob](const void* p, size_t bytes) {
+    const uint32_t at = uint32_t(blob.size());
+    blob.insert(blob.end(), static_cast<const unsigned char*>(p), static_cast<const unsigned char*>(p) + bytes);
+    blob.resize((blob.size() + 15) & ~size_t(15), 0);
+    return at;
+  };
+  GatherSegments G = build_gather_segments(ctx, P);
+  T.o_g_src = put(G.src.data(), G.src.size() * 4);
+  T.o_g_dst = put(G.dst.data(), G.dst.size() * 4);
+  uint32_t n_kr = 0;
+  GatherProgram K = build_companion_program(ctx, P, n_kr);
+  T.o_k_depth = put(K.depth.data(), K.depth.size() * 4);
+  T.o_k_off = put(K.off.data(), K.off.size() * 4);
+  T.o_k_src = put(K.src.data(), K.src.size() * 4);
+  T.o_k_dst = put(K.dst.data(), K.dst.size() * 4);
+  T.n_kr_groups = n_kr;
+  T.n_ks_groups = uint32_t(K.depth.size()) - n_kr;
+  T.g_nseg = G.nseg;
+  T.g_seg_blocks = G.seg_len / kGatherBlock;
   // Which circuits are warp lanes is decided on the programs as rows of 32
   // single ops beside the gathers, so that a call's route does not hang on
   // how they are packed. (The words of a small tape's tasks can take more room
@@ -843,6 +821,7 @@ int32_t upload_tape(esl_ctx* ctx) {
   const size_t least = (P.a_nops + 31) / 32 + (P.b_nops + 31) / 32;
   const size_t most = least + 2 * (size_t(P.a_levels) + P.b_levels);
   constexpr size_t kRowBytes = 32 * sizeof(Op);
+  ctx->warp_bytes = uint32_t(blob.size());
   if (ctx->warp_bytes + least * kRowBytes + lane_bytes > room) return ESL_OK;
   if (ctx->warp_bytes + most * kRowBytes + most_lane <= room) {
     ctx->warp_bytes += uint32_t(most * kRowBytes);
@@ -851,6 +830,28 @@ int32_t upload_tape(esl_ctx* ctx) {
     ctx->warp_bytes += uint32_t((P.a_ops.size() + P.b_ops.size()) * sizeof(Op));
     if (ctx->warp_bytes + lane_bytes > room) return ESL_OK;
   }
+  // The tasks' words (a stream's first chunk beyond its last is read ahead)
+  // beside the gathers when that leaves room for the largest lane; else in
+  // global memory, with a ring in the CTA for each lane that leaves room for
+  // one (warp_view).
+  TaskStream A, B;
+  compile_warp(P, A, B);
+  const uint32_t chunk = 32 * task_words(true) * 4;
+  T.a_chunks = A.off[1] - kTaskRing;
+  T.b_chunks = B.off[1] - kTaskRing;
+  if (blob.size() + size_t(T.a_chunks + T.b_chunks + 2) * chunk + most_lane <= room) {
+    T.o_a_tasks = put(A.words.data(), (T.a_chunks + 1) * chunk);
+    T.o_b_tasks = put(B.words.data(), (T.b_chunks + 1) * chunk);
+  } else {
+    T.b_first = A.off[1];
+    A.words.insert(A.words.end(), B.words.begin(), B.words.end());
+    ESL_CUDA(upload(ctx->d_tasks, A.words, s));
+    T.tasks = ctx->d_tasks.as<uint32_t>();
+  }
+  ESL_CUDA(upload(ctx->d_prog, blob, s));
+  T.prog = ctx->d_prog.as<unsigned char>();
+  T.prog_bytes = uint32_t(blob.size());
+  T.ring_bytes = 0;
   ctx->lanes_eff = warp_fit(ctx, lane_bytes);
   // Transient lanes add the accepted points, the charge rings and dynamic
   // currents over the rows and the LTE states: cur | prev | q[4] | ip over
@@ -957,6 +958,8 @@ void build_block_gather(const esl_ctx* ctx, uint32_t W, std::vector<uint32_t>& t
   }
 }
 
+// Shared memory a block lane may take: a CTA's 227 KB, less the static
+// reduction words.
 constexpr size_t kBlockSmemRoom = size_t(227) * 1024 - 256;
 
 uint32_t block_width(uint32_t threads) { return threads == kBlockNarrow ? 1u : threads == kBlockBroad ? 2u : 0u; }
@@ -1011,9 +1014,6 @@ void block_layout(const TopoDev& T, uint32_t nv, bool mixed, uint32_t split, Blo
   D.cold_bytes = uint32_t(split ? at : 0);
 }
 
-// Shared memory a block lane may take (kBlockSmemRoom: a CTA's 227 KB, less
-// the static reduction words).
-
 // The placement with the most CTAs an SM: the working set in shared memory,
 // its hot part there (split 1, 2; the rest in the CTA's slab), or all of it
 // in the slab; on a tie, the most in shared memory. Returns the CTAs.
@@ -1037,9 +1037,27 @@ int block_place(const TopoDev& T, bool mixed, uint32_t threads, BlockDev& D) {
   return std::max(best, 1);
 }
 
-// The launch view of the block lanes for n_lanes lanes: the CTA's width,
-// programs, layout, where the working set lives, the persistent grid and its
-// slab. The narrow CTAs (DC lanes alone) when there are more lanes than the
+// A width's programs take the host about as long to pack as some 4,000 Newton
+// iterations of their lanes take the GPU, and as some 50,000 save when they
+// run at their best width in place of another (analog block, 5-8 ms: 800 and
+// 10,000 DC lanes). So a call that finds another width's tables runs on those
+// unless it is as large as that, and packs the ones it wanted while its kernel
+// runs once it and those before it come to twice the former (analog block,
+// mixed, a context's first call on 1,000 / 4,000 lanes after its nominal
+// point: 18.7 / 32.6 ms when it packed first, 8.6 / 23 so; 9.7 / 29 with rows
+// of single ops, which had one width).
+constexpr uint64_t kPackBeside = 8192, kPackFirst = 49152;
+
+// The CTA widths a call's kernels come in, its Newton iterations over all
+// lanes (estimated), and the width to pack while it runs (0: none).
+struct BlockCall {
+  bool narrow = false, broad = false;
+  uint64_t iterations = 0;
+  uint32_t pack = 0;
+};
+
+// The CTA width that n_lanes lanes run best at, their placement at that width
+// (D) and the CTAs an SM. The narrow CTAs (DC lanes alone) when there are more lanes than the
 // wide ones hold at once and the narrow ones hold more of them: a lane's
 // rows are a chain of latencies that issues on a quarter of the cycles, so
 // four narrow lanes on an SM take less than twice the time of two wide ones
@@ -1049,16 +1067,15 @@ int block_place(const TopoDev& T, bool mixed, uint32_t threads, BlockDev& D) {
 // take half the rows (2,000-unknown digital block: 1,113 -> 620; working
 // sets in shared memory are smaller, their rows are chains that 256 threads
 // already hold).
-int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D, bool narrow_ok = false,
-                   bool broad_ok = false) {
+uint32_t block_choose(const esl_ctx* ctx, bool mixed, uint32_t n_lanes, const BlockCall& call, BlockDev& D, int& best) {
   const TopoDev& T = ctx->topo;
   D = BlockDev{};
   uint32_t threads = kBlockThreads;
-  int best = block_place(T, mixed, threads, D);
-  if (broad_ok && !D.in_smem && n_lanes <= uint32_t(ctx->sms)) {
+  best = block_place(T, mixed, threads, D);
+  if (call.broad && !D.in_smem && n_lanes <= uint32_t(ctx->sms)) {
     threads = kBlockBroad;
     best = block_place(T, mixed, threads, D);
-  } else if (narrow_ok && n_lanes > uint32_t(ctx->sms) * uint32_t(best)) {
+  } else if (call.narrow && n_lanes > uint32_t(ctx->sms) * uint32_t(best)) {
     BlockDev N{};
     const int narrow = block_place(T, mixed, kBlockNarrow, N);
     if (N.in_smem && narrow > best) {
@@ -1066,6 +1083,26 @@ int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D, bool
       best = narrow;
       threads = kBlockNarrow;
     }
+  }
+  return threads;
+}
+
+// The launch view of the block lanes for a call on n_lanes lanes: the CTA's
+// width, programs, layout, where the working set lives, the persistent grid
+// and its slab.
+int32_t block_view(esl_ctx* ctx, bool mixed, uint32_t n_lanes, BlockDev& D, BlockCall& call) {
+  const TopoDev& T = ctx->topo;
+  int best = 0;
+  uint32_t threads = block_choose(ctx, mixed, n_lanes, call, D, best);
+  BlockTables& wanted = ctx->block[block_width(threads)];
+  const uint32_t other = threads == kBlockThreads ? kBlockBroad : kBlockThreads;
+  if (!wanted.have && ctx->block[block_width(other)].have && (other == kBlockThreads || call.broad) &&
+      call.iterations < kPackFirst) {
+    wanted.missed += call.iterations;
+    if (wanted.missed >= kPackBeside) call.pack = threads;
+    threads = other;
+    D = BlockDev{};
+    best = block_place(T, mixed, threads, D);
   }
   if (int32_t rc = ensure_block(ctx, threads)) return rc;
   const BlockTables& B = ctx->block[block_width(threads)];
@@ -1108,6 +1145,12 @@ bool use_block(const esl_ctx* ctx) {
 // The lead lane's first Jacobian in pattern order: the warp assembly kernel
 // when its working set fits a CTA's shared memory, else the block lanes'
 // (global scratch). The same gathers in the same order: the same bits.
+// The tables a running call wanted (BlockCall.pack): the host has nothing
+// else to do meanwhile. That they cannot be had is no fault of the call.
+void pack_beside(esl_ctx* ctx, const BlockCall& call) {
+  if (call.pack && ensure_block(ctx, call.pack) != ESL_OK) cudaGetLastError();
+}
+
 cudaError_t lead_jacobian(esl_ctx* ctx, const LaneDev& L, double* out) {
   const TopoDev& T = ctx->topo;
   const size_t smem = size_t(4 * T.n + T.nv + T.n_stage + T.nlim + 2) * sizeof(double);
@@ -1471,8 +1514,11 @@ int32_t dc_solve(esl_ctx* ctx, const esl_newton_opts* opts, double* d_x, int col
     return ctx->fail(ESL_NOT_ELIGIBLE, ctx->warp_ok ? "the warp lanes solve in FP64 only" : "the tape exceeds the warp lanes");
   const bool mixed = ctx->precision == ESL_PREC_MIXED && !d_rung;
   BlockDev D{};
+  BlockCall call;
   if (block) {
-    if (int32_t rc = block_view(ctx, mixed, N, D, !d_rung, !d_rung)) return rc;
+    call.narrow = call.broad = !d_rung;  // the ladder's kernel has one width
+    call.iterations = uint64_t(N) * 5;
+    if (int32_t rc = block_view(ctx, mixed, N, D, call)) return rc;
     if (D.refine_out) ESL_CUDA(cudaMemsetAsync(D.refine_out, 0, size_t(N) * 4, s));
     if (D.prof) ESL_CUDA(cudaMemsetAsync(D.prof, 0, kBlockPhases * sizeof(unsigned long long), s));
   }
@@ -1483,6 +1529,7 @@ int32_t dc_solve(esl_ctx* ctx, const esl_newton_opts* opts, double* d_x, int col
   };
   ESL_CUDA(cudaEventRecord(ctx->ev0, s));
   ESL_CUDA(launch(L));
+  pack_beside(ctx, call);
   uint32_t launches = 1;
   for (;;) {
     bool any = false;
@@ -1711,7 +1758,10 @@ int32_t run_tran_block(esl_ctx* ctx, LaneDev L, TranDev P, const LaneOpts& lo) {
   if (P.meas) return ctx->fail(ESL_NOT_ELIGIBLE, "the block transient lanes stream no measure cards");
   const bool mixed = ctx->precision == ESL_PREC_MIXED;
   BlockDev D{};
-  if (int32_t rc = block_view(ctx, mixed, N, D, false, true)) return rc;
+  BlockCall call;
+  call.broad = true;
+  call.iterations = uint64_t(double(N) * 2.0 * std::min(P.t_stop / P.dt_max, 1e6));
+  if (int32_t rc = block_view(ctx, mixed, N, D, call)) return rc;
   if (mixed) ESL_CUDA(cudaMemsetAsync(D.refine_out, 0, size_t(N) * 4, s));
   ESL_CUDA(ctx->d_tran_slab.ensure(size_t(D.grid) * tran_block_slab(ctx->topo) * 8));
   ESL_CUDA(ctx->d_x_good.ensure(size_t(N) * ctx->topo.n * 8));
@@ -1720,6 +1770,7 @@ int32_t run_tran_block(esl_ctx* ctx, LaneDev L, TranDev P, const LaneOpts& lo) {
   std::memset(&ctx->last_peels, 0, sizeof(ctx->last_peels));
   ESL_CUDA(cudaEventRecord(ctx->ev0, s));
   ESL_CUDA(launch_tran_block(D, L, P, lo, mixed, topo_has_b3(ctx->topo), ctx->d_tran_slab.as<double>(), s));
+  pack_beside(ctx, call);
   ctx->last_peels.launches = 1;
   ESL_CUDA(cudaEventRecord(ctx->ev1, s));
   ESL_CUDA(cudaEventSynchronize(ctx->ev1));
@@ -1982,7 +2033,8 @@ int32_t group_block(esl_ctx* const* ctxs, uint32_t n_ctx, const esl_newton_opts*
   size_t smem = 0, stride = 16;
   for (uint32_t c = 0; c < n_ctx; ++c) {
     esl_ctx* x = ctxs[c];
-    if (int32_t rc = block_view(x, mixed, x->n_lanes, Ds[c])) return rc;
+    BlockCall call;  // a group's CTAs have one width
+    if (int32_t rc = block_view(x, mixed, x->n_lanes, Ds[c], call)) return rc;
     if (Ds[c].refine_out) ESL_CUDA(cudaMemsetAsync(Ds[c].refine_out, 0, size_t(x->n_lanes) * 4, x->stream));
     ESL_CUDA(cudaStreamSynchronize(x->stream));
     b3 |= topo_has_b3(x->topo);
@@ -2207,7 +2259,8 @@ int32_t esl_block_info(esl_ctx* ctx, esl_block_info_t* info) {
   info->warp_ok = ctx->warp_ok;
   for (int m = 0; m < 2; ++m) {
     BlockDev D{};
-    if (int32_t rc = block_view(ctx, m == 1, ctx->n_lanes ? ctx->n_lanes : 1, D)) return rc;
+    BlockCall call;
+    if (int32_t rc = block_view(ctx, m == 1, ctx->n_lanes ? ctx->n_lanes : 1, D, call)) return rc;
     info->lane_bytes[m] = D.lane_bytes;
     info->in_smem[m] = D.in_smem;
     info->ctas_per_sm[m] = uint32_t(std::max(

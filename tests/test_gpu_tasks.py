@@ -65,6 +65,27 @@ def test_narrow_ctas_equal_wide(deck, size, precision):
         assert np.array_equal(u[pick], v)
 
 
+@pytest.mark.parametrize("deck,size,precision,n", [
+    (mesh, 200, lanes.PREC_MIXED, 700), (mesh, 200, lanes.PREC_FP64, 1500),
+    (mesh, 1000, lanes.PREC_FP64, 300), (mesh, 1000, lanes.PREC_MIXED, 1000)])
+def test_calls_after_another_width(deck, size, precision, n):
+    """A batch on a context that solved one lane at another width runs there at
+    first and changes over later: the same bits in every call."""
+    fr, slots, values = deck(size)
+    v = values(n)
+    want = solve(fr, slots, v, precision, lanes.PATH_BLOCK)
+    ctx = lanes.DcLanes(fr)
+    ctx.set_mode(precision=precision, path=lanes.PATH_BLOCK)
+    ctx.set_lanes(slots, v[:1])
+    ctx.solve(x0=np.zeros(fr.n))
+    ctx.set_lanes(slots, v)
+    for _ in range(8):
+        x, it, st, _ = ctx.solve(x0=np.zeros(fr.n))
+        for u, w in zip((x.view(np.uint64), it, st), want):
+            assert np.array_equal(u, w)
+    ctx.close()
+
+
 @pytest.mark.parametrize("deck,size", [(ladder, 1), (ladder, 28), (ladder, 29), (ladder, 61), (grid, 0), (mesh, 50),
                                        (mesh, 110), (mesh, 140)])
 def test_block_lanes_equal_warp_lanes(deck, size):
