@@ -1038,7 +1038,7 @@ def our_arm(args, rank, world):
                     "refinements_per_newton_iter": ref_per_iter,
                     "ctas_per_sm": info["ctas_per_sm"], "lane_bytes": info["lane_bytes"],
                     "note": "cycles of one CTA (one lane) per Newton iteration by phase, thread 0's clock64; "
-                            "rows are CTA-wide steps of the tape programs, each ending in a barrier; "
+                            "rows are the steps of the tape programs between barriers, a CTA's or a warp's; "
                             "levels_over_rows: the dependency bound of program A over its scheduled rows"},
         "setup": dict(setup, train_loss_first_last=[float(loss[0]), float(loss[-1])]),
         "clocks": clk.summary(),

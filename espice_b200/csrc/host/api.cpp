@@ -2245,31 +2245,32 @@ int32_t esl_block_profile(esl_ctx* ctx, uint64_t* cycles) {
 int32_t esl_block_info(esl_ctx* ctx, esl_block_info_t* info) {
   if (!ctx || !info || !ctx->have_tape) return ESL_INVALID_ARGUMENT;
   cudaSetDevice(ctx->device);
-  if (int32_t rc = ensure_block(ctx, kBlockThreads)) return rc;
-  const BlockPrograms& prog = ctx->block[0].prog;
   std::memset(info, 0, sizeof(*info));
-  info->width = kBlockThreads;
-  info->a_rows = prog.a.rows;
-  info->b_rows = prog.b.rows;
-  info->f_rows = prog.f.rows;
-  info->a_levels = prog.a_levels;
   info->a_nops = ctx->prog.a_nops;
   info->b_nops = ctx->prog.b_nops;
   info->ntv = ctx->prog.ntv;
   info->warp_ok = ctx->warp_ok;
+  BlockCall call;
+  call.narrow = call.broad = true;
   for (int m = 0; m < 2; ++m) {
     BlockDev D{};
-    BlockCall call;
-    if (int32_t rc = block_view(ctx, m == 1, ctx->n_lanes ? ctx->n_lanes : 1, D, call)) return rc;
+    int per_sm = 0;
+    const uint32_t threads = block_choose(ctx, m == 1, ctx->n_lanes, call, D, per_sm);
     info->lane_bytes[m] = D.lane_bytes;
     info->in_smem[m] = D.in_smem;
-    info->ctas_per_sm[m] = uint32_t(std::max(
-        0, block_occupancy(m == 1, topo_has_b3(ctx->topo), kBlockThreads,
-                           D.ring_bytes + (D.in_smem ? D.lane_bytes : 0))));
-    info->split[m] = D.split != 0;
+    info->ctas_per_sm[m] = uint32_t(per_sm);
+    info->split[m] = D.split;
     info->cold_bytes[m] = D.cold_bytes;
-    info->gather_terms = ctx->block[0].g_terms;
-    info->gather_cells = ctx->block[0].g_ncells;
+    if (m != (ctx->precision == ESL_PREC_MIXED)) continue;
+    if (int32_t rc = ensure_block(ctx, threads)) return rc;
+    const BlockTables& t = ctx->block[block_width(threads)];
+    info->width = threads;
+    info->a_rows = t.prog.a.rows;
+    info->b_rows = t.prog.b.rows;
+    info->f_rows = t.prog.f.rows;
+    info->a_levels = t.prog.a_levels;
+    info->gather_terms = t.g_terms;
+    info->gather_cells = t.g_ncells;
   }
   return ESL_OK;
 }

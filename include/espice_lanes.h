@@ -141,9 +141,10 @@ typedef struct {
  * stand in for (the pivot tests on them) takes the host's FP64 factor.
  * path: ESL_PATH_AUTO picks the warp lanes (a warp per lane, its working
  * set in shared memory) for FP64 when the tape fits them, else the block
- * lanes (a CTA per lane, block_threads wide: 256, or 0 for 256; the
- * working set in shared memory when it fits, else in global memory, for any
- * circuit size); ESL_PATH_WARP / ESL_PATH_BLOCK force one (the warp lanes
+ * lanes (a CTA per lane; its working set in shared memory when it fits, in
+ * part or whole in global memory otherwise, for any circuit size; a CTA has
+ * 256 threads, or where that is faster 128 or 512, which esl_block_info
+ * tells; block_threads: 0 or 256); ESL_PATH_WARP / ESL_PATH_BLOCK force one (the warp lanes
  * are FP64 only). refine_tol 0 takes 1e-12, refine_max 0 takes 6.
  * refine_skip > 0 (mixed precision): a Newton step whose FP32 solution is
  * still more than refine_skip times its convergence tolerance (the delta
@@ -403,16 +404,19 @@ int32_t esl_group_dc_solve_device(esl_ctx *const *ctxs, uint32_t n_ctx, const es
 int32_t esl_set_mode(esl_ctx *ctx, const esl_solve_mode *mode);
 
 /* The block lanes' programs and working set for the context's tape (after
- * its first solve): rows of `width` ops in programs A (refactor + forward
- * solve, a_levels its longest dependence chain), B and F; the tape's
- * values and ops; per precision (0 FP64, 1 mixed) a lane's working-set
- * bytes in shared memory (all of it, or its hot part when split), whether
- * it sits in shared memory, CTAs per SM, and whether it is split (its
- * previous iterate and staging cells, cold_bytes, in global memory). */
+ * its first solve), as a DC solve of its current lanes runs best. For the
+ * mode's precision: threads of a CTA (`width`); the steps between barriers,
+ * a CTA's or a warp's, of programs A (refactor + forward solve, a_levels its
+ * longest dependence chain), B and F; the assembly's terms and cells a
+ * thread walks. The tape's ops and values. Per precision (0 FP64, 1 mixed):
+ * a lane's working-set bytes in shared memory (all of it, or its hot part
+ * when split; in global memory when not in_smem), CTAs per SM, and how it is
+ * split (1: its previous iterate and staging cells, 2: all but the values
+ * and limits, cold_bytes of it in global memory). */
 typedef struct {
     uint32_t width, a_rows, b_rows, f_rows, a_levels, a_nops, b_nops, ntv, warp_ok;
     uint32_t lane_bytes[2], in_smem[2], ctas_per_sm[2], split[2], cold_bytes[2];
-    uint32_t gather_terms, gather_cells; /* the assembly's terms and cells a thread walks */
+    uint32_t gather_terms, gather_cells;
 } esl_block_info_t;
 int32_t esl_block_info(esl_ctx *ctx, esl_block_info_t *info);
 

@@ -51,6 +51,18 @@ def solve(fr, slots, values, precision, path):
     return x.view(np.uint64), it, st
 
 
+def width(fr, slots, values, precision):
+    """Threads of the CTAs these lanes run best on."""
+    ctx = lanes.DcLanes(fr)
+    ctx.set_mode(precision=precision, path=lanes.PATH_BLOCK)
+    ctx.set_lanes(slots, values[:1])
+    ctx.solve(x0=np.zeros(fr.n))
+    ctx.set_lanes(slots, values)
+    w = ctx.block_info()["width"]
+    ctx.close()
+    return w
+
+
 @pytest.mark.parametrize("precision", [lanes.PREC_FP64, lanes.PREC_MIXED])
 @pytest.mark.parametrize("deck,size", [(ladder, 1), (ladder, 31), (ladder, 130), (grid, 0), (mesh, 50), (mesh, 200),
                                        (mesh, 400)])
@@ -63,16 +75,20 @@ def test_narrow_ctas_equal_wide(deck, size, precision):
     b = solve(fr, slots, big[pick], precision, lanes.PATH_BLOCK)
     for u, v in zip(a, b):
         assert np.array_equal(u[pick], v)
+    # (four narrow FP64 lanes of the 400-unknown mesh would lie in global memory: it stays wide)
+    narrow = 256 if (deck, size, precision) == (mesh, 400, lanes.PREC_FP64) else 128
+    assert (width(fr, slots, big, precision), width(fr, slots, big[pick], precision)) == (narrow, 256)
 
 
-@pytest.mark.parametrize("deck,size,precision,n", [
-    (mesh, 200, lanes.PREC_MIXED, 700), (mesh, 200, lanes.PREC_FP64, 1500),
-    (mesh, 1000, lanes.PREC_FP64, 300), (mesh, 1000, lanes.PREC_MIXED, 1000)])
-def test_calls_after_another_width(deck, size, precision, n):
+@pytest.mark.parametrize("deck,size,precision,n,widths", [
+    (mesh, 200, lanes.PREC_MIXED, 700, (256, 128)), (mesh, 200, lanes.PREC_FP64, 1500, (256, 128)),
+    (mesh, 1000, lanes.PREC_FP64, 300, (512, 256)), (mesh, 1000, lanes.PREC_MIXED, 1000, (512, 256))])
+def test_calls_after_another_width(deck, size, precision, n, widths):
     """A batch on a context that solved one lane at another width runs there at
     first and changes over later: the same bits in every call."""
     fr, slots, values = deck(size)
     v = values(n)
+    assert (width(fr, slots, v[:1], precision), width(fr, slots, v, precision)) == widths
     want = solve(fr, slots, v, precision, lanes.PATH_BLOCK)
     ctx = lanes.DcLanes(fr)
     ctx.set_mode(precision=precision, path=lanes.PATH_BLOCK)
@@ -84,6 +100,24 @@ def test_calls_after_another_width(deck, size, precision, n):
         for u, w in zip((x.view(np.uint64), it, st), want):
             assert np.array_equal(u, w)
     ctx.close()
+
+
+@pytest.mark.parametrize("precision", [lanes.PREC_FP64, lanes.PREC_MIXED])
+def test_broad_transients_equal_wide(precision):
+    """A digital block's transient lanes with an SM each (512 threads) and one
+    lane more (256)."""
+    fr, slots = decks.digital_block(size=1500, n_cells=37, n_inputs=8)
+    v = decks.digital_block_vto(len(slots), 149, seed=3)
+    out = []
+    for n in (149, 148):
+        ctx = lanes.DcLanes(fr)
+        ctx.set_mode(precision=precision, path=lanes.PATH_BLOCK)
+        ctx.set_lanes(slots, v[:n])
+        stats, x = ctx.tran(lanes.tran_opts(2e-11, 1e-11, 1e-11))[3:5]
+        out.append((x.view(np.uint64)[:148], stats[:148]))
+        assert ctx.block_info()["width"] == (256 if n == 149 else 512)
+        ctx.close()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
 
 
 @pytest.mark.parametrize("deck,size", [(ladder, 1), (ladder, 28), (ladder, 29), (ladder, 61), (grid, 0), (mesh, 50),
