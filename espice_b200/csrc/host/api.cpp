@@ -274,6 +274,7 @@ struct esl_ctx {
   LuJitKernels lu_jit;                               // the tape-compiled lane LU of the current tape
   LuJitKernels lu_jit_dx;                            // its form without the factors
   int lu_jit_dx_state = 0;
+  uint32_t lu_jit_dx_planes = 0;                     // and the scratch planes it uses
   DevBuf d_lu_scratch;                               // its tape-value plane when the caller passes none
   LuJitKernels lu_jit_mixed;                         // the compiled mixed-precision form
   int lu_jit_mixed_state = 0;
@@ -684,7 +685,7 @@ std::vector<Op> lane_sequence(const Programs& P, uint32_t& n_a, uint32_t& n_all,
 // the same order as the warp programs', so the same bits), which keeps
 // fewer values live at once than the programs' level-packed rows.
 std::string compiled_lu_source(uint32_t nnz, const SparseLu& lu, const Programs& P, uint32_t resident = 0,
-                               bool mixed = false, bool factors_out = true) {
+                               bool mixed = false, bool factors_out = true, uint32_t* planes = nullptr) {
   std::vector<Op> seq = P.a_list;
   const uint32_t n_a = uint32_t(seq.size());
   seq.insert(seq.end(), P.b_list.begin(), P.b_list.end());
@@ -719,7 +720,7 @@ std::string compiled_lu_source(uint32_t nnz, const SparseLu& lu, const Programs&
   }
   if (mixed) in.resident_values = 48;  // the refinement loop needs the registers (more spilled)
   if (resident) in.resident_values = resident;
-  return lu_jit_source(in);
+  return lu_jit_source(in, planes);
 }
 
 // Warp lanes of lane_bytes a CTA holds beside the staged programs, each with
@@ -2455,13 +2456,14 @@ int32_t esl_lu_lanes_compiled_device(esl_ctx* ctx, const double* lead, uint32_t 
     if (ctx->prog.a_nops + ctx->prog.b_nops > kLuJitMaxOps)
       return ctx->fail(ESL_NOT_ELIGIBLE, "the tape is too long to compile");
     const std::string src =
-        compiled_lu_source(ctx->topo.nnz, ctx->lead, ctx->prog, 0, false, d_tv != nullptr);
+        compiled_lu_source(ctx->topo.nnz, ctx->lead, ctx->prog, 0, false, d_tv != nullptr,
+                           d_tv ? nullptr : &ctx->lu_jit_dx_planes);
     if (!lu_jit_build(src, jit)) return ctx->fail(ESL_NOT_ELIGIBLE, "compiling the tape failed: " + jit.log);
     state = 1;
   }
   if (state < 0) return ctx->fail(ESL_NOT_ELIGIBLE, "the tape could not be compiled");
   if (!d_tv) {
-    ESL_CUDA(ctx->d_lu_scratch.ensure(size_t(ctx->prog.ntv) * n_lanes * 8));
+    ESL_CUDA(ctx->d_lu_scratch.ensure(size_t(ctx->lu_jit_dx_planes) * n_lanes * 8));
     d_tv = ctx->d_lu_scratch.as<double>();
   }
   ESL_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));

@@ -64,11 +64,15 @@ struct Gen {
   std::vector<int64_t> pos;
   int64_t cur_stage = -1;
   uint32_t n_stages = 0;
-  // factors_out false: the entries no op writes, whose home is A (or zero)
+  // factors_out false: the entries no op writes, whose home is A (or zero);
+  // each value's plane, and their number
   std::vector<uint8_t> kept;
+  std::vector<int64_t> plane;
+  uint32_t planes = 0;
 
   explicit Gen(const LuJitInput& i) : in(i) {
     defined.assign(in.nv, 0);
+    plane.assign(in.ntv, -1);
     slot_of.assign(in.nv, -1);
     row_of.assign(in.nv, -1);
     pos.assign(in.nv, -1);
@@ -92,11 +96,15 @@ struct Gen {
   uint32_t next_use(uint32_t v) const { return next[v] < uses[v].size() ? uses[v][next[v]] : kNever; }
   bool constant(uint32_t v) const { return v >= in.nv - 3; }
 
-  // The home of value v, as an expression for this lane.
-  std::string home(uint32_t v) const {
+  // The home of value v, as an expression for this lane (without the factors
+  // a tape value takes a scratch plane when it first needs one).
+  std::string home(uint32_t v) {
     std::ostringstream h;
     if (v < in.ntv && kept[v]) h << "al[" << slot_of[v] << " * N]";
-    else if (v < in.ntv) h << "tl[" << v << " * N]";
+    else if (v < in.ntv) {
+      if (plane[v] < 0) plane[v] = in.factors_out ? int64_t(v) : int64_t(planes++);
+      h << "tl[" << plane[v] << " * N]";
+    }
     else h << "dx[" << (*in.qcol)[v - in.ntv] << " * N + lane]";
     return h.str();
   }
@@ -326,7 +334,7 @@ static void refinement(const LuJitInput& in, std::ostringstream& os) {
      << "  if (refine_out) refine_out[lane] = refined;\n";
 }
 
-std::string lu_jit_source(const LuJitInput& in) {
+std::string lu_jit_source(const LuJitInput& in, uint32_t* planes) {
   const std::vector<Op>& seq = *in.seq;
   // the last op that writes each value, per program
   std::vector<int64_t> last_a(in.nv, -1), last_all(in.nv, -1);
@@ -429,6 +437,7 @@ std::string lu_jit_source(const LuJitInput& in) {
   if (in.mixed) refinement(in, os);
   os << "  bad_out[lane] = bad;\n"
      << "}\n";
+  if (planes) *planes = in.factors_out ? in.ntv : g.planes;
   return os.str();
 }
 

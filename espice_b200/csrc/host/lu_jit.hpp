@@ -43,8 +43,8 @@ struct LuJitInput {
 // statement in the given order; the tape values go to their plane `tv`
 // (the caller's, or scratch) as they become final and come back from it
 // when their next use is far off. A caller that wants no factors gets the
-// form without their stores (factors_out).
-std::string lu_jit_source(const LuJitInput& in);
+// form without their stores (factors_out). `planes`: those of `tv` it uses.
+std::string lu_jit_source(const LuJitInput& in, uint32_t* planes = nullptr);
 
 struct LuJitKernels {
   cudaLibrary_t lib = nullptr;
