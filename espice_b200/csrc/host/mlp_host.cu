@@ -77,7 +77,11 @@ struct esl_mlp {
   Dev<float> dz, dh, t, loss, xf;
   Dev<__nv_bfloat16> dzb, dzt;
   Dev<int> gerr;
-  Dev<uint32_t> perm, at;        // training: an epoch's order, the step within it
+  // training: the loss's stream beside the gradients, the events that order
+  // it, an epoch's order, the step within it
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  Dev<uint32_t> perm, at;
   Dev<esl::AdamRate> rates;      // and each step's rate and bias corrections
 
   int32_t fail(int32_t code, const std::string& what) {
@@ -276,9 +280,14 @@ int32_t esl_mlp_destroy(esl_mlp* m) {
   if (!m) return ESL_MLP_OK;
   cudaSetDevice(m->device);
   cudaStream_t s = m->stream;
+  const cudaStream_t side = m->side;
   if (s) cudaStreamSynchronize(s);
+  if (side) cudaStreamSynchronize(side);
+  for (cudaEvent_t e : {m->fork, m->join})
+    if (e) cudaEventDestroy(e);
   delete m;
-  if (s) cudaStreamDestroy(s);
+  for (cudaStream_t x : {s, side})
+    if (x) cudaStreamDestroy(x);
   return ESL_MLP_OK;
 }
 
@@ -309,32 +318,19 @@ int32_t esl_mlp_set_scaling(esl_mlp* m, const float* in_mu, const float* in_sig,
   return ESL_MLP_OK;
 }
 
-// A training run's second stream (the loss beside the gradients), the
-// events that order it, and the step's graph: for the run alone, since the
-// inputs' addresses are in it.
+// The step's graph: for one run alone, since the inputs' addresses are in it.
 struct TrainRun {
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  cudaError_t init() {
-    cudaError_t e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
-    return e;
-  }
   ~TrainRun() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
-    if (fork) cudaEventDestroy(fork);
-    if (join) cudaEventDestroy(join);
-    if (side) cudaStreamDestroy(side);
   }
 };
 
 // One training step's launches on the network's stream: the batch at
 // perm[*at], forward, the gradients, Adam on every tensor, the next step.
-static int32_t train_step(esl_mlp* m, TrainRun& run, const float* d_x, const float* d_y, int B) {
+static int32_t train_step(esl_mlp* m, const float* d_x, const float* d_y, int B) {
   cudaStream_t s = m->stream;
   Layer& last = *m->layers.back();
   const int kin = m->layers[0]->k;
@@ -345,10 +341,10 @@ static int32_t train_step(esl_mlp* m, TrainRun& run, const float* d_x, const flo
                                                          m->d_out_sig.p, nullptr, m->t.p);
   MLP_CUDA(cudaGetLastError());
   if (int32_t rc = forward(m, B)) return rc;
-  MLP_CUDA(cudaEventRecord(run.fork, s));
-  MLP_CUDA(cudaStreamWaitEvent(run.side, run.fork, 0));
-  MLP_CUDA(esl::launch_mse_loss(m->z.back()->p, m->t.p, B, m->n_out, last.n, m->loss.p, run.side));
-  MLP_CUDA(cudaEventRecord(run.join, run.side));
+  MLP_CUDA(cudaEventRecord(m->fork, s));
+  MLP_CUDA(cudaStreamWaitEvent(m->side, m->fork, 0));
+  MLP_CUDA(esl::launch_mse_loss(m->z.back()->p, m->t.p, B, m->n_out, last.n, m->loss.p, m->side));
+  MLP_CUDA(cudaEventRecord(m->join, m->side));
   MLP_CUDA(esl::launch_mse_grad(m->z.back()->p, m->t.p, B, m->n_out, last.n, m->dz.p, s));
   if (int32_t rc = backward(m, B)) return rc;
   esl::AdamTensors T{};
@@ -361,15 +357,15 @@ static int32_t train_step(esl_mlp* m, TrainRun& run, const float* d_x, const flo
     T.t[T.n++] = {ly->b, ly->gb, ly->mb, ly->vb, nullptr, nullptr, 1, ly->n, 0};
   }
   MLP_CUDA(esl::launch_adam(T, m->rates.p, m->at.p, s));
-  MLP_CUDA(cudaStreamWaitEvent(s, run.join, 0));
+  MLP_CUDA(cudaStreamWaitEvent(s, m->join, 0));
   MLP_CUDA(esl::launch_next_step(m->at.p, s));
   return ESL_MLP_OK;
 }
 
-// The first step is launched as it is; the others replay it as a graph: a
-// step is some two dozen short kernels, and launched one by one they cost
-// the host 18 us each, tensor maps included (512 hidden, batch 256: 460 us a
-// step, 100 as a graph).
+// The first step is launched as it is; the others replay it as a graph, made
+// when the second comes: a step is some two dozen short kernels, and launched
+// one by one they cost the host 18 us each, tensor maps included (512 hidden,
+// batch 256: 460 us a step, 100 as a graph).
 int32_t esl_mlp_train(esl_mlp* m, const float* d_x, const float* d_y, uint32_t n, uint32_t epochs, uint32_t batch,
                       float lr, float lr_end, uint64_t seed, float* loss_out) {
   if (!m || !d_x || !d_y || n == 0 || batch == 0 || batch % 16) return ESL_MLP_INVALID_ARGUMENT;
@@ -394,8 +390,11 @@ int32_t esl_mlp_train(esl_mlp* m, const float* d_x, const float* d_y, uint32_t n
     p1 *= esl::kAdamB1;
     p2 *= esl::kAdamB2;
   }
+  if (!m->side) MLP_CUDA(cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking));
+  for (cudaEvent_t* e : {&m->fork, &m->join})
+    if (!*e) MLP_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   TrainRun run;
-  MLP_CUDA(run.init());
+  bool first = true;
   std::vector<esl::AdamRate> rates(n_batches);
   for (uint32_t ep = 0; ep < epochs; ++ep) {
     // geometric decay from lr to lr_end over the epochs
@@ -414,18 +413,20 @@ int32_t esl_mlp_train(esl_mlp* m, const float* d_x, const float* d_y, uint32_t n
     MLP_CUDA(cudaMemsetAsync(m->at.p, 0, 4, s));
     MLP_CUDA(cudaMemsetAsync(m->loss.p, 0, 4, s));
     for (uint32_t bi = 0; bi < n_batches; ++bi) {
-      if (run.exec) {
-        MLP_CUDA(cudaGraphLaunch(run.exec, s));
+      if (first) {
+        first = false;
+        if (int32_t rc = train_step(m, d_x, d_y, B)) return rc;
         continue;
       }
-      int32_t rc = train_step(m, run, d_x, d_y, B);
-      if (rc) return rc;
-      MLP_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      rc = train_step(m, run, d_x, d_y, B);
-      const cudaError_t ended = cudaStreamEndCapture(s, &run.graph);
-      if (rc) return rc;
-      MLP_CUDA(ended);
-      MLP_CUDA(cudaGraphInstantiate(&run.exec, run.graph, 0));
+      if (!run.exec) {
+        MLP_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        const int32_t rc = train_step(m, d_x, d_y, B);
+        const cudaError_t ended = cudaStreamEndCapture(s, &run.graph);
+        if (rc) return rc;
+        MLP_CUDA(ended);
+        MLP_CUDA(cudaGraphInstantiate(&run.exec, run.graph, 0));
+      }
+      MLP_CUDA(cudaGraphLaunch(run.exec, s));
     }
     float l = 0;
     MLP_CUDA(cudaMemcpyAsync(&l, m->loss.p, 4, cudaMemcpyDeviceToHost, s));

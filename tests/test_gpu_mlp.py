@@ -6,11 +6,15 @@
 - The network's gradients against the numpy restatement (oracle/mlp_ref.py),
   which rounds to BF16 where the GPU does: relative error of each gradient
   tensor below 1e-3 (FP32 summation order, and a BF16 rounding it flips).
-- Training on the GPU fits a smooth map.
+- Training on the GPU fits a smooth map, takes the steps of a host
+  restatement, and does not depend on work queued on the default stream; the
+  loss of uneven, infinite and NaN errors.
 - A completion wait that runs out (every wait bounded to no rounds) raises
   the timeout status and stores nothing; the next unbounded GEMM on the same
   device is correct (the drained MMAs left the context usable).
 """
+
+import subprocess
 
 import numpy as np
 import pytest
@@ -182,6 +186,88 @@ def test_training_beside_work_on_the_default_stream(passes):
 
     (la, wa), (lb, wb) = run(passes), run(0)
     assert np.array_equal(la, lb) and np.array_equal(wa.view(np.uint32), wb.view(np.uint32))
+
+
+SHUFFLE = r"""
+#include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+#include <vector>
+int main(int, char** v) {
+  std::mt19937_64 rng(std::strtoull(v[1], nullptr, 10));
+  std::vector<unsigned> p(std::atoi(v[2]));
+  for (unsigned i = 0; i < p.size(); ++i) p[i] = i;
+  for (int e = std::atoi(v[3]); e--;) {
+    std::shuffle(p.begin(), p.end(), rng);
+    for (unsigned i : p) std::printf("%u ", i);
+  }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def orders(tmp_path_factory):
+    """The runs' sample orders: the C++ library's shuffle of 0 .. n - 1, epoch after epoch."""
+    d = tmp_path_factory.mktemp("shuffle")
+    (d / "s.cpp").write_text(SHUFFLE)
+    subprocess.run(["g++", "-O1", str(d / "s.cpp"), "-o", str(d / "s")], check=True)
+    return lambda seed, n, epochs: np.array(
+        subprocess.run([str(d / "s"), str(seed), str(n), str(epochs)], check=True, capture_output=True,
+                       text=True).stdout.split(), np.int64).reshape(epochs, n)
+
+
+def test_training_steps_match_the_restatement(orders):
+    """Two runs of several epochs and batches of distinct rows on one network,
+    the rate decaying: batches, rates and bias corrections as a host
+    restatement takes them (the numpy gradients, Adam in FP64). Each step's
+    gradients agree to 1e-3 of their norm; of the elements, about that part
+    lies below the error and may turn the sign of its step, sqrt(1e-3) = 3%
+    of a step's norm, and ten steps add up. A wrong batch, rate or
+    correction moves the weights elsewhere altogether."""
+    torch = _torch()
+    rng = np.random.default_rng(21)
+    n_in, n_out, batch, n = 6, 20, 32, 70  # two batches and a rest an epoch
+    x = rng.normal(size=(n, n_in)).astype(np.float32)
+    y = (np.sin(2.0 * x @ rng.normal(size=(n_in, n_out))) + rng.normal(size=(n, n_out))).astype(np.float32)
+    dx, dy = torch.tensor(x, device="cuda"), torch.tensor(y, device="cuda")
+    torch.cuda.synchronize()
+    net = mlp.Mlp(n_in, 48, 3, n_out, seed=6)
+    layers = [(w.astype(np.float64), b.astype(np.float64)) for w, b in net.weights()]
+    start = np.concatenate([a.ravel() for layer in layers for a in layer])
+    mom = [[np.zeros_like(a) for a in layer] for layer in layers]
+    var = [[np.zeros_like(a) for a in layer] for layer in layers]
+    one = np.ones(max(n_in, n_out), np.float32)
+    t = 0
+    for epochs, lr, lr_end, seed in ((3, 2e-2, 5e-3, 4), (2, 1e-2, 2e-3, 9)):
+        got = net.train(dx.data_ptr(), dy.data_ptr(), n, epochs=epochs, batch=batch, lr=lr, lr_end=lr_end, seed=seed)
+        perm = orders(seed, n, epochs)
+        for ep in range(epochs):
+            rate = lr * (lr_end / lr) ** (ep / (epochs - 1))
+            losses = []
+            for b in range(n // batch):
+                rows = perm[ep][b * batch:(b + 1) * batch]
+                loss, grads = mlp_ref.gradients([(w.astype(np.float32), c.astype(np.float32)) for w, c in layers],
+                                                x[rows], y[rows], 0 * one[:n_in], one[:n_in], 0 * one[:n_out],
+                                                one[:n_out])
+                losses.append(loss)
+                t += 1
+                new = []
+                for k, layer in enumerate(layers):
+                    out = []
+                    for j, a in enumerate(layer):
+                        g = grads[k][j].astype(np.float64)
+                        mom[k][j] = 0.9 * mom[k][j] + 0.1 * g
+                        var[k][j] = 0.999 * var[k][j] + 0.001 * g * g
+                        out.append(a - rate * (mom[k][j] / (1 - 0.9 ** t)) / (np.sqrt(var[k][j] / (1 - 0.999 ** t))
+                                                                             + 1e-8))
+                    new.append(tuple(out))
+                layers = new
+            assert abs(got[ep] - np.mean(losses)) <= 1e-2 * np.mean(losses)
+        want = np.concatenate([a.ravel() for layer in layers for a in layer]) - start
+        moved = np.concatenate([a.ravel() for layer in net.weights() for a in layer]) - start
+        assert np.linalg.norm(moved - want) <= 0.1 * np.linalg.norm(want)
+    net.close()
 
 
 def test_gemm_wait_runs_out_and_stores_nothing():
