@@ -224,7 +224,6 @@ struct esl_ctx {
   std::string err;
   uint32_t lanes_per_block = 0;  // 0: as many as the lane count spreads over the SMs
   uint32_t lanes_eff = 4;  // lanes per CTA that fit beside the staged programs
-  uint32_t tran_lanes_eff = 0;  // the same for the transient kernel (0: does not fit)
   int sms = 148;
 
   Csc pat;
@@ -267,7 +266,7 @@ struct esl_ctx {
   DevBuf d_tran_state, d_tran_save;    // paused transient lanes' state
   esl_stats last_peels{};              // the last call's peel counts (esl_peel_stats)
   uint64_t last_tran_refinements = 0;  // the last block transient's FP64 corrections (mixed)
-  uint32_t warp_bytes = 0;  // what decides whether a lane is a warp lane (upload_tape)
+  size_t warp_bytes = 0;  // the gathers, which with the rows decide whether a lane is a warp lane (warp_holds)
   bool have_seq = false;
   uint32_t n_seq_a = 0, n_seq = 0, seq_warps = 0;  // lane-interleaved op list
   uint32_t n_seq_f = 0, mixed_warps = 0;            // its forward-only tail, the mixed kernel's warps
@@ -713,7 +712,9 @@ std::string compiled_lu_source(uint32_t nnz, const SparseLu& lu, const Programs&
   // A tape of at most 256 values keeps most of them in 112 registers' worth
   // of two CTAs an SM: its traffic falls by more than the halved warps cost
   // (131,072 lanes, ring's 226 values: with the factors 123 -> 100 us,
-  // without 106 -> 82; the grid's 789 values: 938 -> 1,151).
+  // without 106 -> 82; the grid's 789 values: 938 -> 1,151; 65,536 lanes of
+  // meshes, with the factors: 209 values 79 -> 69 us, 265 values 103 -> 92,
+  // 313 values 127 -> 159, 363 values 151 -> 196).
   if (!mixed && P.ntv + P.n <= 256) {
     in.resident_values = 112;
     in.min_blocks = 2;
@@ -721,6 +722,25 @@ std::string compiled_lu_source(uint32_t nnz, const SparseLu& lu, const Programs&
   if (mixed) in.resident_values = 48;  // the refinement loop needs the registers (more spilled)
   if (resident) in.resident_values = resident;
   return lu_jit_source(in, planes);
+}
+
+// Whether a warp lane of lane_bytes fits a CTA's shared memory. It is decided
+// on the programs as rows of 32 single ops beside the gathers, so that a
+// call's route does not hang on how they are packed. (The words of a small
+// tape's tasks can take more room than its rows; they lie in shared memory
+// only where every lane has room beside them, and a lane beside the gathers
+// alone needs no ring.) The rows are packed only when their bounds leave it
+// open: a full row takes 32 ops, and of two rows that are not full the
+// longest path to the end gets shorter.
+bool warp_holds(esl_ctx* ctx, size_t lane_bytes) {
+  Programs& P = ctx->prog;
+  constexpr size_t kRoom = size_t(227) * 1024, kRowBytes = 32 * sizeof(Op);
+  const size_t least = (P.a_nops + 31) / 32 + (P.b_nops + 31) / 32;
+  const size_t most = least + 2 * (size_t(P.a_levels) + P.b_levels), beside = ctx->warp_bytes + lane_bytes;
+  if (beside + least * kRowBytes > kRoom) return false;
+  if (beside + most * kRowBytes <= kRoom) return true;
+  pack_op_rows(P);
+  return beside + (P.a_ops.size() + P.b_ops.size()) * sizeof(Op) <= kRoom;
 }
 
 // Warp lanes of lane_bytes a CTA holds beside the staged programs, each with
@@ -812,25 +832,8 @@ int32_t upload_tape(esl_ctx* ctx) {
   T.n_ks_groups = uint32_t(K.depth.size()) - n_kr;
   T.g_nseg = G.nseg;
   T.g_seg_blocks = G.seg_len / kGatherBlock;
-  // Which circuits are warp lanes is decided on the programs as rows of 32
-  // single ops beside the gathers, so that a call's route does not hang on
-  // how they are packed. (The words of a small tape's tasks can take more room
-  // than its rows; they lie in shared memory only where every lane has room
-  // beside them, and a lane beside the gathers alone needs no ring.) The rows are
-  // packed only when their bounds leave it open: a full row takes 32 ops, and
-  // of two rows that are not full the longest path to the end gets shorter.
-  const size_t least = (P.a_nops + 31) / 32 + (P.b_nops + 31) / 32;
-  const size_t most = least + 2 * (size_t(P.a_levels) + P.b_levels);
-  constexpr size_t kRowBytes = 32 * sizeof(Op);
-  ctx->warp_bytes = uint32_t(blob.size());
-  if (ctx->warp_bytes + least * kRowBytes + lane_bytes > room) return ESL_OK;
-  if (ctx->warp_bytes + most * kRowBytes + most_lane <= room) {
-    ctx->warp_bytes += uint32_t(most * kRowBytes);
-  } else {
-    pack_op_rows(P);
-    ctx->warp_bytes += uint32_t((P.a_ops.size() + P.b_ops.size()) * sizeof(Op));
-    if (ctx->warp_bytes + lane_bytes > room) return ESL_OK;
-  }
+  ctx->warp_bytes = blob.size();
+  if (!warp_holds(ctx, lane_bytes)) return ESL_OK;
   // The tasks' words (a stream's first chunk beyond its last is read ahead)
   // beside the gathers when that leaves room for the largest lane; else in
   // global memory, with a ring in the CTA for each lane that leaves room for
@@ -860,8 +863,6 @@ int32_t upload_tape(esl_ctx* ctx) {
   // current time point and the PULSE corner timers (4 start/period pairs
   // per source).
   T.tran_doubles = (T.smem_doubles + 7 * T.n + 5 * T.n_qt + 9 * T.n_src + 1) & ~1u;
-  const size_t tran_bytes = size_t(T.tran_doubles) * 8;
-  ctx->tran_lanes_eff = ctx->warp_bytes + tran_bytes > room ? 0 : warp_fit(ctx, tran_bytes);
   ctx->warp_ok = true;
   return ESL_OK;
 }
@@ -1839,8 +1840,9 @@ int32_t esl_tran_device(esl_ctx* ctx, const esl_tran_opts* opts, double* d_x, ui
   if (int32_t rc = ensure_tape_cold(ctx)) return rc;
   // the block lanes when asked for, for mixed precision (the warp lanes are
   // FP64), or when a warp lane cannot hold the run
+  const size_t lane_bytes = size_t(ctx->topo.tran_doubles) * 8;
   const bool block = ctx->path == ESL_PATH_BLOCK || ctx->precision == ESL_PREC_MIXED || !ctx->warp_ok ||
-                     ctx->tran_lanes_eff == 0;
+                     !warp_holds(ctx, lane_bytes);
   P.stats = d_stats;
   P.n_probes = max_pts ? n_probes : 0;
   P.max_pts = max_pts;
@@ -1852,7 +1854,7 @@ int32_t esl_tran_device(esl_ctx* ctx, const esl_tran_opts* opts, double* d_x, ui
   L.x = d_x;
   if (block) {
     if (int32_t rc = run_tran_block(ctx, L, P, lo)) return rc;
-  } else if (int32_t rc = run_tran(ctx, L, P, lo, lanes_per_cta(ctx, ctx->n_lanes, ctx->tran_lanes_eff))) {
+  } else if (int32_t rc = run_tran(ctx, L, P, lo, lanes_per_cta(ctx, ctx->n_lanes, warp_fit(ctx, lane_bytes)))) {
     return rc;
   }
   if (ms) cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1);
@@ -1886,8 +1888,8 @@ int32_t esl_dc_sweep_device(esl_ctx* ctx, const esl_slot* slot, const double* va
   }
   if (int32_t rc = warp_only(ctx)) return rc;
   const TopoDev& T = ctx->topo;
-  const size_t lane_bytes = size_t(sweep_doubles(T)) * 8, room = size_t(227) * 1024;
-  if (ctx->warp_bytes + lane_bytes > room) return ctx->fail(ESL_NOT_ELIGIBLE, "a sweep lane exceeds a CTA's shared memory");
+  const size_t lane_bytes = size_t(sweep_doubles(T)) * 8;
+  if (!warp_holds(ctx, lane_bytes)) return ctx->fail(ESL_NOT_ELIGIBLE, "a sweep lane exceeds a CTA's shared memory");
   const uint32_t fit = warp_fit(ctx, lane_bytes);
   ESL_CUDA(ctx->d_sweep_values.ensure(size_t(n_pts) * 8));
   ESL_CUDA(cudaMemcpyAsync(ctx->d_sweep_values.p, values, size_t(n_pts) * 8, cudaMemcpyHostToDevice, s));
@@ -1961,8 +1963,8 @@ int32_t esl_tran_meas_device(esl_ctx* ctx, const esl_tran_opts* opts, const esl_
   if (int32_t rc = ensure_tape_cold(ctx)) return rc;
   if (int32_t rc = warp_only(ctx)) return rc;
   const TopoDev& T = ctx->topo;
-  const size_t lane_bytes = (size_t(T.tran_doubles) + size_t(kMeasDoubles) * n_meas) * 8, room = size_t(227) * 1024;
-  if (ctx->warp_bytes + lane_bytes > room) return ctx->fail(ESL_NOT_ELIGIBLE, "a transient lane exceeds a CTA's shared memory");
+  const size_t lane_bytes = (size_t(T.tran_doubles) + size_t(kMeasDoubles) * n_meas) * 8;
+  if (!warp_holds(ctx, lane_bytes)) return ctx->fail(ESL_NOT_ELIGIBLE, "a transient lane exceeds a CTA's shared memory");
   const uint32_t fit = warp_fit(ctx, lane_bytes);
   cudaStream_t s = ctx->stream;
   ESL_CUDA(ctx->d_meas.ensure(size_t(n_meas) * sizeof(esl_measure)));
