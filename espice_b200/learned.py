@@ -44,8 +44,10 @@ class LearnedWarmStart:
         import torch
         # the moments on the device, in FP64 as before: on the host they took
         # longer than the training's first epochs (8,192 x 498 targets: 15 ms)
-        v = torch.as_tensor(np.ascontiguousarray(values, np.float64), device="cuda")
-        t = torch.as_tensor(np.ascontiguousarray(x, np.float64), device="cuda")
+        def on_device(a):
+            a = np.ascontiguousarray(a, np.float64)
+            return torch.as_tensor(a if a.flags.writeable else a.copy(), device="cuda")  # (read-only ones warn)
+        v, t = on_device(values), on_device(x)
         m = torch.cat([v.mean(0), v.std(0, correction=0), t.mean(0), t.std(0, correction=0)]).cpu().numpy()
         mu_in, sig_in, mu_out, sig_out = np.split(m, np.cumsum([v.shape[1], v.shape[1], t.shape[1]]))
         self.net.set_scaling(mu_in, np.where(sig_in > 0, sig_in, 1.0), mu_out,

@@ -54,3 +54,25 @@ def test_learned_warm_start_cuts_newton_iterations():
     ws.close()
     fb.close()
     ctx.close()
+
+
+def test_fit_takes_arrays_as_they_come():
+    """Read-only, sliced and 32-bit arrays, lists: no warning, the same fit."""
+    import warnings
+    rng = np.random.default_rng(8)
+    values = rng.uniform(0.5, 1.5, (64, 3)).astype(np.float32).astype(np.float64)
+    x = np.sin(values @ rng.normal(size=(3, 5))).astype(np.float32).astype(np.float64)
+    frozen = values.copy(), x.copy()
+    for a in frozen:
+        a.flags.writeable = False
+    out = []
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        for v, t in ((values, x), frozen, (np.repeat(values, 2, 0)[::2], x[:, ::-1][:, ::-1]),
+                     (values.astype(np.float32), x.astype(np.float32)), (values.tolist(), x.tolist())):
+            ws = learned.LearnedWarmStart(3, 5, hidden=16, layers=2, seed=3)
+            out.append((ws.fit(v, t, epochs=2, batch=32), [w for layer in ws.net.weights() for w in layer]))
+            ws.close()
+    for loss, weights in out[1:]:
+        assert np.array_equal(loss, out[0][0])
+        assert all(np.array_equal(a, b) for a, b in zip(weights, out[0][1]))
