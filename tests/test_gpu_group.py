@@ -63,8 +63,8 @@ def test_autotune_keeps_results():
 def test_block_group_uneven_batch_against_oracle(precision):
     """The uneven batch on the block lanes: the eight mesh-with-gates
     topologies (50 to 2,000 unknowns), six supply values each, in one launch
-    (work items largest topology first; the two largest keep their working
-    set in global memory). FP64: every lane bitwise the oracle, the same
+    (work items largest topology first; the largest are most of the work and
+    lie in global memory, so all do). FP64: every lane bitwise the oracle, the same
     iteration counts. Mixed: the oracle's convergence, values within 1e-9
     relative or 1e-12 absolute."""
     import torch
@@ -99,4 +99,35 @@ def test_block_group_uneven_batch_against_oracle(precision):
         else:
             assert np.array_equal(conv, cvo.astype(bool))
             assert parity.close(x[conv], xo[conv]).all(), float(np.max(np.abs(x[conv] - xo[conv])))
+        c.close()
+
+
+@pytest.mark.parametrize("precision", [lanes.PREC_FP64, lanes.PREC_MIXED])
+@pytest.mark.parametrize("sizes,counts", [
+    ((50, 100, 200), (40, 40, 40)),      # all in shared memory
+    ((50, 200, 1500), (300, 300, 4)),    # the small ones there, the large one in global memory
+    ((200, 2500), (400, 2)),             # and its words of the wide form, for one ring
+    ((50, 200, 1500), (4, 4, 8)),        # all in global memory
+])
+def test_block_group_placements(sizes, counts, precision):
+    """Where a group's working sets lie changes no bit: its lanes are those of
+    each topology solved alone."""
+    import torch
+    ctxs, bufs, alone = [], [], []
+    for size, n in zip(sizes, counts):
+        fr, slots = decks.mesh_gates(size)
+        c = lanes.DcLanes(fr)
+        c.set_mode(precision=precision, path=lanes.PATH_BLOCK)
+        c.set_lanes(slots, np.linspace(0.8, 1.8, n).reshape(-1, 1))
+        alone.append(c.solve(x0=None)[:3])
+        ctxs.append(c)
+        bufs.append((torch.zeros((n, fr.n), dtype=torch.float64, device="cuda"),
+                     torch.zeros(n, dtype=torch.int32, device="cuda"),
+                     torch.zeros(n, dtype=torch.int32, device="cuda")))
+    torch.cuda.synchronize()
+    lanes.group_solve_device(ctxs, [b[0].data_ptr() for b in bufs], [b[1].data_ptr() for b in bufs],
+                             [b[2].data_ptr() for b in bufs], cold=[True] * len(ctxs))
+    for c, b, (x, it, st) in zip(ctxs, bufs, alone):
+        assert np.array_equal(b[0].cpu().numpy().view(np.uint64), x.view(np.uint64))
+        assert np.array_equal(b[1].cpu().numpy(), it) and np.array_equal(b[2].cpu().numpy(), st)
         c.close()
