@@ -7,10 +7,11 @@
 // Program A is the refactor with the forward substitution through unit L
 // merged in (a column's forward updates run as soon as its L entries and
 // y entry are final, overlapping later columns' refactor); program B is the
-// back substitution through U. Each is list-scheduled into rows of 32 ops,
-// one op per thread of the lane's warp, padded with no-ops; a row holds
-// divisions only or multiply-subtracts only, so the kernel's branch between
-// the two is uniform across the warp.
+// back substitution through U. Each is list-scheduled into rows of tasks
+// (common.h: up to three updates of one value and its division), one task
+// per thread of the lane's warp or CTA; and, for the interpreted lane LU,
+// into rows of 32 single ops, each row of divisions only or
+// multiply-subtracts only.
 #pragma once
 
 #include <cstdint>
@@ -35,9 +36,9 @@ struct Programs {
   uint32_t nv = 0;                 // value space: ntv + n (y) + 0.0, 1.0, sink
   std::vector<uint32_t> amap;      // pattern slot -> tape value
   std::vector<uint32_t> fill;      // tape values no pattern slot writes
-  std::vector<Op> a_ops;           // rows x 32: refactor + forward solve
+  std::vector<Op> a_ops;           // rows x 32: refactor + forward solve (pack_op_rows)
   std::vector<Op> b_ops;           // rows x 32: back solve
-  std::vector<Op> a_list, b_list;  // the same ops in the replay's sequential order (column by column)
+  std::vector<Op> a_list, b_list;  // the ops in the replay's sequential order (column by column), 16-bit indices
   std::vector<Op4> a_seq, b_seq;   // the same, with 32-bit indices (any value space)
   uint32_t a_rows = 0, b_rows = 0, a_levels = 0, b_levels = 0;  // levels: longest chain
   uint32_t a_nops = 0, b_nops = 0; // real ops (no padding)

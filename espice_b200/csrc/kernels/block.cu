@@ -10,14 +10,13 @@
 // per-thread stream of staging indices read eight terms ahead, so neither
 // waits on an L2 round trip per row or per term.
 //
-// Where the working set lives: x | rhs | diag | dx | limited images |
-// (mixed: the FP64 matrix) | v = [tape values | y | 0.0 | 1.0 | sink] |
-// xo | staging, in the CTA's shared memory when it fits; or its hot part
-// (up to v) there and xo and the staging cells (written once and read once
-// an iteration, by the evaluation and the assembly) in a per-CTA slab of
-// global memory, when that lets more CTAs share an SM; else all of it in
-// the slab (L2-resident for the lane's solve; one CTA writes and reads it,
-// ordered by its barriers).
+// Where the working set lives: limited images | v = [tape values | y | 0.0 |
+// 1.0 | sink] | x | rhs | diag | dx | (mixed: the FP64 matrix) | xo |
+// staging, in the CTA's shared memory when it fits; or its hot part there and
+// the rest in a per-CTA slab of global memory, when that lets more CTAs share
+// an SM (xo and the staging cells, written once and read once an iteration
+// by the evaluation and the assembly; or all from x on); else all of it in
+// the slab (one CTA writes and reads it, ordered by its barriers).
 //
 // Two precisions. FP64: the refactor and solves are bitwise the CPU replay
 // (sparse_lu.zig refactor + solve), as the warp programs are. Mixed: the
@@ -142,7 +141,7 @@ __device__ __forceinline__ BlockMem<V> block_carve(const BlockDev& D, unsigned c
 // gmin > 0 adds loadExtras' diagonal and residual terms; gs > 0 the
 // gmin-stepping rung's at the cells that carry a stamp (c.w: 1 on a stamped
 // slot, the column + 1 on a stamped row). Fill-in tape values are zeroed.
-template <typename V, uint32_t kW>
+template <typename V>
 __device__ __forceinline__ void gather_store(const BlockDev& D, const BlockMem<V>& b, const uint4& c, double s,
                                              double gmin, double gs) {
   constexpr bool kMixed = sizeof(V) == 4;
@@ -193,7 +192,7 @@ __device__ void block_assemble(const BlockDev& D, const BlockMem<V>& b, double g
     for (uint32_t j = 0; j < kGBatch; ++j) {
       s = __dadd_rn(s, x.v[j]);
       if (x.ends >> j & 1u) {
-        gather_store<V, kW>(D, b, cell, s, gmin, gs);
+        gather_store<V>(D, b, cell, s, gmin, gs);
         s = 0.0;
         cell = next;
         next = __ldg(cells);

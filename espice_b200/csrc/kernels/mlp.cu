@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(kThreads) gemm_bf16_tc(const __grid_constant__
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
 }
 
-// dZ = dH * (1 - tanh(Z)^2) for a tanh layer (zpre given; dz is dH's buffer
-// turned in place), dZ as it stands for the output layer; its BF16 copy and
+// dZ = dH * (1 - tanh(Z)^2) for a tanh layer (zpre given), dH as it stands
+// for the output layer, whose dZ it is; its BF16 copy and
 // that copy's transpose, through a 32 x 32 tile, in the same pass.
 __global__ void layer_grad(const float* dh, const float* zpre, int rows, int cols, float* dz, __nv_bfloat16* dzb,
                            __nv_bfloat16* dzt) {
