@@ -274,11 +274,12 @@ def reference_arm(args, rank, world):
 
 
 # DRAM bytes per point of one mixed dc_block_kernel launch on the analog
-# block, from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum,
-# --set full) of a 4,096-point learned step: 419.1 MB read, 121.8 MB
-# written. The kernel reads a point's records once and keeps its working set
-# on chip, so the traffic grows with points, not with iterations.
-C4_BLOCK_DRAM_BYTES_PER_LANE = (419.072256e6 + 121.783296e6) / 4096
+# block, from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum)
+# of a 4,096-point learned step: 2,411.9 MB read, 3,449.9 MB written. The
+# narrow CTAs keep the tape values and limits in shared memory and the rest
+# of a point's working set in their slabs, whose lines L2 writes back while
+# the records stream through it.
+C4_BLOCK_DRAM_BYTES_PER_LANE = (2411.851e6 + 3449.881e6) / 4096
 
 # DRAM bytes per lane of one tran_kernel launch, from an ncu capture
 # (dram__bytes_read.sum + dram__bytes_write.sum, --set full) of 148 ring
@@ -1026,9 +1027,10 @@ def our_arm(args, rank, world):
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one mixed "
                                        "dc_block_kernel launch on a reduced point count, scaled by points",
                      "peak_source": peak_src,
-                     "note": "each lane's working set stays in its CTA's shared memory for the whole solve, so "
-                             "HBM carries only records, starts and solutions: the kernel is bound by the "
-                             "latency of its dependent program rows (the latency block)"},
+                     "note": "a lane's tape values stay in its CTA's shared memory for the whole solve, the rest "
+                             "of its working set in the CTA's slab (mostly L2), so HBM carries little beside "
+                             "records, starts and solutions: the kernel is bound by the latency of its dependent "
+                             "program rows (the latency block)"},
         "latency": {"cycles_per_newton_iter": {k: round(v) for k, v in cyc.items()},
                     "rows_per_newton_iter": rows_per_iter,
                     "refactor_cycles_per_row": cyc["refactor"] / info["a_rows"],

@@ -248,7 +248,7 @@ constexpr int kSlack = 300;
 // alone, and between two such rows no CTA barrier is needed.
 // Against rows of single ops (434 rows for the 498-unknown analog block's
 // refactor, 233 for its back solve) a task keeps its value in a register
-// over its updates and its division: 178 and 88 rows, and 3 loads an update
+// over its updates and its division: 176 and 107 rows, and 3 loads an update
 // in place of 4 accesses.
 // Where the rows are bound by their number and not by the paths through them
 // (a full row's tasks for all the ops make up the longest path), tasks that
