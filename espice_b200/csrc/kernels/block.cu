@@ -602,7 +602,7 @@ cudaError_t launch_t(const BlockDev& D, const LaneDev& L, const LaneOpts& o, cud
     }
   }
   const size_t smem = D.ring_bytes + (D.in_smem ? D.lane_bytes : 0);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   const uint32_t grid = D.grid < L.n_lanes ? D.grid : L.n_lanes;
   k<<<grid > 0 ? grid : 1, D.threads, smem, s>>>(D, L, o);
@@ -613,7 +613,7 @@ template <typename V, bool kHasB3>
 int occupancy_t(uint32_t threads, size_t smem) {
   int per_sm = 0;
   auto* k = dc_kernel<V, kHasB3>(threads);
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return 0;
+  if (allow_smem(k, smem) != cudaSuccess) return 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, int(threads), smem);
   return per_sm;
 }
@@ -623,7 +623,7 @@ cudaError_t launch_group_t(const BlockDev* Ds, const LaneDev* Ls, const uint2* i
                            uint32_t* next, const LaneOpts& o, unsigned char* slab, size_t slab_stride, size_t smem,
                            uint32_t grid, cudaStream_t s) {
   auto* k = dc_block_group_kernel<V, kHasB3, kBlockThreads>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(next, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
@@ -635,7 +635,7 @@ template <typename V, bool kHasB3>
 int group_occupancy_t(size_t smem) {
   int per_sm = 0;
   auto* k = dc_block_group_kernel<V, kHasB3, kBlockThreads>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return 0;
+  if (allow_smem(k, smem) != cudaSuccess) return 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, int(kBlockThreads), smem);
   return per_sm;
 }
@@ -1129,7 +1129,7 @@ cudaError_t launch_tran_t(const BlockDev& D, const LaneDev& L, const TranDev& P,
   auto* k = D.threads == kBlockBroad ? tran_block_kernel<V, kHasB3, kBlockBroad>
                                      : tran_block_kernel<V, kHasB3, kBlockThreads>;
   const size_t smem = D.ring_bytes + (D.in_smem ? D.lane_bytes : 0);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   const uint32_t grid = D.grid < L.n_lanes ? D.grid : L.n_lanes;
   k<<<grid > 0 ? grid : 1, D.threads, smem, s>>>(D, L, P, o, tslab, tslab_stride);

@@ -8,6 +8,7 @@
 #include <cstdint>
 
 #include "lanes.cuh"
+#include "smem.h"
 
 namespace esl {
 

@@ -6,6 +6,7 @@
 #include <cstdint>
 
 #include "lanes.cuh"
+#include "smem.h"
 
 namespace esl {
 

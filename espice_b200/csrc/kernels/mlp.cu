@@ -19,6 +19,7 @@
 #include <cstdint>
 
 #include "mlp.h"
+#include "smem.h"
 
 namespace esl {
 
@@ -466,7 +467,7 @@ cudaError_t launch_gemm_bf16(const __nv_bfloat16* a, int lda, const __nv_bfloat1
   const int stages = bn <= 128 ? 3 : 2;
   const size_t stage_bytes = size_t(kTileM) * kTileK * 2 + size_t(bn) * kTileK * 2;
   const size_t smem = std::max<size_t>(100 * 1024, size_t(stages) * stage_bytes + 1024);
-  e = cudaFuncSetAttribute(gemm_bf16_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  e = allow_smem(gemm_bf16_tc, smem);
   if (e != cudaSuccess) return e;
   dim3 grid((M + kTileM - 1) / kTileM, N / bn);
   gemm_bf16_tc<<<grid, kThreads, smem, s>>>(ta, tb, M, K, bn, stages, bias, c, ldc, h, ldh, act, err,

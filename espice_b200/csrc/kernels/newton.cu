@@ -544,7 +544,7 @@ static cudaError_t launch_dc_newton_t(const TopoDev& T, const LaneDev& L, const 
                                       cudaStream_t s) {
   const size_t smem = T.prog_bytes + T.ring_bytes + lanes_per_block * lane_smem_bytes(T);
   auto* k = o.ladder ? dc_newton_kernel<kHasB3, true> : dc_newton_kernel<kHasB3, false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   k<<<persistent_grid(k, L.n_lanes, lanes_per_block, smem), 32 * lanes_per_block, smem, s>>>(T, L, o);
   return cudaGetLastError();
@@ -561,7 +561,7 @@ cudaError_t launch_assemble(const TopoDev& T, const LaneDev& L, uint32_t lane, d
   // tape values: x, xo, rhs, diag, staging and the limited images (nv = 0).
   const size_t smem = size_t(4 * T.n + T.nv + T.n_stage + T.nlim + 2) * sizeof(double);
   auto* k = topo_has_b3(T) ? assemble_kernel<true> : assemble_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   k<<<1, 32, smem, s>>>(T, L, lane, out);
   return cudaGetLastError();
@@ -571,7 +571,7 @@ cudaError_t launch_lu_replay(const TopoDev& T, uint32_t n_lanes, const double* a
                              double* dx, uint8_t* bad, uint32_t lanes_per_block, cudaStream_t s) {
   const size_t per = size_t(T.nv + T.n + 1) * sizeof(double);
   const size_t smem = T.prog_bytes + T.ring_bytes + lanes_per_block * per;
-  cudaError_t e = cudaFuncSetAttribute(lu_replay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(lu_replay_kernel, smem);
   if (e != cudaSuccess) return e;
   lu_replay_kernel<<<persistent_grid(lu_replay_kernel, n_lanes, lanes_per_block, smem), 32 * lanes_per_block, smem,
                      s>>>(T, n_lanes, a, rhs, tv, dx, bad);
@@ -847,7 +847,7 @@ cudaError_t launch_lu_lanes_mixed(const TopoDev& T, const uint2* seq, uint32_t n
                                   uint32_t n_seq_f, uint32_t n_lanes, const double* a, const double* rhs, double* dx,
                                   uint8_t* bad, uint8_t* refine, uint32_t warps, cudaStream_t s) {
   const size_t smem = lu_lanes_mixed_smem(T, n_seq + n_seq_f, warps);
-  cudaError_t e = cudaFuncSetAttribute(lu_lanes_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(lu_lanes_mixed_kernel, smem);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 148, per_sm = 1;
   cudaGetDevice(&dev);
@@ -870,7 +870,7 @@ cudaError_t launch_lu_lanes(const TopoDev& T, const uint2* seq, uint32_t n_seq_a
                             const double* a, const double* rhs, double* tv, double* dx, uint8_t* bad,
                             uint32_t warps, cudaStream_t s) {
   const size_t smem = lu_lanes_smem(T, n_seq, warps);
-  cudaError_t e = cudaFuncSetAttribute(lu_lanes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(lu_lanes_kernel, smem);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 148, per_sm = 1;
   cudaGetDevice(&dev);
@@ -2145,7 +2145,7 @@ cudaError_t launch_dc_newton_group(const TopoDev* d_topos, const LaneDev* d_lane
                                    const uint32_t* d_cta_first, const uint32_t* d_ctx_lpb, uint32_t n_ctas,
                                    uint32_t max_lpb, size_t smem, const LaneOpts& o, bool has_b3, cudaStream_t s) {
   auto* k = has_b3 ? dc_newton_group_kernel<true> : dc_newton_group_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   k<<<n_ctas, 32 * max_lpb, smem, s>>>(d_topos, d_lanes, d_cta_ctx, d_cta_first, d_ctx_lpb, o);
   return cudaGetLastError();
@@ -2196,7 +2196,7 @@ cudaError_t launch_sweep(const TopoDev& T, const LaneDev& L, const SweepDev& P, 
                          uint32_t lanes_per_block, cudaStream_t s) {
   const size_t smem = T.prog_bytes + T.ring_bytes + lanes_per_block * size_t(sweep_doubles(T)) * sizeof(double);
   auto* k = topo_has_b3(T) ? sweep_kernel<true> : sweep_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(P.next_lane, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
@@ -2209,7 +2209,7 @@ cudaError_t launch_tran(const TopoDev& T, const LaneDev& L, const TranDev& P, co
   const size_t smem =
       T.prog_bytes + T.ring_bytes + lanes_per_block * size_t(T.tran_doubles + kMeasDoubles * P.n_meas) * sizeof(double);
   auto* k = topo_has_b3(T) ? tran_kernel<true> : tran_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  cudaError_t e = allow_smem(k, smem);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(P.next_lane, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
