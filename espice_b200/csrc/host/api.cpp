@@ -1066,7 +1066,7 @@ struct BlockCall {
 // (analog block, mixed, 12,288 points: 78.9 -> 64.7 ms when this came in);
 // with fewer lanes the wide CTA's lane is the faster one. The broad CTA for
 // slab lanes that have an SM each: their rows wait for L2, and sixteen warps
-// take half the rows (2,000-unknown digital block: 1,113 -> 620; working
+// take about half the rows (2,000-unknown digital block: 1,155 -> 643; working
 // sets in shared memory are smaller, their rows are chains that 256 threads
 // already hold).
 uint32_t block_choose(const esl_ctx* ctx, bool mixed, uint32_t n_lanes, const BlockCall& call, BlockDev& D, int& best) {
